@@ -1,0 +1,297 @@
+// cgchip2d.cuh -- the CG loop of a mesh that fits on chip as one persistent
+// cooperative kernel (2D, FP64, four external faces).
+//
+// A mesh cut into strips of at most kChipRows rows, 8 strips per SM (about 1.2
+// million cells on 148 SMs), keeps its CG state on the SMs for the whole loop.
+// A thread holds one column of a pair of vertically adjacent strips (up to
+// 16 rows): p, r and w in registers, the face coefficients in shared memory
+// (in registers for strips of two rows), u in registers or shared memory. Two
+// strips per thread rather than one leave 128 registers a thread, of which
+// the temporaries take their share once, not twice. The strips, the row
+// order in a strip and the reduction trees are those of k_cg_w_fused and
+// k_cg_ur_fused, so p, r, u, w, the scalars and the trip count are theirs bit
+// for bit.
+//
+// One trip is two grid-wide sums with the stencil between them. A pair needs p
+// one cell beyond its edges: it carries those ghost cells itself and updates
+// them as their owners do, p = beta p + r, from the edge cells of r that
+// every warp hands over as tagged words (gridsum.cuh). An edge word is
+// rewritten after the next p.w sum, to which each of its readers has
+// contributed a partial formed with it; a slot of one sum after the other
+// sum, to which every block contributes only when it has read all the slots.
+//
+// What bounds it: two sums per trip, each one hand-over through L2, three block
+// barriers and two shuffle trees (about 2 us of a trip); then, from about 8
+// rows a thread, shared-memory bandwidth. Measured, us per trip of a whole
+// timestep: 64^2 5.7 against 20 for the two launches per trip it replaces,
+// 512^2 6.5 against 27, 1000^2 10.2; 1080^2, just past the limit, still takes
+// 37 with two launches.
+#pragma once
+
+#include "gridsum.cuh"
+#include "suite2d_impl.hpp"
+
+namespace tl2d {
+
+struct ChipArgs {
+    double *p, *r, *u, *w;
+    const double *kx, *ky;
+    tl::TagWord* words;        // kChipWords per pair: all sums p.w, all r.r, side cells, edge rows
+    unsigned long long tag0;   // tags tag0 + 1 .. tag0 + max_iters are new to the words
+    int gx, gy;                // strips of the mesh
+    int groups;                // strip pairs per block
+    DevState* st;
+    double *alphas, *betas;
+    DevParams prm;
+    int* host_mirror;
+    int* err;                  // device word: a wait gave up
+    int* err_host;             // its mapped copy for the host
+};
+
+// Where a block keeps the arrays other than p, r and w: registers while 128 a
+// thread suffice, else shared memory, laid out for the largest block. The
+// operator is held as the face coefficient left of each cell, the one below
+// and, while there is room, the diagonal 1 + (kxr + kxc) + (kyu + kyc); kx is
+// laid out 33 to a warp, the last being the one right of its columns.
+constexpr int kChipT = BX * kChipPairs, kChipWarps = kChipT / 32;
+template <int H>
+struct ChipPlace {
+    static constexpr int R = 2 * H;            // rows of a pair
+    static constexpr bool kRegK = H <= 2;      // the operator in registers
+    static constexpr bool kRegU = H <= 4;      // u in registers
+    static constexpr bool kDiag = H <= 6;      // the diagonal kept
+    static constexpr int KXW = kChipWarps * 33;
+    static constexpr int kd = 0;                                          // [R][T]
+    static constexpr int kx = kd + (kRegK || !kDiag ? 0 : R * kChipT);    // [R][warps][33]
+    static constexpr int ky = kx + (kRegK ? 0 : R * KXW);                 // [R + 1][T]
+    static constexpr int u = ky + (kRegK ? 0 : (R + 1) * kChipT);     // [R][T]
+    static constexpr int bytes = (int)sizeof(double) * (u + (kRegU ? 0 : R * kChipT));
+};
+
+template <int H>
+static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
+{
+    extern __shared__ double chip_smem_raw[];
+    __shared__ tl::StripSumSmem sums;
+    __shared__ double side[kChipWarps][32];   // per warp: rows 0 .. left, 16 .. right of its columns
+    using P = ChipPlace<H>;
+    constexpr int R = P::R;
+    constexpr bool kRegK = P::kRegK, kRegU = P::kRegU, kDiag = P::kDiag;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int pair = blockIdx.x * a.groups + tid / BX;
+    const int by = pair / a.gx * 2, bx = pair % a.gx;
+    const bool has = by < a.gy;
+    const int pairs = a.gx * ((a.gy + 1) / 2), strips = a.gx * a.gy;
+    for (int n = tid; n < 3 * (int)blockDim.x; n += blockDim.x) {
+        const int row = (n >> 1) / a.gx * 2 + (n & 1);
+        sums.strip_of[n] = (short)(row < a.gy ? (n >> 1) % a.gx + row * a.gx : -1);
+    }
+    if (tid == 0) sums.bad = 0;
+    const int k = g.hd + bx * BX + tid % BX;
+    const int j0 = has ? g.hd + by * g.rows : g.hd, j1 = min(j0 + 2 * g.rows, g.y - g.hd);
+    const int nr = has ? j1 - j0 : 1;
+    const bool active = has && k < g.x - g.hd;
+    const int kk = min(k, g.x - g.hd - 1);   // lanes past the interior load its last column
+    const bool at_l = k == g.hd, at_r = k == g.x - g.hd - 1;
+    const bool refl_d = j0 == g.hd || !active, refl_u = j1 == g.y - g.hd || !active;
+    const int x = g.x, i0 = kk + j0 * x;     // a mesh that fits on chip has 32-bit indices
+    // side cells: lane q has row q of the column left of the warp's, lane 16 + q of the one right of them
+    const int gq = lane & 15, gk = k - lane + (lane < 16 ? -1 : 32);
+    const bool ghost = has && gq < nr && gk >= g.hd && gk < g.x - g.hd;
+    const int gi = gk + (j0 + gq) * x;       // (valid when ghost)
+    // and hands over row q of its own first (0 ..) or last (16 ..) column
+    const bool edge = has && gq < nr && k - lane + (lane < 16 ? 0 : 31) < g.x - g.hd;
+    // word indices: the warps of a row of pairs in column order; the rows of edge cells bottom, top
+    const int side_w = 4 * pairs + (pair * 4 + (warp & 3)) * 32 + lane;
+    const int side_r = lane < 16 ? side_w - 32 + 16 : side_w + 32 - 16;
+    const int row_w = 132 * pairs + pair * 2 * BX + tid % BX;
+    const int down_r = row_w - (2 * a.gx - 1) * BX, up_r = row_w + 2 * a.gx * BX;
+    double* const mine = side[warp];
+    const double* const mine_l = mine + (lane == 0 ? 0 : 16);   // the neighbour a lane at the warp's edge lacks
+    const bool first = lane == 0, last = lane == 31 || at_r;
+    const bool lone = first && at_r;         // a warp of one column: its right neighbour is itself
+    const bool wl = k - lane == g.hd, wr = k - lane + 32 >= g.x - g.hd;   // warp at the domain's left / right
+
+    double* const KD = chip_smem_raw + P::kd + tid;
+    double* const KX = chip_smem_raw + P::kx + warp * 33 + lane;
+    double* const KY = chip_smem_raw + P::ky + tid;
+    double* const U = chip_smem_raw + P::u + tid;
+    double p[R], r[R], w[R], u[kRegU ? R : 1], kdv[kRegK ? R : 1], kxv[kRegK ? R : 1], kyv[kRegK ? R : 1];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int i = i0 + (q < nr ? q : 0) * x;
+        p[q] = a.p[i];
+        r[q] = a.r[i];
+        w[q] = 0.0;
+        if (kRegU) u[kRegU ? q : 0] = a.u[i];
+        else U[q * kChipT] = a.u[i];
+        const double kxc = a.kx[i], kyc = a.ky[i];
+        const double kd = 1.0 + (a.kx[i + 1] + kxc) + (a.ky[i + x] + kyc);
+        if (kRegK) {
+            kdv[kRegK ? q : 0] = kd;
+            kxv[kRegK ? q : 0] = kxc;
+            kyv[kRegK ? q : 0] = kyc;
+        } else {
+            if (kDiag) KD[q * kChipT] = kd;
+            KX[q * P::KXW] = kxc;
+            if (lane == 31) KX[q * P::KXW + 1] = a.kx[i + 1];
+            KY[q * kChipT] = kyc;
+        }
+    }
+    const double ky_top = a.ky[i0 + nr * x];   // the face above the pair
+    if (!kRegK) KY[nr * kChipT] = ky_top;
+    double p_d = refl_d ? 0.0 : a.p[i0 - x];
+    double p_u = refl_u ? 0.0 : a.p[i0 + nr * x];
+    double p_s = ghost ? a.p[gi] : 0.0;
+    const double k_s = ghost && lane >= 16 ? a.kx[gi] : 1.0;   // right of the warp: the face's coefficient
+    double rro = a.st->rro, pw = 0.0, alpha = 0.0, beta = 0.0;
+    int trip = 0, reason = 0;
+    bool ok = true;
+    __syncthreads();
+
+    // w = A p and p.w over the pair's rows; FULL: all R of them. The term of
+    // the right neighbour, kxr r, is that cell's own kxc c, formed there.
+    auto sweep_w = [&](auto full, double (&acc)[2]) {
+        constexpr bool FULL = decltype(full)::value;
+        double pd = refl_d ? p[0] : p_d;
+        double kyc = kRegK ? kyv[0] : KY[0];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            if (!FULL && q >= nr) break;
+            const double pc = p[q];
+            const bool top = FULL ? q == R - 1 : q == nr - 1;
+            const double pu = top ? (refl_u ? pc : p_u) : p[q + 1 < R ? q + 1 : q];
+            const double kxc = kRegK ? kxv[kRegK ? q : 0] : KX[q * P::KXW];
+            const double gh = mine_l[q];
+            double pl = __shfl_up_sync(kFull, pc, 1);
+            double xr = __shfl_down_sync(kFull, kxc * pc, 1);
+            if (first) pl = gh;
+            if (last) xr = gh;
+            if (lone) xr = mine[16 + q];
+            const double kyu = kRegK ? (top ? ky_top : kyv[kRegK && q + 1 < R ? q + 1 : 0]) : KY[(q + 1) * kChipT];
+            double kd;
+            if (kRegK) kd = kdv[kRegK ? q : 0];
+            else if (kDiag) kd = KD[q * kChipT];
+            else kd = 1.0 + (KX[q * P::KXW + 1] + kxc) + (kyu + kyc);
+            const double v = kd * pc - (xr + kxc * pl) - (kyu * pu + kyc * pd);   // smvp
+            w[q] = v;
+            acc[FULL ? q / H : (q < g.rows ? 0 : 1)] += v * pc;
+            pd = pc;
+            kyc = kyu;
+        }
+    };
+    // r -= alpha w and r.r, rows in the order of k_cg_ur_fused
+    auto sweep_r = [&](auto full, double (&acc)[2]) {
+        constexpr bool FULL = decltype(full)::value;
+#pragma unroll
+        for (int n = 0; n < R; ++n) {
+            const int q = TL2D_UR_REVERSE ? R - 1 - n : n;
+            if (!FULL && q >= nr) continue;
+            const double rn = r[q] - alpha * w[q];
+            r[q] = rn;
+            acc[FULL ? q / H : (q < g.rows ? 0 : 1)] += rn * rn;
+            if (lane == 0 || lane == 31) mine[(lane & 16) + q] = rn;
+        }
+    };
+    const bool full = nr == R && g.rows == H;
+
+    while (reason == 0) {
+        const unsigned long long tag = a.tag0 + 1 + (unsigned long long)trip;
+        if (trip > 0) {   // p = beta p + r, the ghosts with their owners' r
+            double r_d = 0.0, r_u = 0.0, r_s = 0.0;
+            const bool gd = refl_d || word_load(a.words + down_r, tag - 1, r_d);
+            const bool gu = refl_u || word_load(a.words + up_r, tag - 1, r_u);
+            const bool gs = !ghost || word_load(a.words + side_r, tag - 1, r_s);
+#pragma unroll
+            for (int q = 0; q < R; ++q) p[q] = beta * p[q] + r[q];
+            if (!gd) r_d = tl::word_wait(a.words + down_r, tag - 1, a.err, &sums.bad);
+            if (!gu) r_u = tl::word_wait(a.words + up_r, tag - 1, a.err, &sums.bad);
+            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, a.err, &sums.bad);
+            p_s = beta * p_s + r_s;
+            p_d = beta * p_d + r_d;
+            p_u = beta * p_u + r_u;
+        }
+        __syncwarp();
+        mine[lane] = k_s * p_s;
+        __syncwarp();
+        if (wl || wr) {   // the reflective halo: the edge cell itself
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                if (at_l) mine[q] = p[q];
+                if (at_r) mine[16 + q] = __ldg(a.kx + i0 + (q < nr ? q : 0) * x + 1) * p[q];
+            }
+            __syncwarp();
+        }
+        double acc[2] = {0.0, 0.0};
+        if (full) sweep_w(std::true_type(), acc);
+        else sweep_w(std::false_type(), acc);
+        if (!active) acc[0] = acc[1] = 0.0;
+        ok = tl::strip_sum(acc, has ? pair : -1, strips, sums, a.words, tag, a.err, [] {},
+                           [&](double t) { return rro / t; }, pw, alpha);
+        if (!ok) break;
+        acc[0] = acc[1] = 0.0;
+        if (full) sweep_r(std::true_type(), acc);
+        else sweep_r(std::false_type(), acc);
+        if (!active) acc[0] = acc[1] = 0.0;
+        __syncwarp();
+        if (edge) tl::word_store(a.words + side_w, mine[lane], tag);
+        if (active) {
+            tl::word_store(a.words + row_w, r[0], tag);
+            double top = r[R - 1];
+            if (!full) {
+                top = r[0];
+#pragma unroll
+                for (int q = 1; q < R; ++q) top = q < nr ? r[q] : top;
+            }
+            tl::word_store(a.words + row_w + BX, top, tag);
+        }
+        double rrn;
+        ok = tl::strip_sum(acc, has ? pair : -1, strips, sums, a.words + 2 * pairs, tag, a.err,
+                           [&] {
+#pragma unroll
+                               for (int q = 0; q < R; ++q) {
+                                   if (kRegU) u[kRegU ? q : 0] += alpha * p[q];
+                                   else U[q * kChipT] += alpha * p[q];
+                               }
+                           },
+                           [&](double t) { return t / rro; }, rrn, beta);
+        if (!ok) break;
+        if (blockIdx.x == 0 && tid == 0) {
+            a.alphas[trip] = alpha;
+            a.betas[trip] = beta;
+        }
+        rro = rrn;
+        reason = tl::trip_reason(a.prm, rrn, trip);
+        ++trip;
+    }
+
+    if (active) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            if (q < nr) {
+                const int i = i0 + q * x;
+                a.p[i] = p[q];
+                a.r[i] = r[q];
+                a.w[i] = w[q];
+                a.u[i] = kRegU ? u[kRegU ? q : 0] : U[q * kChipT];
+            }
+        }
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        DevState* st = a.st;
+        st->pw = pw;
+        st->rro = st->rrn = st->error = rro;
+        st->alpha = alpha;
+        st->beta = beta;
+        st->trip = trip;
+        st->done = 1;
+        st->reason = reason;
+        if (!ok) *(volatile int*)a.err_host = 1;
+        a.host_mirror[0] = 1;
+        a.host_mirror[1] = trip;
+        a.host_mirror[2] = reason;
+    }
+}
+
+}  // namespace tl2d

@@ -18,6 +18,7 @@
 //
 // diffuse_overload (2d/application.h:9-11) runs every timestep this way.
 #include "blocked2d.cuh"
+#include "cgchip2d.cuh"
 #include "host_maths.hpp"
 #include "pcg2d.cuh"
 #include "suite2d_impl.hpp"
@@ -138,11 +139,44 @@ struct Run {
     // pending). Closes the phase: last p update and the halo of u and p.
     DevState cg_phase(int from, bool fresh)
     {
+        if (from == 0 && fresh && s->chip_words && prm.max_iters > 0) return cg_close(cg_chip(), chunk->r);
         FinCgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
         const Scalar alpha{0.0, &s->d_state->alpha};
         return cg_trips(from, fresh, chunk->r, [&](double* p) {
             launch_cg_ur2(s, gi, alpha, chunk->u, p, chunk->r, chunk->w, done(), fin_ur);
         });
+    }
+
+    // The whole loop in one launch (k_cg_chip) for a mesh whose state fits on
+    // the SMs; its strip pairs spread over as many SMs as there are.
+    DevState cg_chip()
+    {
+        const int pairs = gi.x * tl::ceil_div(gi.y, 2);
+        ChipArgs a{chunk->p, chunk->r, chunk->u, chunk->w, chunk->kx, chunk->ky, s->chip_words, s->chip_tag,
+                    (int)gi.x, (int)gi.y, tl::ceil_div(pairs, s->sm_count), s->d_state, s->d_cg_alphas, s->d_cg_betas,
+                   prm, s->d_mirror, s->chip_err, s->d_mirror + kTmaErrWord2};
+        s->chip_tag += (unsigned long long)prm.max_iters;
+        switch (s->g.rows) {
+            case 2: launch_chip<2>(a, pairs); break;
+            case 3: launch_chip<3>(a, pairs); break;
+            case 4: launch_chip<4>(a, pairs); break;
+            case 5: launch_chip<5>(a, pairs); break;
+            case 6: launch_chip<6>(a, pairs); break;
+            case 7: launch_chip<7>(a, pairs); break;
+            default: launch_chip<kChipRows>(a, pairs); break;
+        }
+        return read_state();
+    }
+    template <int H>
+    void launch_chip(ChipArgs& a, int pairs)
+    {
+        const int threads = a.groups * BX;
+        constexpr size_t smem = ChipPlace<H>::bytes;
+        TL_CUDA(cudaFuncSetAttribute(k_cg_chip<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        void* args[] = {&s->g, &a};
+        TL_LAUNCH(s, "k_cg_chip", TL_CUDA(cudaLaunchCooperativeKernel((const void*)k_cg_chip<H>,
+                                                                      dim3(tl::ceil_div(pairs, a.groups)),
+                                                                      dim3(threads), args, smem, s->stream)));
     }
 
     // The CG loop with `fold` the field of the p update p = beta p + fold (r
@@ -173,6 +207,14 @@ struct Run {
         const int flips = fresh ? std::max(0, ran - 1) : ran;
         double* pcur = buf[flips & 1];
         if (pcur != chunk->p) swap_alt(s, chunk, ALT_P);
+        return cg_close(st, fold);
+    }
+
+    // Closes a CG phase that ended in state st: the last p update, the halos
+    // of p and u, and the host's coefficients.
+    DevState cg_close(const DevState& st, const double* fold)
+    {
+        const Scalar beta{0.0, &s->d_state->beta};
         TL_LAUNCH(s, "k_cg_close", (k_cg_close<<<gi, BX, 0, s->stream>>>(s->g, fc, beta, 1, chunk->p, fold,
                                                                            chunk->u)));
         // host copies of the CG coefficients (the reference drivers keep them on the host)

@@ -40,20 +40,26 @@ struct DevParams {
 // Stop test of the solver loops: 2D tests the error itself, 3D its square
 // root (3d/drivers/cg_solver_driver.c:24-25); the switch from CG to
 // Chebyshev/PPCG is evaluated for the next trip (2d/drivers/cheby_driver.c:30-32).
+// 0: another trip follows trip tt, whose error (as tested) is e.
+__device__ __forceinline__ int trip_reason(const DevParams& prm, double e, int tt)
+{
+    if (fabs(e) < prm.eps) return 1;
+    if (tt + 1 >= prm.max_iters) return 3;
+    if (prm.switch_enabled) {
+        const bool sw = prm.error_switch ? (e < prm.eps_lim) && (tt + 1 > kCgItersForEigenvalues)
+                                         : (tt + 1 > prm.presteps) && (e < kErrorSwitchMax);
+        if (sw) return 2;
+    }
+    return 0;
+}
+
 __device__ __forceinline__ void end_of_trip(DevState* st, const DevParams& prm, double error, int* host_mirror)
 {
     const double e = prm.dims3 ? sqrt(error) : error;
     st->error = e;
     const int tt = st->trip;
     st->trip = tt + 1;
-    int reason = 0;
-    if (fabs(e) < prm.eps) reason = 1;
-    else if (tt + 1 >= prm.max_iters) reason = 3;
-    else if (prm.switch_enabled) {
-        const bool sw = prm.error_switch ? (e < prm.eps_lim) && (tt + 1 > kCgItersForEigenvalues)
-                                         : (tt + 1 > prm.presteps) && (e < kErrorSwitchMax);
-        if (sw) reason = 2;
-    }
+    const int reason = trip_reason(prm, e, tt);
     if (reason) {
         st->done = 1;
         st->reason = reason;

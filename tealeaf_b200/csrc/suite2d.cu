@@ -398,6 +398,8 @@ void run_kernel_initialise(Chunk* chunk, Settings* settings)
     for (const Req& r : reqs) bytes += align((size_t)r.count * sizeof(double));
     bytes += align((size_t)s->partial_capacity * sizeof(double)) + align(tl::kMaxSums * sizeof(double)) + 256;
     bytes += align(sizeof(DevState));
+    const int pairs = chip_pairs(s->g, s->sm_count);
+    bytes += align((size_t)pairs * kChipWords * sizeof(tl::TagWord)) + 256;
     if (!TL_CUDA(cudaMalloc(&s->slab, bytes))) return;
     s->slab_bytes = bytes;
     TL_CUDA(cudaMemsetAsync(s->slab, 0, bytes, s->stream));
@@ -413,6 +415,10 @@ void run_kernel_initialise(Chunk* chunk, Settings* settings)
     s->rs.ticket = (unsigned int*)cur;
     cur += 256;
     s->d_state = (DevState*)cur;
+    cur += align(sizeof(DevState));
+    s->chip_err = (int*)cur;
+    cur += 256;
+    if (pairs > 0) s->chip_words = (tl::TagWord*)cur;
     if (!TL_CUDA(cudaHostAlloc((void**)&s->h_out, tl::kMaxSums * sizeof(double) + 64, cudaHostAllocMapped))) return;
     double* dev_view = nullptr;
     if (!TL_CUDA(cudaHostGetDevicePointer((void**)&dev_view, s->h_out, 0))) return;

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "blocked2d.cuh"
+#include "gridsum.cuh"
 
 #include <cuda_runtime.h>
 
@@ -50,6 +51,13 @@ struct TlSuite2D {
     double* d_cheby_alphas = nullptr;
     double* d_cheby_betas = nullptr;
     int table_len = 0;
+
+    // CG loop of a mesh that fits on chip (cgchip2d.cuh): the words its blocks
+    // exchange (null for a larger mesh), the last tag used in them and the
+    // word its bounded waits raise.
+    tl::TagWord* chip_words = nullptr;
+    unsigned long long chip_tag = 0;
+    int* chip_err = nullptr;
 
     // Device-resident driver: Chebyshev trips / PPCG inner steps temporally
     // blocked in shared memory (blocked2d.cuh); off = one launch per step.
@@ -144,6 +152,22 @@ inline int choose_rows(int nx, int ny, int sm_count, int min_blocks = TL2D_MINB,
         if (rows <= max_rows) return rows;
     }
 }
+// Vertical pairs of strips of a mesh whose CG state fits on the SMs
+// (cgchip2d.cuh): strips of at most kChipRows rows, kChipPairs pairs of BX
+// columns per SM; 0 for a larger mesh. choose_rows cuts one wave of 8 strips per SM,
+// so all but a few meshes with strips that short fit (those whose odd number
+// of strips per band leaves half of the last pairs empty).
+constexpr int kChipRows = 8;
+constexpr int kChipPairs = 4;
+inline int chip_pairs(const Geo& g, int sm_count)
+{
+    const dim3 d = interior_grid(g);
+    const long pairs = (long)d.x * tl::ceil_div(d.y, 2);
+    return g.rows <= kChipRows && pairs <= (long)kChipPairs * sm_count ? (int)pairs : 0;
+}
+// Words of one pair: its two strips' sums, twice; 4 warps' 32 side cells; 2
+// rows of BX edge cells.
+constexpr int kChipWords = 4 + 4 * 32 + 2 * BX;
 // Waits for the stream and returns the published sums.
 bool fetch(TlSuite2D* s, int n, double* out);
 // Runs every pending operation (p update, then halo updates).

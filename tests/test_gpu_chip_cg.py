@@ -1,0 +1,59 @@
+"""The CG loop held on chip (k_cg_chip) against the same loop through run_*
+(one launch per sweep): every field, iteration count and summary bit for bit,
+at the edges of its tiling -- strips of 2 to 8 rows, single strips and odd
+numbers of them, ragged last strips, meshes one column past a warp or a
+128-column band, caps of 1 and 2 trips and a solve to convergence."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tealeaf_b200 import problems
+from tealeaf_b200.host import Host
+
+pytestmark = pytest.mark.gpu
+
+FIELDS2 = ("u", "u0", "p", "r", "w", "kx", "ky", "energy")
+
+
+def both(dims, cells, cap, steps=1, **kw):
+    text = problems.seeded(dims, cells, 11, 4, 0 if dims == 3 else 2, solver="cg", end_step=steps,
+                           max_iters=cap, name="chip", **kw).tea_in()
+    return Host(text, dims), Host(text, dims)
+
+
+@pytest.mark.parametrize("cells,cap,steps", [
+    ((5, 1), 3, 1), ((2, 3), 20000, 2), ((33, 5), 20000, 2), ((32, 2), 40, 1), ((129, 37), 20000, 2),
+    ((65, 4), 1, 1), ((257, 129), 2, 1), ((640, 61), 30, 1), ((1024, 440), 25, 1), ((513, 941), 25, 1),
+    ((1000, 700), 25, 1), ((900, 880), 25, 1), ((1025, 900), 25, 1), ((1000, 1180), 25, 1), ((1024, 1184), 25, 1),
+])
+def test_chip_cg_is_bit_identical(cells, cap, steps):
+    a, b = both(2, cells, cap, steps)
+    try:
+        n0 = b.lib.tl2d_launch_count(C.byref(b.chunk))
+        for tt in range(steps):
+            ra, rb = a.solve(tt), b.solve_device(tt)
+            assert ra.iterations == rb.iterations
+            assert ra.error == rb.error
+            assert ra.summary == rb.summary
+            for f in FIELDS2:
+                assert np.array_equal(a.download(f), b.download(f)), (tt, f)
+        # the whole loop ran as one launch, not two per trip
+        assert b.lib.tl2d_launch_count(C.byref(b.chunk)) - n0 <= 16 * steps
+    finally:
+        a.finalise()
+        b.finalise()
+
+
+def test_chip_cg_two_chunks_in_turn():
+    """Two chunks of different sizes stepped in turn keep their own words."""
+    a, b = both(2, (130, 66), 20000, 3)
+    c, d = both(2, (70, 300), 20000, 3)
+    try:
+        for tt in range(3):
+            for x, y in ((a, b), (c, d)):
+                assert x.solve(tt).iterations == y.solve_device(tt).iterations
+                assert np.array_equal(x.download("u"), y.download("u"))
+    finally:
+        for h in (a, b, c, d):
+            h.finalise()
