@@ -400,6 +400,8 @@ void run_kernel_initialise(Chunk* chunk, Settings* settings)
     bytes += align(sizeof(DevState));
     const int pairs = chip_pairs(s->g, s->sm_count);
     bytes += align((size_t)pairs * kChipWords * sizeof(tl::TagWord)) + 256;
+    s->sum_cells = (x - 2L * settings->halo_depth) * (y - 2L * settings->halo_depth);
+    bytes += tl::sum_scratch_bytes(s->sum_cells);
     if (!TL_CUDA(cudaMalloc(&s->slab, bytes))) return;
     s->slab_bytes = bytes;
     TL_CUDA(cudaMemsetAsync(s->slab, 0, bytes, s->stream));
@@ -419,6 +421,8 @@ void run_kernel_initialise(Chunk* chunk, Settings* settings)
     s->chip_err = (int*)cur;
     cur += 256;
     if (pairs > 0) s->chip_words = (tl::TagWord*)cur;
+    cur += align((size_t)pairs * kChipWords * sizeof(tl::TagWord));
+    s->sum_scratch = cur;
     if (!TL_CUDA(cudaHostAlloc((void**)&s->h_out, tl::kMaxSums * sizeof(double) + 64, cudaHostAllocMapped))) return;
     double* dev_view = nullptr;
     if (!TL_CUDA(cudaHostGetDevicePointer((void**)&dev_view, s->h_out, 0))) return;
@@ -563,10 +567,10 @@ void run_field_summary(Chunk* chunk, Settings* settings, double* vol, double* ma
     (void)settings;
     TlSuite2D* s = ready(chunk);
     if (!s) return;
-    TL_LAUNCH(s, "k_field_summary_ordered",
-              tl::launch_field_summary_ordered(s->stream, s->g.x, s->g.y, 1, s->g.hd, 0, chunk->volume,
-                                               chunk->density, chunk->energy0, chunk->u, s->rs.out_dev,
-                                               s->rs.out_host));
+    const tl::SumFields f{s->g.x, s->g.hd, 0, s->g.x - 2 * s->g.hd, s->g.y - 2 * s->g.hd, (long)s->g.x * s->g.y, s->sum_cells,
+                          chunk->volume, chunk->density, chunk->energy0, chunk->u};
+    tl::field_summary_ordered(s->stream, f, tl::sum_scratch(s->sum_scratch, f.n), s->rs.out_dev, s->rs.out_host,
+                              [&](const char* name, auto call) { TL_LAUNCH(s, name, call()); });
     double o[4];
     if (!fetch(s, 4, o)) return;
     *vol += o[0];

@@ -5,6 +5,7 @@
 
 #include "blocked2d.cuh"
 #include "gridsum.cuh"
+#include "summary.cuh"
 
 #include <cuda_runtime.h>
 
@@ -26,6 +27,8 @@ struct TlSuite2D {
     tl::ReduceSlots rs{};
     double* h_out = nullptr;          // mapped pinned result slots
     long partial_capacity = 0;        // doubles
+    long sum_cells = 0;               // interior cells of the field summary
+    void* sum_scratch = nullptr;      // its tile sums and pairs (summary.cuh)
     State* d_states = nullptr;
     int d_states_cap = 0;
     double* d_comm = nullptr;         // pack/unpack staging

@@ -352,6 +352,8 @@ void run_kernel_initialise(Chunk* chunk, Settings* settings)
     for (const Req& r : reqs) bytes += align((size_t)r.count * sizeof(double));
     bytes += align((size_t)s->partial_capacity * sizeof(double)) + align(tl::kMaxSums * sizeof(double)) + 256;
     bytes += align(sizeof(tl::DevState));
+    s->sum_cells = (x - 2L * settings->halo_depth) * (y - 2L * settings->halo_depth) * (z - 2L * settings->halo_depth);
+    bytes += tl::sum_scratch_bytes(s->sum_cells);
     if (!TL_CUDA(cudaMalloc(&s->slab, bytes))) return;
     s->slab_bytes = bytes;
     TL_CUDA(cudaMemsetAsync(s->slab, 0, bytes, s->stream));
@@ -367,6 +369,8 @@ void run_kernel_initialise(Chunk* chunk, Settings* settings)
     s->rs.ticket = (unsigned int*)cur;
     cur += 256;
     s->d_state = (tl::DevState*)cur;
+    cur += align(sizeof(tl::DevState));
+    s->sum_scratch = cur;
     if (!TL_CUDA(cudaHostAlloc((void**)&s->h_out, tl::kMaxSums * sizeof(double) + 64, cudaHostAllocMapped))) return;
     double* dev_view = nullptr;
     if (!TL_CUDA(cudaHostGetDevicePointer((void**)&dev_view, s->h_out, 0))) return;
@@ -502,10 +506,10 @@ void run_field_summary(Chunk* chunk, Settings* settings, double* vol, double* ma
     (void)settings;
     TlSuite3D* s = ready(chunk);
     if (!s) return;
-    TL3_LAUNCH(s, "k_field_summary_ordered",
-               tl::launch_field_summary_ordered(s->stream, s->g.x, s->g.y, s->g.z, s->g.hd, s->g.hd, chunk->volume,
-                                                chunk->density, chunk->energy0, chunk->vec_u, s->rs.out_dev,
-                                                s->rs.out_host));
+    const tl::SumFields f{s->g.x, s->g.hd, s->g.hd, s->g.x - 2 * s->g.hd, s->g.y - 2 * s->g.hd, s->g.xy(), s->sum_cells,
+                          chunk->volume, chunk->density, chunk->energy0, chunk->vec_u};
+    tl::field_summary_ordered(s->stream, f, tl::sum_scratch(s->sum_scratch, f.n), s->rs.out_dev, s->rs.out_host,
+                              [&](const char* name, auto call) { TL3_LAUNCH(s, name, call()); });
     double o[4];
     if (!fetch(s, 4, o)) return;
     *vol += o[0];

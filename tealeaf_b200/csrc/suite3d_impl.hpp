@@ -5,6 +5,7 @@
 
 #include "blocked3d.cuh"
 #include "kernels3d.cuh"
+#include "summary.cuh"
 
 #include <cuda_runtime.h>
 
@@ -22,6 +23,8 @@ struct TlSuite3D {
     tl::ReduceSlots rs{};
     double* h_out = nullptr;
     long partial_capacity = 0;
+    long sum_cells = 0;               // interior cells of the field summary
+    void* sum_scratch = nullptr;      // its tile sums and pairs (summary.cuh)
     State* d_states = nullptr;
     int d_states_cap = 0;
     double* d_comm = nullptr;
