@@ -28,16 +28,17 @@ using namespace tl2d::rf;
 
 namespace {
 
-constexpr int kBatch = 16;
+constexpr int kGroup = 8;   // trips per launched group
 
 template <typename T, bool FUSE_P>
 __global__ void __launch_bounds__(BX, Pack<T>::MINB) k_rf_w(Lay L, const MxState* __restrict__ st,
-                                                            const T* __restrict__ p_in, T* __restrict__ p_out,
-                                                            const T* __restrict__ r, T* __restrict__ w,
-                                                            const T* __restrict__ kx, const T* __restrict__ ky,
-                                                            ReduceSlots rs, FinMxW fin)
+                                                            T* p0, T* p1, const T* __restrict__ r,
+                                                            T* __restrict__ w, const T* __restrict__ kx,
+                                                            const T* __restrict__ ky, ReduceSlots rs, FinMxW fin)
 {
     if (mx_idle(st)) return;
+    T* const p_out = st->trip & 1 ? p1 : p0;
+    const T* const p_in = FUSE_P ? (st->trip & 1 ? p0 : p1) : p_out;
     const double bt = FUSE_P ? st->beta : 0.0;
     double acc[1] = {rf_w_tile<T, FUSE_P, false, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, bt, p_in, p_out,
                                                                          r, w, kx, ky)};
@@ -46,10 +47,12 @@ __global__ void __launch_bounds__(BX, Pack<T>::MINB) k_rf_w(Lay L, const MxState
 
 template <typename T>
 __global__ void __launch_bounds__(BX, Pack<T>::MINB) k_rf_ur(Lay L, const MxState* __restrict__ st, T* __restrict__ xs,
-                                                             const T* __restrict__ p, T* __restrict__ r,
-                                                             const T* __restrict__ w, ReduceSlots rs, FinMxUr fin)
+                                                             const T* __restrict__ p0, const T* __restrict__ p1,
+                                                             T* __restrict__ r, const T* __restrict__ w,
+                                                             ReduceSlots rs, FinMxUr fin)
 {
     if (mx_idle(st)) return;
+    const T* const p = st->trip & 1 ? p1 : p0;
     double acc[1] = {rf_ur_tile<T, false, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, st->alpha, xs, p, r, w)};
     tl::grid_sum<1, BX>(acc, rs, block_id(), block_count(), fin);
 }
@@ -169,19 +172,20 @@ const CUtensorMap* rf_map(TlSuite2D* s, const Lay& L, const T* ptr, bool ring)
     });
 }
 
-// The refinement w sweep (k_rf_w semantics), by TMA where the maps encode.
-// Internal linkage with the kernels, as the drop-in helpers.
+// The refinement w sweep (k_rf_w semantics), by TMA where the maps encode; r:
+// the field folded into p. Internal linkage with the kernels, as the drop-in
+// helpers.
 template <typename T, bool FUSE_P>
-void rf_w(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, const T* p_in, T* p_out, const T* r,
-          FinMxW fin)
+void rf_w(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, const T* r, FinMxW fin)
 {
     if (s->tma) {
-        const CUtensorMap *mp = rf_map(s, b.L, p_in, false), *mph = rf_map(s, b.L, p_in, true);
+        const CUtensorMap *mp0 = rf_map<T>(s, b.L, b.f[RF_P0], false), *mp1 = rf_map<T>(s, b.L, b.f[RF_P1], false);
+        const CUtensorMap *mh0 = rf_map<T>(s, b.L, b.f[RF_P0], true), *mh1 = rf_map<T>(s, b.L, b.f[RF_P1], true);
         const CUtensorMap *mr = rf_map(s, b.L, r, false), *mrh = rf_map(s, b.L, r, true);
         const CUtensorMap *mkx = rf_map<T>(s, b.L, b.f[RF_KX], false), *mkxh = rf_map<T>(s, b.L, b.f[RF_KX], true);
         const CUtensorMap* mky = rf_map<T>(s, b.L, b.f[RF_KY], false);
-        if (mp && mph && mr && mrh && mkx && mkxh && mky) {
-            const RfWMaps m{*mp, *mr, *mkx, *mky, *mph, *mrh, *mkxh};
+        if (mp0 && mp1 && mh0 && mh1 && mr && mrh && mkx && mkxh && mky) {
+            const RfWMaps m{{*mp0, *mp1}, *mr, *mkx, *mky, {*mh0, *mh1}, *mrh, *mkxh};
             constexpr size_t smem = rf_w_tma_bytes<T>();
             static unsigned attr_set = 0;
             if (!(attr_set & (1u << (s->device & 31)))) {
@@ -190,25 +194,26 @@ void rf_w(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, const 
                 attr_set |= 1u << (s->device & 31);
             }
             TL_LAUNCH(s, name, (k_rf_w_tma<T, FUSE_P><<<gl, BX, smem, s->stream>>>(
-                                   b.L, b.st, m, p_out, b.f[RF_W], s->rs, fin, s->d_mirror + kTmaErrWord2)));
+                                   b.L, b.st, m, b.f[RF_P0], b.f[RF_P1], b.f[RF_W], s->rs, fin,
+                                   s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
-    TL_LAUNCH(s, name, (k_rf_w<T, FUSE_P><<<gl, BX, 0, s->stream>>>(b.L, b.st, p_in, p_out, r, b.f[RF_W],
+    TL_LAUNCH(s, name, (k_rf_w<T, FUSE_P><<<gl, BX, 0, s->stream>>>(b.L, b.st, b.f[RF_P0], b.f[RF_P1], r, b.f[RF_W],
                                                                      b.f[RF_KX], b.f[RF_KY], s->rs, fin)));
 }
 
 // The refinement u/r update (k_rf_ur semantics), by TMA where the maps encode.
 template <typename T>
-void rf_ur(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, const T* p, T* r, FinMxUr fin)
+void rf_ur(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, FinMxUr fin)
 {
     if (s->tma) {
         const CUtensorMap* mx = rf_map<T>(s, b.L, b.f[RF_XS], false);
-        const CUtensorMap* mp = rf_map(s, b.L, p, false);
-        const CUtensorMap* mr = rf_map<T>(s, b.L, r, false);
+        const CUtensorMap *mp0 = rf_map<T>(s, b.L, b.f[RF_P0], false), *mp1 = rf_map<T>(s, b.L, b.f[RF_P1], false);
+        const CUtensorMap* mr = rf_map<T>(s, b.L, b.f[RF_R], false);
         const CUtensorMap* mw = rf_map<T>(s, b.L, b.f[RF_W], false);
-        if (mx && mp && mr && mw) {
-            const RfUMaps m{*mx, *mp, *mr, *mw};
+        if (mx && mp0 && mp1 && mr && mw) {
+            const RfUMaps m{*mx, {*mp0, *mp1}, *mr, *mw};
             constexpr size_t smem = rf_u_tma_bytes<T>();
             static unsigned attr_set = 0;
             if (!(attr_set & (1u << (s->device & 31)))) {
@@ -216,34 +221,34 @@ void rf_ur(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, const
                                              (int)smem));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, name, (k_rf_ur_tma<T><<<gl, BX, smem, s->stream>>>(b.L, b.st, m, b.f[RF_XS], r, s->rs, fin,
-                                                                           s->d_mirror + kTmaErrWord2)));
+            TL_LAUNCH(s, name, (k_rf_ur_tma<T><<<gl, BX, smem, s->stream>>>(b.L, b.st, m, b.f[RF_XS], b.f[RF_R],
+                                                                           s->rs, fin, s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
-    TL_LAUNCH(s, name, (k_rf_ur<T><<<gl, BX, 0, s->stream>>>(b.L, b.st, b.f[RF_XS], p, r, b.f[RF_W], s->rs, fin)));
+    TL_LAUNCH(s, name, (k_rf_ur<T><<<gl, BX, 0, s->stream>>>(b.L, b.st, b.f[RF_XS], b.f[RF_P0], b.f[RF_P1], b.f[RF_R],
+                                                              b.f[RF_W], s->rs, fin)));
 }
 
-// Launches trips t = 0.. in batches of kBatch, looking at the mapped done word
-// of the previous batch while the current one runs (as driver2d.cu).
-template <typename F>
-void batched(TlSuite2D* s, int max_trips, F&& launch_trip)
+// Launches groups of up to kGroup trips, each followed by `update`, looking at
+// the mapped done word of the previous group while the current one runs (as
+// driver2d.cu). Every group runs at least one trip until the solve has ended,
+// so max_trips groups reach it; a group has no more trips than are allowed.
+template <typename F, typename U>
+void batched(TlSuite2D* s, int max_trips, F&& launch_trip, U&& update)
 {
     cudaEvent_t ev[2];
     cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
     cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming);
-    int t = 0, batch = 0;
-    bool pending_prev = false;
-    while (t < max_trips && !tl::failed()) {
-        const int end = std::min(max_trips, t + kBatch);
-        for (; t < end; ++t) launch_trip(t);
-        cudaEventRecord(ev[batch & 1], s->stream);
-        if (pending_prev) {
-            cudaEventSynchronize(ev[(batch + 1) & 1]);
+    int t = 0;
+    for (int group = 0; group < max_trips && !tl::failed(); ++group) {
+        for (int q = 0; q < std::min(kGroup, max_trips); ++q) launch_trip(t++);
+        update();
+        cudaEventRecord(ev[group & 1], s->stream);
+        if (group > 0) {
+            cudaEventSynchronize(ev[(group + 1) & 1]);
             if (*(volatile int*)&s->h_mirror[0]) break;
         }
-        pending_prev = true;
-        ++batch;
     }
     cudaStreamSynchronize(s->stream);
     cudaEventDestroy(ev[0]);
@@ -280,16 +285,11 @@ int solve_refined(TlSuite2D* s, Chunk* chunk, int max_iters, double rel_tol, int
                             s->g.x, s->g.hd, L, chunk->r, chunk->u0, chunk->kx, chunk->ky, b.f[RF_KX], b.f[RF_KY], b.f[RF_R],
                             b.f[RF_P0], b.f[RF_P1], b.f[RF_W], b.f[RF_XS], s->rs,
                             FinMxInit{b.st, rel_tol * rel_tol, 0.0, max_iters, s->d_mirror})));
-    T* pb[2] = {b.f[RF_P0], b.f[RF_P1]};
-    int cur = 0;
     batched(s, max_iters, [&](int t) {
-        if (t == 0) {
-            rf_w<T, false>(s, b, gl, nm[1], pb[cur], pb[cur], b.f[RF_R], FinMxW{b.st});
-        } else {
-            rf_w<T, true>(s, b, gl, nm[1], pb[cur], pb[cur ^ 1], b.f[RF_R], FinMxW{b.st});
-            cur ^= 1;
-        }
-        rf_ur<T>(s, b, gl, nm[2], pb[cur], b.f[RF_R], FinMxUr{b.st, s->d_mirror});
+        if (t == 0) rf_w<T, false>(s, b, gl, nm[1], b.f[RF_R], FinMxW{b.st});
+        else rf_w<T, true>(s, b, gl, nm[1], b.f[RF_R], FinMxW{b.st});
+        rf_ur<T>(s, b, gl, nm[2], FinMxUr{b.st, s->d_mirror});
+    }, [&] {
         TL_LAUNCH(s, nm[3], (k_rf_fold<T><<<gl, BX, 0, s->stream>>>(L, b.st, s->g.x, s->g.hd, chunk->u,
                                                                      b.f[RF_XS])));
         TL_LAUNCH(s, nm[4], (k_rf_resid<T><<<gl, BX, 0, s->stream>>>(L, b.st, s->g.x, s->g.hd, chunk->u,
@@ -351,12 +351,10 @@ int solve_refined_ppcg(TlSuite2D* s, Chunk* chunk, Settings* settings, double re
                             s->g.x, s->g.hd, L, chunk->r, chunk->u0, chunk->kx, chunk->ky, b.f[RF_KX], b.f[RF_KY],
                             b.f[RF_R], b.f[RF_P0], b.f[RF_P1], b.f[RF_W], b.f[RF_XS], s->rs,
                             FinMxInit{b.st, rel_tol * rel_tol, 0.0, max_iters, s->d_mirror})));
-    T* pb[2] = {b.f[RF_P0], b.f[RF_P1]};
     T* sb[2] = {b.f[RF_SD0], b.f[RF_SD1]};
     T* qb[2] = {b.f[RF_S0], b.f[RF_S1]};
     T* const r = b.f[RF_R];
     T* const z = b.f[RF_Z];
-    int cur = 0;
     auto fold_resid = [&](double* betas) {
         TL_LAUNCH(s, nm[3], (k_rf_fold<T><<<gl, BX, 0, s->stream>>>(L, b.st, s->g.x, s->g.hd, chunk->u,
                                                                      b.f[RF_XS])));
@@ -364,23 +362,15 @@ int solve_refined_ppcg(TlSuite2D* s, Chunk* chunk, Settings* settings, double re
                                                                       chunk->u0, chunk->kx, chunk->ky, r, s->rs,
                                                                       FinMxRes{b.st, s->d_mirror, betas})));
     };
-    auto w_sweep = [&](int t, double* alphas) {
-        if (t == 0) {
-            rf_w<T, false>(s, b, gl, nm[1], pb[cur], pb[cur], r, FinMxW{b.st, alphas});
-        } else {
-            rf_w<T, true>(s, b, gl, nm[1], pb[cur], pb[cur ^ 1], r, FinMxW{b.st, alphas});
-            cur ^= 1;
-        }
-    };
     // CG trips up to the switch (2d/shared.h:41-42 for the constants)
     const FinMxUr cg_fin = settings->error_switch
                                ? FinMxUr{b.st, s->d_mirror, s->d_cg_betas, 20, settings->eps_lim}
                                : FinMxUr{b.st, s->d_mirror, s->d_cg_betas, settings->presteps, 1.0};
     batched(s, max_iters, [&](int t) {
-        w_sweep(t, s->d_cg_alphas);
-        rf_ur<T>(s, b, gl, nm[2], pb[cur], r, cg_fin);
-        fold_resid(s->d_cg_betas);
-    });
+        if (t == 0) rf_w<T, false>(s, b, gl, nm[1], r, FinMxW{b.st, s->d_cg_alphas});
+        else rf_w<T, true>(s, b, gl, nm[1], r, FinMxW{b.st, s->d_cg_alphas});
+        rf_ur<T>(s, b, gl, nm[2], cg_fin);
+    }, [&] { fold_resid(s->d_cg_betas); });
     MxState st{};
     TL_CUDA(cudaMemcpy(&st, b.st, sizeof(MxState), cudaMemcpyDeviceToHost));
     *cg_trips = st.trip;
@@ -440,11 +430,9 @@ int solve_refined_ppcg(TlSuite2D* s, Chunk* chunk, Settings* settings, double re
                                         L, b.st, theta, ca, cb, ni - 1, sb[c], qb[c], z, r, s->rs, FinPcgZ{b.st})));
             }
             // p = z + beta p, w = A p, alpha = r.z / p.w
-            rf_w<T, true>(s, b, gl, nm[1], pb[cur], pb[cur ^ 1], z, FinMxW{b.st, nullptr, true});
-            cur ^= 1;
-            rf_ur<T>(s, b, gl, nm[2], pb[cur], r, FinMxUr{b.st, s->d_mirror});
-            fold_resid(nullptr);
-        });
+            rf_w<T, true>(s, b, gl, nm[1], z, FinMxW{b.st, nullptr, true});
+            rf_ur<T>(s, b, gl, nm[2], FinMxUr{b.st, s->d_mirror});
+        }, [&] { fold_resid(nullptr); });
         TL_CUDA(cudaMemcpy(&st, b.st, sizeof(MxState), cudaMemcpyDeviceToHost));
     }
     *updates = st.updates;

@@ -50,7 +50,12 @@ struct MxState {
 };
 
 __device__ __forceinline__ int vol_read(const int* p) { return *(volatile const int*)p; }
-__device__ __forceinline__ bool mx_idle(const MxState* st) { return vol_read(&st->done) != 0; }
+// The sweeps of a trip run unless the solve has ended or waits for a residual
+// replacement (the rest of the trips launched with the one that asked for it).
+__device__ __forceinline__ bool mx_idle(const MxState* st)
+{
+    return vol_read(&st->done) != 0 || vol_read(&st->upd) != 0;
+}
 __device__ __forceinline__ bool mx_no_update(const MxState* st)
 {
     return vol_read(&st->done) != 0 || vol_read(&st->upd) == 0;

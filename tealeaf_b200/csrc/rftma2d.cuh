@@ -64,12 +64,12 @@ struct RfRowsU {
 };
 
 // Maps of the w sweep: tile rows (W x kRfRows) of p, r, kx, ky and ring
-// boxes (H x kRfRows) of p, r, kx.
+// boxes (H x kRfRows) of p, r, kx; both p buffers (trip t writes buffer t & 1).
 struct RfWMaps {
-    CUtensorMap p, r, kx, ky, ph, rh, kxh;
+    CUtensorMap p[2], r, kx, ky, ph[2], rh, kxh;
 };
 struct RfUMaps {
-    CUtensorMap xs, p, r, w;
+    CUtensorMap xs, p[2], r, w;
 };
 
 template <typename T>
@@ -88,13 +88,15 @@ constexpr size_t rf_u_tma_bytes()
 // upper neighbours are in stages b and b+1.
 template <typename T, bool FUSE_P>
 __global__ void __launch_bounds__(BX, 4) k_rf_w_tma(Lay L, const MxState* __restrict__ st,
-                                                    const __grid_constant__ RfWMaps m, T* __restrict__ p_out,
+                                                    const __grid_constant__ RfWMaps m, T* p0, T* p1,
                                                     T* __restrict__ w, ReduceSlots rs, FinMxW fin, int* err)
 {
     extern __shared__ __align__(128) unsigned char rw_raw[];
     using S = RfRowsW<T>;
     constexpr int N = Pack<T>::N, W = S::W, H = S::H;
     if (mx_idle(st)) return;
+    const int par = st->trip & 1, in = FUSE_P ? par ^ 1 : par;
+    T* const p_out = par ? p1 : p0;
     unsigned char* base = rw_raw + ((128 - (tl::smem_addr(rw_raw) & 127)) & 127);
     S* ring = reinterpret_cast<S*>(base);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kRfStages * sizeof(S));
@@ -109,9 +111,9 @@ __global__ void __launch_bounds__(BX, 4) k_rf_w_tma(Lay L, const MxState* __rest
         unsigned long long* bar = &bars[b % kRfStages];
         const int y0 = s.j0 + b * kRfRows;
         tl::mbar_expect_tx(bar, kMain * (FUSE_P ? 4u : 3u) + kRing * (FUSE_P ? 5u : 3u));
-        tl::tma_load_3d(&Q.P[0][0], &m.p, cb, y0, 0, bar);
-        tl::tma_load_3d(&Q.PL[0][0], &m.ph, cb - H, y0, 0, bar);
-        tl::tma_load_3d(&Q.PR[0][0], &m.ph, cb + W, y0, 0, bar);
+        tl::tma_load_3d(&Q.P[0][0], &m.p[in], cb, y0, 0, bar);
+        tl::tma_load_3d(&Q.PL[0][0], &m.ph[in], cb - H, y0, 0, bar);
+        tl::tma_load_3d(&Q.PR[0][0], &m.ph[in], cb + W, y0, 0, bar);
         if (FUSE_P) {
             tl::tma_load_3d(&Q.R[0][0], &m.r, cb, y0, 0, bar);
             tl::tma_load_3d(&Q.RL[0][0], &m.rh, cb - H, y0, 0, bar);
@@ -221,6 +223,7 @@ __global__ void __launch_bounds__(BX, 4) k_rf_ur_tma(Lay L, const MxState* __res
     using S = RfRowsU<T>;
     constexpr int N = Pack<T>::N, W = S::W;
     if (mx_idle(st)) return;
+    const int par = st->trip & 1;
     unsigned char* base = ru_raw + ((128 - (tl::smem_addr(ru_raw) & 127)) & 127);
     S* ring = reinterpret_cast<S*>(base);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kRfStagesU * sizeof(S));
@@ -234,7 +237,7 @@ __global__ void __launch_bounds__(BX, 4) k_rf_ur_tma(Lay L, const MxState* __res
         const int y0 = s.j0 + 1 + b * kRfRows;
         tl::mbar_expect_tx(bar, 4u * sizeof(T) * kRfRows * W);
         tl::tma_load_3d(&Q.X[0][0], &m.xs, cb, y0, 0, bar);
-        tl::tma_load_3d(&Q.P[0][0], &m.p, cb, y0, 0, bar);
+        tl::tma_load_3d(&Q.P[0][0], &m.p[par], cb, y0, 0, bar);
         tl::tma_load_3d(&Q.R[0][0], &m.r, cb, y0, 0, bar);
         tl::tma_load_3d(&Q.Wv[0][0], &m.w, cb, y0, 0, bar);
     };
