@@ -139,7 +139,7 @@ struct Run {
     // pending). Closes the phase: last p update and the halo of u and p.
     DevState cg_phase(int from, bool fresh)
     {
-        if (from == 0 && fresh && s->chip_words && prm.max_iters > 0) return cg_close(cg_chip(), chunk->r);
+        if (from == 0 && fresh && s->chip_words && prm.max_iters > 0) return cg_close(cg_chip<0>(s->g, nullptr), chunk->r);
         FinCgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
         const Scalar alpha{0.0, &s->d_state->alpha};
         return cg_trips(from, fresh, chunk->r, [&](double* p) {
@@ -148,35 +148,40 @@ struct Run {
     }
 
     // The whole loop in one launch (k_cg_chip) for a mesh whose state fits on
-    // the SMs; its strip pairs spread over as many SMs as there are.
-    DevState cg_chip()
+    // the SMs, in strips of g.rows rows; its strip pairs spread over as many
+    // SMs as there are. BS, z: the preconditioned CG's block and field.
+    template <int BS>
+    DevState cg_chip(Geo g, double* z)
     {
-        const int pairs = gi.x * tl::ceil_div(gi.y, 2);
-        ChipArgs a{chunk->p, chunk->r, chunk->u, chunk->w, chunk->kx, chunk->ky, s->chip_words, s->chip_tag,
-                    (int)gi.x, (int)gi.y, tl::ceil_div(pairs, s->sm_count), s->d_state, s->d_cg_alphas, s->d_cg_betas,
-                   prm, s->d_mirror, s->chip_err, s->d_mirror + kTmaErrWord2};
+        const dim3 grid = interior_grid(g);
+        const int pairs = chip_pairs(g, s->sm_count);
+        ChipArgs a{chunk->p, chunk->r, chunk->u, chunk->w, z, chunk->kx, chunk->ky, chunk->mi, s->chip_words,
+                   s->chip_tag, (int)grid.x, (int)grid.y, tl::ceil_div(pairs, s->sm_count), s->d_state,
+                   s->d_cg_alphas, s->d_cg_betas, prm, s->d_mirror, s->chip_err, s->d_mirror + kTmaErrWord2};
         s->chip_tag += (unsigned long long)prm.max_iters;
-        switch (s->g.rows) {
-            case 2: launch_chip<2>(a, pairs); break;
-            case 3: launch_chip<3>(a, pairs); break;
-            case 4: launch_chip<4>(a, pairs); break;
-            case 5: launch_chip<5>(a, pairs); break;
-            case 6: launch_chip<6>(a, pairs); break;
-            case 7: launch_chip<7>(a, pairs); break;
-            default: launch_chip<kChipRows>(a, pairs); break;
+        switch (g.rows) {
+            case 2: launch_chip<2, BS>(g, a, pairs); break;
+            case 3: launch_chip<3, BS>(g, a, pairs); break;
+            case 4: launch_chip<4, BS>(g, a, pairs); break;
+            case 5: launch_chip<5, BS>(g, a, pairs); break;
+            case 6: launch_chip<6, BS>(g, a, pairs); break;
+            case 7: launch_chip<7, BS>(g, a, pairs); break;
+            default: launch_chip<kChipRows, BS>(g, a, pairs); break;
         }
         return read_state();
     }
-    template <int H>
-    void launch_chip(ChipArgs& a, int pairs)
+    template <int H, int BS>
+    void launch_chip(Geo& g, ChipArgs& a, int pairs)
     {
-        const int threads = a.groups * BX;
-        constexpr size_t smem = ChipPlace<H>::bytes;
-        TL_CUDA(cudaFuncSetAttribute(k_cg_chip<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        void* args[] = {&s->g, &a};
-        TL_LAUNCH(s, "k_cg_chip", TL_CUDA(cudaLaunchCooperativeKernel((const void*)k_cg_chip<H>,
-                                                                      dim3(tl::ceil_div(pairs, a.groups)),
-                                                                      dim3(threads), args, smem, s->stream)));
+        if constexpr (BS == 0 || H % BS == 0) {
+            const int threads = a.groups * BX;
+            constexpr size_t smem = ChipPlace<H, BS>::bytes;
+            TL_CUDA(cudaFuncSetAttribute(k_cg_chip<H, BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            void* args[] = {&g, &a};
+            TL_LAUNCH(s, "k_cg_chip", TL_CUDA(cudaLaunchCooperativeKernel((const void*)k_cg_chip<H, BS>,
+                                                                          dim3(tl::ceil_div(pairs, a.groups)),
+                                                                          dim3(threads), args, smem, s->stream)));
+        }
     }
 
     // The CG loop with `fold` the field of the p update p = beta p + fold (r
@@ -244,6 +249,8 @@ struct Run {
                                        gb, fc, chunk->r, chunk->kx, chunk->ky, chunk->mi, z, chunk->p, s->rs,
                                        FinCgInit{s->d_state, s->d_mirror})));
         read_state();
+        if (s->chip_words && chip_pairs(gb, s->sm_count) > 0 && prm.max_iters > 0)
+            return cg_close(cg_chip<BS>(gb, z), z);
         FinPcgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
         const Scalar alpha{0.0, &s->d_state->alpha};
         if (tma_usable(s)) {

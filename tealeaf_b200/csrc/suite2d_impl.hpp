@@ -168,9 +168,9 @@ inline int chip_pairs(const Geo& g, int sm_count)
     const long pairs = (long)d.x * tl::ceil_div(d.y, 2);
     return g.rows <= kChipRows && pairs <= (long)kChipPairs * sm_count ? (int)pairs : 0;
 }
-// Words of one pair: its two strips' sums, twice; 4 warps' 32 side cells; 2
-// rows of BX edge cells.
-constexpr int kChipWords = 4 + 4 * 32 + 2 * BX;
+// Words of one pair: its two strips' sums, three of them; 4 warps' 32 side
+// cells; 2 rows of BX edge cells.
+constexpr int kChipWords = 6 + 4 * 32 + 2 * BX;
 // Waits for the stream and returns the published sums.
 bool fetch(TlSuite2D* s, int n, double* out);
 // Runs every pending operation (p update, then halo updates).

@@ -57,3 +57,28 @@ def test_chip_cg_two_chunks_in_turn():
     finally:
         for h in (a, b, c, d):
             h.finalise()
+
+
+@pytest.mark.parametrize("pc", ["jac_diag", "jac_block"])
+@pytest.mark.parametrize("cells,cap", [
+    ((5, 3), 20000), ((33, 7), 20000), ((129, 38), 20000), ((1024, 442), 25), ((641, 941), 25), ((1000, 702), 25),
+    ((900, 880), 25), ((1025, 900), 25), ((1000, 1181), 25),
+])
+def test_chip_pcg_against_the_oracle(cells, cap, pc, oracle_lib):
+    """The preconditioned loop on chip: trip counts as the oracle's, the
+    summary within 1e-12 of its."""
+    from tealeaf_b200.config import read_config
+    text = problems.seeded(2, cells, 11, 4, 2, solver="cg", end_step=1, max_iters=cap, preconditioner=pc,
+                           name="chip").tea_in()
+    cfg, states = read_config(text, 2)
+    want = oracle_lib.run(cfg, states)[0]
+    h = Host(text, 2)
+    try:
+        n0 = h.lib.tl2d_launch_count(C.byref(h.chunk))
+        got = h.solve_device(0)
+        assert h.lib.tl2d_launch_count(C.byref(h.chunk)) - n0 <= 18
+        assert got.iterations == want.iterations
+        for x, y in zip(got.summary, want.summary):
+            assert abs(x - y) <= 1e-12 * abs(y)
+    finally:
+        h.finalise()
