@@ -6,7 +6,7 @@
 // local 7-point updates with no global reduction, so L of them (L <= kTB3)
 // run in one launch. A block owns an x-y region of kRX x kRY columns (the
 // tile of kTX3 x kTY3 columns plus a kTB3-column margin) and a segment of
-// kBZ3 z-planes, and streams up z as a wavefront: at step s the region's
+// z-planes (Blocked3Args::planes), and streams up z as a wavefront: at step s the region's
 // plane s is loaded (level 0), and level l (1 <= l <= L) advances plane
 // s - l by one step, so every plane passes through all L steps while only a
 // few planes per level are live. Each thread owns one column (x, y) and
@@ -36,6 +36,7 @@
 
 #include "kernels3d.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace tl3d {
@@ -49,10 +50,6 @@ constexpr int kB3Threads = kRX * kRY;    // 512
 constexpr int kTB3 = TL3D_TB;            // margin: the most steps one launch takes
 constexpr int kTX3 = kRX - 2 * kTB3;     // tile columns
 constexpr int kTY3 = kRY - 2 * kTB3;     // tile rows
-#ifndef TL3D_BZ
-#define TL3D_BZ 64
-#endif
-constexpr int kBZ3 = TL3D_BZ;            // output planes per block
 static_assert(kTX3 > 0 && kTY3 > 0, "the margin must leave a tile");
 
 struct Blocked3Args {
@@ -64,6 +61,7 @@ struct Blocked3Args {
     const double* betas;
     int add_end = 0;      // Chebyshev: each trip ends with its u += p (the kernel-interface calls' order)
                           // instead of starting with the previous trip's
+    int planes = 0;       // output planes per block, set by the launch (blocked3_planes)
 };
 
 template <int MODE>
@@ -93,7 +91,7 @@ static __global__ void __launch_bounds__(kB3Threads, 1) k3_blocked(Geo g, Blocke
     const int my = max(max(kTB3 - cy, cy - (kTB3 + kTY3 - 1)), 0);
     const bool in_tile = colin && mx == 0 && my == 0;
     const bool at_l = gx == ilo, at_r = gx == ihi - 1, at_b = gy == jlo, at_t = gy == jhi - 1;
-    const int Z0 = zlo + blockIdx.z * kBZ3, Z1 = min(Z0 + kBZ3, zhi);   // output planes [Z0, Z1)
+    const int Z0 = zlo + blockIdx.z * a.planes, Z1 = min(Z0 + a.planes, zhi);   // output planes [Z0, Z1)
     const long col = gx + (long)gy * x;   // index of (gx, gy) in plane 0 (used only when colin)
 
     // per level l < kTB3: stencil field of planes z-1, z, z+1 around the plane
@@ -312,7 +310,7 @@ static __global__ void __launch_bounds__(kB3TThreads, 1) k3_blocked_tma(Geo g, B
         at_t[k] = gy == jhi - 1;
         col[k] = gx + (long)gy * x;
     }
-    const int Z0 = zlo + blockIdx.z * kBZ3, Z1 = min(Z0 + kBZ3, zhi);
+    const int Z0 = zlo + blockIdx.z * a.planes, Z1 = min(Z0 + a.planes, zhi);
 
     // per level l < kTB3 and row k: stencil field of the three planes around
     // the plane level l + 1 advances next; B of that plane (bp) and the newest (bn)
@@ -509,12 +507,6 @@ static __global__ void __launch_bounds__(kB3TThreads, 1) k3_blocked_tma(Geo g, B
     // every issued plane was waited for (planes s_begin .. load_end - 1 at their steps)
 }
 
-inline dim3 blocked3_tma_grid(const Geo& g)
-{
-    return dim3(tl::ceil_div(g.x - 2 * g.hd, kTX3), tl::ceil_div(g.y - 2 * g.hd, kTYT3),
-                tl::ceil_div(g.z - 2 * g.hd, kBZ3));
-}
-
 // sum(b^2) over the interior with the partition and order of the one-step
 // fused sweeps (k3_cheby_trip, k3_ppcg_step: grid gh, the halo-duty z-plane
 // of blocks adding nothing), then `fin`; skipped once the loop has ended.
@@ -544,10 +536,34 @@ static __global__ void k3_finish_only(const int* __restrict__ done, Finish fin)
     fin(t);
 }
 
-inline dim3 blocked3_grid(const Geo& g)
+// Output planes per block for `tiles` x-y tiles: one block of either kernel
+// fits an SM, so a launch takes waves x (planes + the 2 kTB3 planes beyond the
+// segment + about 6 steps' worth of start and ring fill); the segment length
+// with the least of that. At most 64 planes: beyond, at 256^3, one wave of 130
+// blocks of 256 planes measured 40.0 ms for 200 trips against 37.9 for four
+// waves of 64. With 64 at every size, a 130 x 97 x 110 mesh of 25 tiles had 50
+// blocks on 148 SMs: 10.3 ms against 5.5, 64^3 9.3 against 2.6.
+constexpr int kMaxPlanes3 = 64;
+inline int blocked3_planes(int nz, long tiles, int sm_count)
 {
-    return dim3(tl::ceil_div(g.x - 2 * g.hd, kTX3), tl::ceil_div(g.y - 2 * g.hd, kTY3),
-                tl::ceil_div(g.z - 2 * g.hd, kBZ3));
+    int best = std::min(nz, kMaxPlanes3);
+    long least = -1;
+    for (int planes = best; planes >= 1; --planes) {
+        const long waves = tl::ceil_div(tiles * tl::ceil_div(nz, planes), sm_count);
+        const long cost = waves * (planes + 2 * kTB3 + 6);
+        if (least < 0 || cost < least) {
+            least = cost;
+            best = planes;
+        }
+    }
+    return best;
+}
+// Blocks of a launch over tiles of tx x ty columns; sets the segment length.
+inline dim3 blocked3_grid(const Geo& g, int tx, int ty, int sm_count, int& planes)
+{
+    const int bx = tl::ceil_div(g.x - 2 * g.hd, tx), by = tl::ceil_div(g.y - 2 * g.hd, ty), nz = g.z - 2 * g.hd;
+    planes = blocked3_planes(nz, (long)bx * by, sm_count);
+    return dim3(bx, by, tl::ceil_div(nz, planes));
 }
 
 }  // namespace tl3d

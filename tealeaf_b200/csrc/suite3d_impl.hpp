@@ -158,7 +158,7 @@ inline bool tma_failed(const TlSuite3D* s) { return s->h_mirror && s->h_mirror[k
 // boundaries (even halo depth, margin and row length), else per-thread
 // loads; the same results either way. Internal linkage, like the kernels.
 template <int MODE, int HS>
-static void launch_blocked3_tma(TlSuite3D* s, const char* name, const Blocked3Args& a, const Blocked3Maps& m,
+static void launch_blocked3_tma(TlSuite3D* s, const char* name, Blocked3Args a, const Blocked3Maps& m,
                                 double* A_out, double* B_out, double* u, double* w, double* r, const int* done)
 {
     static unsigned set = 0;   // devices on which the shared-memory size was raised
@@ -167,13 +167,14 @@ static void launch_blocked3_tma(TlSuite3D* s, const char* name, const Blocked3Ar
                                      (int)kBlocked3TmaBytes));
         set |= 1u << (s->device & 31);
     }
-    TL3_LAUNCH(s, name, (k3_blocked_tma<MODE, HS><<<blocked3_tma_grid(s->g), dim3(kRX, kTYT), kBlocked3TmaBytes,
+    const dim3 grid = blocked3_grid(s->g, kTX3, kTYT3, s->sm_count, a.planes);
+    TL3_LAUNCH(s, name, (k3_blocked_tma<MODE, HS><<<grid, dim3(kRX, kTYT), kBlocked3TmaBytes,
                                                     s->stream>>>(s->g, a, m, A_out, B_out, u, w, r, done,
                                                                  s->d_mirror + kTmaErrWord)));
 }
 
 template <int MODE>
-static void launch_blocked3(TlSuite3D* s, Chunk* chunk, const Blocked3Args& a, const double* A_in,
+static void launch_blocked3(TlSuite3D* s, Chunk* chunk, Blocked3Args a, const double* A_in,
                             const double* B_in, double* A_out, double* B_out, const double* u0, double* u, double* w,
                             double* r, const int* done)
 {
@@ -192,7 +193,8 @@ static void launch_blocked3(TlSuite3D* s, Chunk* chunk, const Blocked3Args& a, c
             return;
         }
     }
-    TL3_LAUNCH(s, name, (k3_blocked<MODE><<<blocked3_grid(s->g), dim3(kRX, kRY), 0, s->stream>>>(
+    const dim3 grid = blocked3_grid(s->g, kTX3, kTY3, s->sm_count, a.planes);
+    TL3_LAUNCH(s, name, (k3_blocked<MODE><<<grid, dim3(kRX, kRY), 0, s->stream>>>(
                             s->g, a, A_in, B_in, A_out, B_out, u0, u, w, r, chunk->vec_kx, chunk->vec_ky,
                             chunk->vec_kz, done)));
 }
