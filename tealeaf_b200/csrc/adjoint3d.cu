@@ -28,6 +28,7 @@
 // field summary's temperature restricted to a box (3d/c_kernels/omp3/
 // field_summary.c:8-49: sum of volume * density * u over cells whose centre
 // lies in the box), and the result is dJ/d(log rho) = rho dJ/drho per cell.
+#include "cgchip3d.cuh"
 #include "suite3d_impl.hpp"
 
 #include <algorithm>
@@ -186,6 +187,12 @@ int adjoint_solve(TlSuite3D* s, Chunk* chunk, const double* rhs, double* lam, do
     DevParams prm{};
     prm.eps = rel_tol * rel_tol * gg;
     prm.max_iters = max_iters;
+    if (cg_chip3(s, chunk, lam, prm)) {
+        DevState st{};
+        TL_CUDA(cudaMemcpyAsync(&st, s->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
+        TL_CUDA(cudaStreamSynchronize(s->stream));
+        return st.trip;
+    }
     double* buf[2] = {chunk->vec_p, s->alt[ALT3_P]};
     tl::FinCgW fin_w{s->d_state, s->d_cg_alphas};
     tl::FinCgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};

@@ -81,13 +81,13 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
 {
     extern __shared__ double chip_smem_raw[];
     constexpr int NV = BS ? 2 : 1;   // sums of the second sweep
-    __shared__ tl::StripSumSmem<NV> sums;
+    __shared__ tl::StripSumSmem<2, NV> sums;
     __shared__ double side[kChipWarps][32];   // per warp: rows 0 .. left, 16 .. right of its columns
     using P = ChipPlace<H, BS>;
     constexpr int R = P::R;
     constexpr bool kRegK = P::kRegK, kRegU = P::kRegU, kDiag = P::kDiag;
     static_assert(BS == 0 || H % BS == 0, "a strip holds whole blocks of M");
-    static_assert(P::bytes + sizeof(tl::StripSumSmem<NV>) + sizeof(double) * kChipWarps * 32 <= 227 * 1024,
+    static_assert(P::bytes + sizeof(tl::StripSumSmem<2, NV>) + sizeof(double) * kChipWarps * 32 <= 227 * 1024,
                   "shared memory of a block");
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -148,7 +148,7 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
             kyv[kRegK ? q : 0] = kyc;
         } else {
             if (kDiag) KD[q * kChipT] = kd;
-            KX[q * P::KXW] = kxc;
+            KX[q * P::KXW] = a.kx[i + (k > kk ? 1 : 0)];   // (past the interior: its right face)
             if (lane == 31) KX[q * P::KXW + 1] = a.kx[i + 1];
             KY[q * kChipT] = kyc;
         }
@@ -291,7 +291,7 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
         if (full) sweep_w(std::true_type(), aw[0]);
         else sweep_w(std::false_type(), aw[0]);
         if (!active) aw[0][0] = aw[0][1] = 0.0;
-        ok = tl::strip_sum<1>(aw, has ? pair : -1, strips, 2 * pairs, sums, a.words, tag, a.err, [] {},
+        ok = tl::strip_sum<BX, 2, 1>(aw, has ? pair : -1, strips, 2 * pairs, sums, a.words, tag, a.err, [] {},
                               [&](const double* t) { return rro / t[0]; }, pw, alpha);
         if (!ok) break;
         double ar[NV][2] = {};
@@ -317,7 +317,7 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
             }
             tl::word_store(a.words + row_w + BX, top, tag);
         }
-        ok = tl::strip_sum<NV>(ar, has ? pair : -1, strips, 2 * pairs, sums, a.words + 2 * pairs, tag, a.err,
+        ok = tl::strip_sum<BX, 2, NV>(ar, has ? pair : -1, strips, 2 * pairs, sums, a.words + 2 * pairs, tag, a.err,
                                [&] {
 #pragma unroll
                                    for (int q = 0; q < R; ++q) {

@@ -9,6 +9,7 @@
 // (3d/drivers/cheby_solver_driver.c:70-71). Jacobi is driven from the host
 // through the suite's own kernel-interface entry points.
 #include "blocked3d.cuh"
+#include "cgchip3d.cuh"
 #include "host_maths.hpp"
 #include "suite3d_impl.hpp"
 
@@ -135,6 +136,7 @@ struct Run3 {
     // cg_solver_main_step_driver trips until the loop ends; closes the phase.
     DevState cg_phase(int from, bool fresh)
     {
+        if (from == 0 && fresh && cg_chip3(s, chunk, chunk->vec_u, prm)) return cg_close(read_state());
         double* buf[2] = {chunk->vec_p, s->alt[ALT3_P]};
         tl::FinCgW fin_w{s->d_state, s->d_cg_alphas};
         tl::FinCgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
@@ -155,6 +157,14 @@ struct Run3 {
         const int ran = st.trip - from;
         const int flips = fresh ? std::max(0, ran - 1) : ran;
         if (buf[flips & 1] != chunk->vec_p) swap_alt(s, chunk, ALT3_P);
+        return cg_close(st);
+    }
+
+    // Closes a CG phase that ended in state st: the last p update, the halos
+    // of p and u, and the host's coefficients.
+    DevState cg_close(const DevState& st)
+    {
+        const Scalar beta{0.0, &s->d_state->beta};
         TL3_LAUNCH(s, "k3_cg_close", k3_cg_close<<<gi, bl, 0, s->stream>>>(s->g, fc, beta, 1, chunk->vec_p,
                                                                             chunk->vec_r, chunk->vec_u));
         if (st.trip > 0) {

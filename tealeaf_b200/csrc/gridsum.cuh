@@ -69,53 +69,62 @@ static __device__ __noinline__ double word_wait(const TagWord* s, unsigned long 
     return v;
 }
 
-// Shared memory of strip_sum for up to NV sums at once; `bad` starts at 0.
-constexpr int kStripMax = 1280;   // strips of a mesh: 10 per thread of the final pass
-template <int NV>
+// Shared memory of strip_sum for up to NV sums of up to NH strips at once;
+// `bad` starts at 0.
+constexpr int kStripMax = 1280;   // strips of a mesh
+// Words a group of NH strips has per sum: whole sectors.
+constexpr int strip_words(int nh) { return (nh + 1) / 2 * 2; }
+template <int NH, int NV>
 struct StripSumSmem {
     double vals[NV][kStripMax];
     short strip_of[3 * 512];   // the strip whose sums each word holds (negative: none)
-    double warp[NV][2][16];    // warp sums of this block's strips
-    double fin[NV][4];         // warp sums of the final pass
+    double warp[NV][NH][16];   // warp sums of this block's strips
+    double fin[NV][8];         // warp sums of the final pass
     double out[NV + 1];
     int bad;
 };
 
-// NV sums over the whole grid of the strips' values. A group of 128 threads
-// (one of up to four in the block) holds values v[.][h] per thread for each
-// of two strips and hands their sums over in words 2 pair and 2 pair + 1 of
-// the `words` words of each sum (pair negative: the group has none);
-// sm.strip_of says which strip each word belongs to, of at most three words
-// per thread of a block. The same tree as tl::grid_sum<NV, 128> over blocks of
-// 128 threads, bit for bit: warp shuffles, the four warps as (0 + 2) + (1 +
-// 3), then thread t < 128 adds the sums of strips t, t + 128, ... in turn and
-// the 128 results go through the same tree. `between` runs after the block's
-// words are stored, before the wait. `scalar(totals)` runs in four warps;
-// every thread gets the totals and its value. False when a wait gave up.
-template <int NV, int NS, typename Between, typename Scalar_>
-__device__ __forceinline__ bool strip_sum(double (&v)[NV][2], int pair, int strips, int words, StripSumSmem<NS>& sm,
-                                          TagWord* slots, unsigned long long tag, int* err, Between between,
-                                          Scalar_ scalar, double (&total)[NV], double& derived)
+// The values of NT / 32 warps in the order of tl::block_sum's second stage.
+template <int NT>
+__device__ __forceinline__ double warps_sum(const double* q)
+{
+    static_assert(NT == 128 || NT == 256, "four or eight warps");
+    if (NT == 128) return (q[0] + q[2]) + (q[1] + q[3]);
+    return ((q[0] + q[4]) + (q[2] + q[6])) + ((q[1] + q[5]) + (q[3] + q[7]));
+}
+
+// NV sums over the whole grid of the strips' values. A group of NT threads
+// (blocks have up to 512) holds values v[.][h] per thread for each of NH
+// strips and hands their sums over in the first of words strip_words(NH) unit
+// .. of the `words` words of each sum (unit, the group's number in the grid;
+// negative: it has no strips); sm.strip_of says which strip each word belongs to, of at
+// most three words per thread of a block. The same tree as tl::grid_sum<NV,
+// NT> over blocks of NT threads, bit for bit: warp shuffles, the block's warps,
+// then thread t < NT adds the sums of strips t, t + NT, ... in turn and the NT
+// results go through the same tree. `between` runs after the block's words
+// are stored, before the wait. `scalar(totals)` runs in NT threads; every
+// thread gets the totals and its value. False when a wait gave up.
+template <int NT, int NH, int NV, int NS, typename Between, typename Scalar_>
+__device__ __forceinline__ bool strip_sum(double (&v)[NV][NH], int unit, int strips, int words,
+                                          StripSumSmem<NH, NS>& sm, TagWord* slots, unsigned long long tag, int* err,
+                                          Between between, Scalar_ scalar, double (&total)[NV], double& derived)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int n = 0; n < NV; ++n) {
-            v[n][0] += __shfl_down_sync(0xffffffffu, v[n][0], o);
-            v[n][1] += __shfl_down_sync(0xffffffffu, v[n][1], o);
-        }
+        for (int n = 0; n < NV; ++n)
+#pragma unroll
+            for (int h = 0; h < NH; ++h) v[n][h] += __shfl_down_sync(0xffffffffu, v[n][h], o);
     if (lane == 0)
 #pragma unroll
-        for (int n = 0; n < NV; ++n) {
-            sm.warp[n][0][warp] = v[n][0];
-            sm.warp[n][1][warp] = v[n][1];
-        }
+        for (int n = 0; n < NV; ++n)
+#pragma unroll
+            for (int h = 0; h < NH; ++h) sm.warp[n][h][warp] = v[n][h];
     __syncthreads();
-    if ((tid & 127) < 2 * NV && pair >= 0) {   // the first threads of each group publish its strips
-        const int h = tid & 1, n = (tid & 127) >> 1;
-        const double* q = sm.warp[n][h] + (tid >> 7) * 4;
-        word_store(slots + n * words + 2 * pair + h, (q[0] + q[2]) + (q[1] + q[3]), tag);
+    if ((tid & (NT - 1)) < NH * NV && unit >= 0) {   // the first threads of each group publish its strips
+        const int h = (tid & (NT - 1)) % NH, n = (tid & (NT - 1)) / NH;
+        word_store(slots + n * words + strip_words(NH) * unit + h, warps_sum<NT>(sm.warp[n][h] + tid / NT * (NT / 32)), tag);
     }
     between();
     {   // every word of the grid into shared memory: a first look at all of this thread's, then one by one
@@ -139,17 +148,18 @@ __device__ __forceinline__ bool strip_sum(double (&v)[NV][2], int pair, int stri
                 }
     }
     __syncthreads();
-    if (tid < 128) {
+    if (tid < NT) {
+        constexpr int per = kStripMax / NT;
         double t[NV];
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            double q[kStripMax / 128];
+            double q[per];
             t[n] = 0.0;
 #pragma unroll
-            for (int m = 0; m < kStripMax / 128; ++m) q[m] = tid + m * 128 < strips ? sm.vals[n][tid + m * 128] : 0.0;
+            for (int m = 0; m < per; ++m) q[m] = tid + m * NT < strips ? sm.vals[n][tid + m * NT] : 0.0;
 #pragma unroll
-            for (int m = 0; m < kStripMax / 128; ++m)
-                if (tid + m * 128 < strips) t[n] += q[m];
+            for (int m = 0; m < per; ++m)
+                if (tid + m * NT < strips) t[n] += q[m];
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -158,9 +168,9 @@ __device__ __forceinline__ bool strip_sum(double (&v)[NV][2], int pair, int stri
         if (lane == 0)
 #pragma unroll
             for (int n = 0; n < NV; ++n) sm.fin[n][warp] = t[n];
-        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+        asm volatile("bar.sync 1, %0;\n" ::"n"(NT) : "memory");
 #pragma unroll
-        for (int n = 0; n < NV; ++n) t[n] = (sm.fin[n][0] + sm.fin[n][2]) + (sm.fin[n][1] + sm.fin[n][3]);
+        for (int n = 0; n < NV; ++n) t[n] = warps_sum<NT>(sm.fin[n]);
         const double d = scalar(t);
         if (tid == 0) {
 #pragma unroll

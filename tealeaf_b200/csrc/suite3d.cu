@@ -353,7 +353,9 @@ void run_kernel_initialise(Chunk* chunk, Settings* settings)
     bytes += align((size_t)s->partial_capacity * sizeof(double)) + align(tl::kMaxSums * sizeof(double)) + 256;
     bytes += align(sizeof(tl::DevState));
     s->sum_cells = (x - 2L * settings->halo_depth) * (y - 2L * settings->halo_depth) * (z - 2L * settings->halo_depth);
-    bytes += tl::sum_scratch_bytes(s->sum_cells);
+    bytes += align(tl::sum_scratch_bytes(s->sum_cells));
+    const Chip3Cut cut = chip3_cut(s->g, s->sm_count);
+    bytes += 256 + (size_t)cut.units * chip3_words(cut.tiles * s->g.zr, cut.tiles) * sizeof(tl::TagWord);
     if (!TL_CUDA(cudaMalloc(&s->slab, bytes))) return;
     s->slab_bytes = bytes;
     TL_CUDA(cudaMemsetAsync(s->slab, 0, bytes, s->stream));
@@ -371,6 +373,9 @@ void run_kernel_initialise(Chunk* chunk, Settings* settings)
     s->d_state = (tl::DevState*)cur;
     cur += align(sizeof(tl::DevState));
     s->sum_scratch = cur;
+    cur += align(tl::sum_scratch_bytes(s->sum_cells));
+    s->chip_err = (int*)cur;
+    if (cut.units > 0) s->chip_words = (tl::TagWord*)(cur + 256);
     if (!TL_CUDA(cudaHostAlloc((void**)&s->h_out, tl::kMaxSums * sizeof(double) + 64, cudaHostAllocMapped))) return;
     double* dev_view = nullptr;
     if (!TL_CUDA(cudaHostGetDevicePointer((void**)&dev_view, s->h_out, 0))) return;

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "blocked3d.cuh"
+#include "gridsum.cuh"
 #include "kernels3d.cuh"
 #include "summary.cuh"
 
@@ -44,6 +45,12 @@ struct TlSuite3D {
     double* d_cheby_alphas = nullptr;
     double* d_cheby_betas = nullptr;
     int table_len = 0;
+    // CG loop of a mesh that fits on chip (cgchip3d.cuh): the words its blocks
+    // exchange (null for a larger mesh), the last tag used in them and the
+    // word its bounded waits raise.
+    tl::TagWord* chip_words = nullptr;
+    unsigned long long chip_tag = 0;
+    int* chip_err = nullptr;
     bool tma = true;   // feed the CG w sweep by TMA where the layout allows (tl3d_set_tma)
     bool temporal_blocking = true;   // Chebyshev / PPCG blocks (tl3d_set_temporal_blocking)
     // Chebyshev trips / PPCG inner steps of the run_* path deferred while the
@@ -106,6 +113,29 @@ inline int choose_zr(int nx, int ny, int nz, int sm_count)
     }
     return best;
 }
+// How a mesh is cut to be held on the SMs (cgchip3d.cuh): units of `tiles`
+// z-pencils, at most kChipPlanes3 planes, two units per SM at most; tiles 0
+// where it does not fit. choose_zr gives pencils of 4 to 6 planes to nearly
+// every mesh small enough. The fewest pencils per unit that fit: more units,
+// less work in each.
+constexpr int kChipPlanes3 = 16;
+struct Chip3Cut {
+    int tiles, units;
+};
+inline Chip3Cut chip3_cut(const Geo& g, int sm_count)
+{
+    const dim3 d = interior_grid(g);
+    if (g.zr >= 4 && g.zr <= 6)
+        for (int t = 1; t * g.zr <= kChipPlanes3; ++t) {
+            const long units = (long)d.x * d.y * tl::ceil_div(d.z, t);
+            if (units <= 2L * sm_count) return {t, (int)units};
+        }
+    return {0, 0};
+}
+// Words of one unit: its sums, twice; 8 rows' 32 side cells; 2 edge rows of
+// its planes; 2 end planes.
+inline size_t chip3_words(int planes, int tiles) { return 2 * tl::strip_words(tiles) + 256 + 64 * (size_t)planes + 2 * NT; }
+
 inline dim3 full_grid(const Geo& g) { return dim3(tl::ceil_div(g.x, FBX), tl::ceil_div(g.y, FBY), g.z); }
 // Interior grid plus the halo-duty z-plane of the fused sweeps.
 inline dim3 fused_grid(const Geo& g)

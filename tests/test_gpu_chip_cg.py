@@ -82,3 +82,51 @@ def test_chip_pcg_against_the_oracle(cells, cap, pc, oracle_lib):
             assert abs(x - y) <= 1e-12 * abs(y)
     finally:
         h.finalise()
+
+
+FIELDS3 = ("u", "u0", "p", "r", "w", "kx", "ky", "kz", "energy")
+
+
+@pytest.mark.parametrize("cells,cap,steps", [
+    ((5, 1, 1), 3, 1), ((3, 2, 4), 20000, 1), ((33, 9, 5), 20000, 2), ((32, 8, 17), 40, 1), ((65, 17, 33), 60, 2),
+    ((48, 48, 48), 1, 1), ((48, 47, 50), 30, 1), ((96, 96, 65), 20, 1), ((97, 90, 100), 20, 1), ((16, 16, 16), 50, 1),
+    ((100, 90, 80), 20, 1), ((64, 63, 150), 20, 1), ((120, 100, 77), 20, 1), ((64, 156, 78), 20, 1),
+    ((39, 133, 82), 20, 1), ((149, 43, 104), 20, 1), ((133, 32, 98), 20, 1), ((128, 128, 72), 20, 1),
+])
+def test_chip_cg_3d_is_bit_identical(cells, cap, steps):
+    """k3_cg_chip against the two launches per trip of the run_* path: units of
+    one to four pencils of 4, 5 and 6 planes, ragged in every direction."""
+    a, b = both(3, cells, cap, steps)
+    try:
+        for tt in range(steps):
+            ra, rb = a.solve(tt), b.solve_device(tt)
+            assert ra.iterations == rb.iterations
+            assert ra.error == rb.error
+            assert ra.summary == rb.summary
+            for f in FIELDS3:
+                assert np.array_equal(a.download(f), b.download(f)), (tt, f)
+    finally:
+        a.finalise()
+        b.finalise()
+
+
+@pytest.mark.parametrize("dims,cells", [
+    (2, (129, 37)), (2, (513, 941)), (2, (1025, 900)), (2, (1000, 1180)), (2, (97, 61)),
+    (3, (33, 9, 5)), (3, (39, 133, 82)), (3, (100, 90, 80)), (3, (65, 17, 33)),
+])
+def test_chip_cg_on_a_rough_density(dims, cells):
+    """Every face coefficient different from its neighbours, those on the
+    domain's edge included."""
+    a, b = both(dims, cells, 30)
+    rng = np.random.default_rng(5)
+    try:
+        rho = 0.05 + 20.0 * rng.random(a.shape)
+        for h in (a, b):
+            h.upload("density", rho)
+        ra, rb = a.solve(0), b.solve_device(0)
+        assert ra.iterations == rb.iterations and ra.error == rb.error
+        for f in FIELDS2 if dims == 2 else FIELDS3:
+            assert np.array_equal(a.download(f), b.download(f)), f
+    finally:
+        a.finalise()
+        b.finalise()
