@@ -46,6 +46,8 @@ sys.path.insert(0, str(REPO))
 # u,r; p update reads p,r writes p; ...
 KERNEL_BYTES_PER_CELL = {
     "k_cg_w_fused": 48,      # reads p_old, r, kx, ky; writes p, w
+    "k_cg_wu_fused": 72,     # the same with two trips' u updates: reads u and the p before, writes u
+    "k_cg_r_fused": 24,      # reads r, w; writes r
     "k_cg_ur_fused": 48,     # reads u, p, r, w; writes u, r
     "k_cheby_trip": 56,      # reads u, p, u0, kx, ky; writes u, p (w, r only on norm trips)
     "k_ppcg_step": 64,       # reads sd, r, kx, ky, u; writes sd, r, u
@@ -61,9 +63,9 @@ KERNEL_BYTES_PER_CELL = {
     "k_cheby_sweep": 64, "k_add_p": 24, "k_ppcg_inner_a": 56, "k_ppcg_inner_b": 24,
     "k_norm2": 8, "k_residual": 40,
 }
-# Algorithmic bytes of one CG iteration per interior cell (12 FP64 streams:
-# sweep 1 r,p,kx,ky -> p,w; sweep 2 u,p,r,w -> u,r).
-CG_BYTES_PER_CELL_ITER = 96
+# Algorithmic bytes of one CG iteration per interior cell (w sweep r,p,kx,ky ->
+# p,w; r sweep r,w -> r; every second w sweep also u and the p before it -> u).
+CG_BYTES_PER_CELL_ITER = 84
 FALLBACK_HBM_GBS = 6650.0
 
 
@@ -419,7 +421,7 @@ def extra_dropin(n: int, dims: int, peak: float, steps: int = 2, warm_cap: int =
     deck; 3D: the 6-box deck of the adjoint configuration): one warm-up
     timestep capped at `warm_cap` iterations, then `steps` full timesteps of
     the device-resident loop to eps 1e-15, timed with CUDA events on the
-    suite stream; the fraction counts 96 (2D) / 104 (3D) algorithmic bytes
+    suite stream; the fraction counts 84 (2D) / 104 (3D) algorithmic bytes
     per cell and iteration."""
     import ctypes as C
 

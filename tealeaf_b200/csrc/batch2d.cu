@@ -494,7 +494,7 @@ void issue_step(TlBatch* B, int iter_cap, bool finish)
         const double rx = dt / (st->dx * st->dx), ry = dt / (st->dy * st->dy);
         launch_halos(B, b, 2, {c->density, c->energy});
         k_cg_init<<<full_grid(s->g), FB, 0, B->stream>>>(s->g, st->coefficient, rx, ry, c->density, c->energy, c->u,
-                                                          c->p, nullptr, c->r, c->w, c->kx, c->ky, B->rs,
+                                                          c->p, nullptr, nullptr, c->r, c->w, c->kx, c->ky, B->rs,
                                                           FinCgInit{B->d_scratch_state, nullptr});
         k_copy_u<<<interior_grid(s->g), BX, 0, B->stream>>>(s->g, c->u0, c->u);
         char* base = (char*)B->slab + B->field_off[b];

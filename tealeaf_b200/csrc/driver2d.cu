@@ -134,17 +134,47 @@ struct Run {
     }
 
     // ------------------------------------------------------------- CG phase
-    // Trips `from`.. of cg_main_step_driver (2d/drivers/cg_driver.c:65-124)
-    // until the loop ends; `fresh`: the first trip follows cg_init (nothing
-    // pending). Closes the phase: last p update and the halo of u and p.
-    DevState cg_phase(int from, bool fresh)
+    // The trips of cg_main_step_driver (2d/drivers/cg_driver.c:65-124) after
+    // cg_init until the loop ends. Closes the phase: last p update and the halo
+    // of u and p.
+    DevState cg_phase()
     {
-        if (from == 0 && fresh && s->chip_words && prm.max_iters > 0) return cg_close(cg_chip<0>(s->g, nullptr), chunk->r);
+        if (s->chip_words && prm.max_iters > 0) return cg_close(cg_chip<0>(s->g, nullptr), chunk->r);
+        return cg_deferred();
+    }
+
+    // The CG loop of a mesh too large for that: the w sweep of every second
+    // trip applies the u updates of the two trips before it (CgU), so p goes
+    // round three buffers, the third the suite's second sd buffer (unused by
+    // CG; cg_init has cleared its halo as p's).
+    DevState cg_deferred()
+    {
+        double* buf[3] = {chunk->p, s->alt[ALT_P], s->alt[ALT_SD]};   // trip t's p is buf[t % 3]
+        FinCgW fin_w{s->d_state, s->d_cg_alphas};
         FinCgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
-        const Scalar alpha{0.0, &s->d_state->alpha};
-        return cg_trips(from, fresh, chunk->r, [&](double* p) {
-            launch_cg_ur2(s, gi, alpha, chunk->u, p, chunk->r, chunk->w, done(), fin_ur);
+        const Scalar beta{0.0, &s->d_state->beta}, alpha{0.0, &s->d_state->alpha};
+        DevState st = loop(0, [&](int t) {
+            double* const p = buf[t % 3];
+            const double* const p1 = buf[(t + 2) % 3];
+            if (t == 0)
+                launch_cg_w2<false, false>(s, chunk, gh, fc, beta, p, p, chunk->r, chunk->w, nullptr, 0, done(), fin_w);
+            else if (t % 2 == 0)
+                launch_cg_w2<true, true, true>(s, chunk, gh, fc, beta, p1, p, chunk->r, chunk->w, nullptr, 0, done(),
+                                               fin_w, CgU{chunk->u, buf[(t + 1) % 3], s->d_cg_alphas, t});
+            else
+                launch_cg_w2<true, true>(s, chunk, gh, fc, beta, p1, p, chunk->r, chunk->w, nullptr, 0, done(), fin_w);
+            launch_cg_r2(s, gi, alpha, chunk->r, chunk->w, done(), fin_ur);
         });
+        const int t = st.trip;   // trips that ran: t - 1 is the last
+        if (t > 0) {
+            TL_LAUNCH(s, "k_cg_u_close", (k_cg_u_close<<<gi, BX, 0, s->stream>>>(
+                                             s->g, chunk->u, buf[(t + 1) % 3], buf[(t + 2) % 3], s->d_cg_alphas, t,
+                                             t % 2 == 0 ? 1 : 0)));
+            chunk->p = buf[(t + 2) % 3];
+            s->alt[ALT_P] = buf[t % 3];
+            s->alt[ALT_SD] = buf[(t + 1) % 3];
+        }
+        return cg_close(st, chunk->r);
     }
 
     // The whole loop in one launch (k_cg_chip) for a mesh whose state fits on
@@ -601,7 +631,7 @@ void tl2d_solve_step(Chunk* chunk, Settings* settings, int tt, TlStepStats* stat
     }
     TL_LAUNCH(s, "k_cg_init", k_cg_init<<<full_grid(s->g), FB, 0, s->stream>>>(
                                   s->g, settings->coefficient, rx, ry, chunk->density, chunk->energy, chunk->u,
-                                  chunk->p, s->alt[ALT_P], chunk->r, chunk->w, chunk->kx, chunk->ky, s->rs,
+                                  chunk->p, s->alt[ALT_P], s->alt[ALT_SD], chunk->r, chunk->w, chunk->kx, chunk->ky, s->rs,
                                   FinCgInit{s->d_state, s->d_mirror}));
     int h1[TL_NUM_FIELDS] = {0};
     h1[TL_FIELD_U] = h1[TL_FIELD_P] = 1;
@@ -612,7 +642,7 @@ void tl2d_solve_step(Chunk* chunk, Settings* settings, int tt, TlStepStats* stat
 
     if (settings->solver == TL_CG_SOLVER && s->precond == kPrecondDiag) st = R.pcg_phase<1>();
     else if (settings->solver == TL_CG_SOLVER && s->precond == kPrecondBlock) st = R.pcg_phase<4>();
-    else st = R.cg_phase(0, true);
+    else st = R.cg_phase();
     error = st.error;
     if (st.reason == 2 && settings->solver == TL_CHEBY_SOLVER) {
         const int tt_sw = st.trip;

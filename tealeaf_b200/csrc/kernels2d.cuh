@@ -345,9 +345,10 @@ static __global__ void __launch_bounds__(BX) k_jacobi_iterate(Geo g, const doubl
 
 // ---- full-array kernels (thread per cell) --------------------------------
 
-// cg_init fused (cg.c:9-85), p written to both p buffers: u = e*rho everywhere; face coefficients on
+// cg_init fused (cg.c:9-85): u = e*rho everywhere; face coefficients on
 // [hd, n-1); w = A u, r = u - w, p = r on the interior with rro = sum(r*p);
-// p = r = 0 elsewhere and w = conductivity on the rest of [1, n-1).
+// p = r = 0 elsewhere and w = conductivity on the rest of [1, n-1). The
+// buffers p2 and p3 that p alternates with have the same cells cleared.
 // Coefficients and neighbour values are recomputed from density/energy with
 // the reference expressions, so they equal the stored ones bit for bit.
 template <typename Finish>
@@ -355,7 +356,7 @@ static __global__ void __launch_bounds__(FB) k_cg_init(Geo g, int coefficient, d
                                                 const double* __restrict__ density,
                                                 const double* __restrict__ energy, double* __restrict__ u,
                                                 double* __restrict__ p, double* __restrict__ p2,
-                                                double* __restrict__ r,
+                                                double* __restrict__ p3, double* __restrict__ r,
                                                 double* __restrict__ w, double* __restrict__ kx,
                                                 double* __restrict__ ky, ReduceSlots rs, Finish fin)
 {
@@ -394,11 +395,11 @@ static __global__ void __launch_bounds__(FB) k_cg_init(Geo g, int coefficient, d
             const double rr = uc - v;
             r[i] = rr;
             p[i] = rr;
-            if (p2) p2[i] = rr;
             acc[0] = rr * rr;
         } else {
             p[i] = 0.0;
             if (p2) p2[i] = 0.0;
+            if (p3) p3[i] = 0.0;
             r[i] = 0.0;
             if (ring) w[i] = wc;
         }
@@ -656,8 +657,20 @@ struct StripC {
 // reflective halo of u (depth uhd, u is not modified here) is written too.
 // p is read from p_in, the new p written to p_out (a second buffer, since
 // neighbours still read the old p; p_out == p_in when !FUSE_P).
-template <bool FUSE_P, bool REFLECT, typename Finish>
-static __global__ void __launch_bounds__(BX, TL2D_MINB) k_cg_w_fused(Geo g, Faces fc, Scalar beta,
+// UPD: the sweep also applies the u updates of the two trips before it, u +=
+// alpha_{t-2} p_{t-2} + alpha_{t-1} p_{t-1}, one after the other: p_{t-1} (p_in)
+// is here anyway, so a trip's pair of sweeps moves u and p_{t-2} every other
+// trip instead of u and p in each u/r sweep: 84 B per cell and trip on average
+// against 96. At 4096^2 two trips take 141.5 + 207.7 + 2 x 71.2 us against 2 x
+// (142.6 + 131.3) (200 trips: 49.8 ms against 55.1).
+struct CgU {
+    double* u;
+    const double* p2;       // p_{t-2}
+    const double* alphas;   // the trips' alphas
+    int t;                  // this trip
+};
+template <bool FUSE_P, bool REFLECT, bool UPD, typename Finish>
+static __global__ void __launch_bounds__(BX, TL2D_MINB) k_cg_w_fused(Geo g, Faces fc, Scalar beta, CgU cu,
                                                           const double* __restrict__ p_in, double* p_out,
                                                           const double* __restrict__ r, double* __restrict__ w,
                                                           const double* __restrict__ kx,
@@ -667,6 +680,7 @@ static __global__ void __launch_bounds__(BX, TL2D_MINB) k_cg_w_fused(Geo g, Face
     if (gate_closed(done)) return;
     double acc[1] = {0.0};
     const double bt = FUSE_P ? beta.get() : 0.0;
+    const double a0 = UPD ? cu.alphas[cu.t - 2] : 0.0, a1 = UPD ? cu.alphas[cu.t - 1] : 0.0;
     auto cur = [&](long idx) { return FUSE_P ? bt * p_in[idx] + r[idx] : p_in[idx]; };
     if (blockIdx.y + 1 < gridDim.y) {
         const StripC s(g);
@@ -694,6 +708,7 @@ TL2D_PRAGMA_UNROLL(TL2D_UNROLL)
                 w[i] = v;
                 acc[0] += v * pc;
                 if (FUSE_P) p_out[i] = pc;
+                if (UPD) cu.u[i] = (cu.u[i] + a0 * cu.p2[i]) + a1 * p_in[i];
             }
             pd = pc;
             pc = pu;
@@ -724,24 +739,33 @@ static_assert((BX * sizeof(double)) % 16 == 0 && ((BX + 4) * sizeof(double)) % 1
                   ((BX + 2) * sizeof(double)) % 16 == 0,
               "TMA boxes of the 2D sweeps must be multiples of 16 bytes wide");
 static_assert(kStagesT >= 3, "row block b reads stages b and b+1 while a later one is in flight");
+template <bool UPD>
 struct RowsT {
     alignas(128) double P[kRowsT][BX + 4];
     alignas(128) double R[kRowsT][BX + 4];
     alignas(128) double KX[kRowsT][BX + 2];
     alignas(128) double KY[kRowsT][BX];
+    // UPD: u and p_{t-2} (75 KB a ring, 3 blocks per SM: 207.7 us at 4096^2, against 216.8 / 208.9 for rings of
+    // two-row stages, 4 / 5 deep, at 4 and 3 per SM)
+    alignas(128) double U[UPD ? kRowsT : 1][UPD ? BX : 16];
+    alignas(128) double P2[UPD ? kRowsT : 1][UPD ? BX : 16];
 };
 struct Tma2Maps {
-    CUtensorMap p, r, kx, ky;
+    CUtensorMap p, r, kx, ky, u, p2;
 };
-constexpr size_t kTmaRowsBytes = kStagesT * sizeof(RowsT) + kStagesT * 8 + 128;   // + barriers + alignment
+template <bool UPD>
+constexpr size_t tma_rows_bytes()   // + barriers + alignment
+{
+    return kStagesT * sizeof(RowsT<UPD>) + kStagesT * 8 + 128;
+}
 
 // k_cg_w_fused with its operand rows brought in by TMA. The same strips,
 // rows in the same order per thread and the same arithmetic, so the same
 // results (partial sums included). Stage b holds rows j0-1+4b .. j0+2+4b;
 // rows j0+4b .. j0+4b+3 read stages b and b+1. `err`: the bounded barrier
 // waits' flag.
-template <bool FUSE_P, bool REFLECT, typename Finish>
-static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc, Scalar beta,
+template <bool FUSE_P, bool REFLECT, bool UPD, typename Finish>
+static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc, Scalar beta, CgU cu,
                                                                       const __grid_constant__ Tma2Maps maps,
                                                                       const double* __restrict__ p_in, double* p_out,
                                                                       const double* __restrict__ r,
@@ -753,12 +777,14 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc
     extern __shared__ __align__(128) unsigned char t2_raw[];
     if (gate_closed(done)) return;
     double acc[1] = {0.0};
+    using Rows = RowsT<UPD>;
     const double bt = FUSE_P ? beta.get() : 0.0;
+    const double a0 = UPD ? cu.alphas[cu.t - 2] : 0.0, a1 = UPD ? cu.alphas[cu.t - 1] : 0.0;
     auto cur = [&](long idx) { return FUSE_P ? bt * p_in[idx] + r[idx] : p_in[idx]; };
     if (blockIdx.y + 1 < gridDim.y) {
         unsigned char* base = t2_raw + ((128 - (tl::smem_addr(t2_raw) & 127)) & 127);
-        RowsT* ring = reinterpret_cast<RowsT*>(base);
-        unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kStagesT * sizeof(RowsT));
+        Rows* ring = reinterpret_cast<Rows*>(base);
+        unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kStagesT * sizeof(Rows));
         const StripC s(g);
         const int x = g.x, tx = threadIdx.x;
         const int k0 = g.hd + blockIdx.x * BX;
@@ -766,15 +792,20 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc
         const int np = (s.j1 - s.j0 + 2 + kRowsT - 1) / kRowsT;   // stages: rows j0-1 .. j1
         constexpr unsigned kP = sizeof(double) * kRowsT * (BX + 4);
         constexpr unsigned kK = sizeof(double) * kRowsT * ((BX + 2) + BX);
+        constexpr unsigned kU = sizeof(double) * kRowsT * BX;
         auto issue = [&](int b) {
-            RowsT& S = ring[b % kStagesT];
+            Rows& S = ring[b % kStagesT];
             unsigned long long* bar = &bars[b % kStagesT];
             const int y0 = jb + b * kRowsT;
-            tl::mbar_expect_tx(bar, kP * (FUSE_P ? 2u : 1u) + kK);
+            tl::mbar_expect_tx(bar, kP * (FUSE_P ? 2u : 1u) + kK + (UPD ? 2u * kU : 0u));
             tl::tma_load_3d(&S.P[0][0], &maps.p, k0 - 2, y0, 0, bar);
             if (FUSE_P) tl::tma_load_3d(&S.R[0][0], &maps.r, k0 - 2, y0, 0, bar);
             tl::tma_load_3d(&S.KX[0][0], &maps.kx, k0, y0, 0, bar);
             tl::tma_load_3d(&S.KY[0][0], &maps.ky, k0, y0, 0, bar);
+            if (UPD) {
+                tl::tma_load_3d(&S.U[0][0], &maps.u, k0, y0, 0, bar);
+                tl::tma_load_3d(&S.P2[0][0], &maps.p2, k0, y0, 0, bar);
+            }
         };
         if (tx == 0) {
             for (int q = 0; q < kStagesT; ++q) tl::mbar_init(&bars[q], 1);
@@ -790,7 +821,7 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc
         };
         auto fused = [&](int j, int dx) -> double {
             const int t = j - jb;
-            const RowsT& S = ring[(t / kRowsT) % kStagesT];
+            const Rows& S = ring[(t / kRowsT) % kStagesT];
             return FUSE_P ? bt * S.P[t % kRowsT][tx + 2 + dx] + S.R[t % kRowsT][tx + 2 + dx]
                           : S.P[t % kRowsT][tx + 2 + dx];
         };
@@ -811,8 +842,8 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc
                 const int j = s.j0 + b * kRowsT + u;
                 if (j >= s.j1) break;
                 const int t = j - jb, tu = t + 1;
-                const RowsT& S = ring[(t / kRowsT) % kStagesT];
-                const RowsT& U = ring[(tu / kRowsT) % kStagesT];
+                const Rows& S = ring[(t / kRowsT) % kStagesT];
+                const Rows& U = ring[(tu / kRowsT) % kStagesT];
                 const bool at_t = j == g.y - g.hd - 1;
                 const double pu = at_t ? ((REFLECT && fc.t) ? pc : raw(j + 1, 0)) : fused(j + 1, 0);
                 const double kyu = U.KY[tu % kRowsT][tx];
@@ -830,6 +861,7 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc
                     w[i] = v;
                     acc[0] += v * pc;
                     if (FUSE_P) p_out[i] = pc;
+                    if (UPD) cu.u[i] = (S.U[t % kRowsT][tx] + a0 * S.P2[t % kRowsT][tx]) + a1 * raw(j, 0);
                 }
                 pd = pc;
                 pc = pu;
@@ -959,6 +991,127 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_ur_fused_tma(Geo g, Scalar 
         }
     }
     tl::grid_sum<1, BX>(acc, rs, bx + by * gridDim.x, block_count(), fin);
+}
+
+// CG sweep 2 where the w sweeps carry u (CgU): r -= alpha w ; rrn = sum(r*r).
+// Strips, rows and sums as k_cg_ur_fused.
+template <typename Finish>
+static __global__ void __launch_bounds__(BX, TL2D_MINB) k_cg_r_fused(Geo g, Scalar alpha, double* __restrict__ r,
+                                                                    const double* __restrict__ w, ReduceSlots rs,
+                                                                    const int* __restrict__ done, Finish fin)
+{
+    if (gate_closed(done)) return;
+    const int bx = ur_bx(), by = ur_by();
+    Strip s(g, bx, by);
+    double acc[1] = {0.0};
+    if (s.active) {
+        const double a = alpha.get();
+        const long step = TL2D_UR_REVERSE ? -(long)g.x : (long)g.x;
+        long i = s.k + (long)(TL2D_UR_REVERSE ? s.j1 - 1 : s.j0) * g.x;
+TL2D_PRAGMA_UNROLL(8)
+        for (int n = 0; n < s.j1 - s.j0; ++n, i += step) {
+            const double rn = r[i] - a * w[i];
+            r[i] = rn;
+            acc[0] += rn * rn;
+        }
+    }
+    tl::grid_sum<1, BX>(acc, rs, bx + by * gridDim.x, block_count(), fin);
+}
+
+// k_cg_r_fused with its rows brought in by TMA (as k_cg_ur_fused_tma): six
+// stages of 4 rows (49 KB, 4 blocks per SM) take 72.3 us at 4096^2, three
+// stages at 8 blocks per SM 74.3; 105 with per-thread loads.
+#ifndef TL2D_TMA_ROWS_R
+#define TL2D_TMA_ROWS_R 4
+#endif
+#ifndef TL2D_TMA_STAGES_R
+#define TL2D_TMA_STAGES_R 6
+#endif
+#ifndef TL2D_MINB_R
+#define TL2D_MINB_R 4
+#endif
+constexpr int kRowsR = TL2D_TMA_ROWS_R;
+constexpr int kStagesR = TL2D_TMA_STAGES_R;
+struct RowsR {
+    alignas(128) double R[kRowsR][BX];
+    alignas(128) double W[kRowsR][BX];
+};
+struct TmaRMaps {
+    CUtensorMap r, w;
+};
+constexpr size_t kTmaRBytes = kStagesR * sizeof(RowsR) + kStagesR * 8 + 128;
+
+template <typename Finish>
+static __global__ void __launch_bounds__(BX, TL2D_MINB_R) k_cg_r_fused_tma(Geo g, Scalar alpha,
+                                                                 const __grid_constant__ TmaRMaps maps,
+                                                                 double* __restrict__ r, ReduceSlots rs,
+                                                                 const int* __restrict__ done, Finish fin, int* err)
+{
+    extern __shared__ __align__(128) unsigned char tr_raw[];
+    if (gate_closed(done)) return;
+    unsigned char* base = tr_raw + ((128 - (tl::smem_addr(tr_raw) & 127)) & 127);
+    RowsR* ring = reinterpret_cast<RowsR*>(base);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kStagesR * sizeof(RowsR));
+    const int bx = ur_bx(), by = ur_by();
+    Strip s(g, bx, by);
+    double acc[1] = {0.0};
+    const int tx = threadIdx.x;
+    const int k0 = g.hd + bx * BX;
+    const int np = (s.j1 - s.j0 + kRowsR - 1) / kRowsR;
+    // stage b holds rows y0(b) .. y0(b) + kRowsR - 1 (the strip's last stage may run past j1)
+    auto stage_y0 = [&](int b) { return s.j0 + (TL2D_UR_REVERSE ? np - 1 - b : b) * kRowsR; };
+    auto issue = [&](int b) {
+        RowsR& S = ring[b % kStagesR];
+        unsigned long long* bar = &bars[b % kStagesR];
+        tl::mbar_expect_tx(bar, 2u * sizeof(double) * kRowsR * BX);
+        tl::tma_load_3d(&S.R[0][0], &maps.r, k0, stage_y0(b), 0, bar);
+        tl::tma_load_3d(&S.W[0][0], &maps.w, k0, stage_y0(b), 0, bar);
+    };
+    if (tx == 0) {
+        for (int q = 0; q < kStagesR; ++q) tl::mbar_init(&bars[q], 1);
+        tl::mbar_fence_init();
+    }
+    __syncthreads();
+    if (tx == 0)
+        for (int b = 0; b < kStagesR - 1 && b < np; ++b) issue(b);
+    const double a = alpha.get();
+    for (int b = 0; b < np; ++b) {
+        __syncthreads();   // every thread is past stage b-1: its slot is free
+        if (tx == 0 && b + kStagesR - 1 < np) issue(b + kStagesR - 1);
+        tl::mbar_wait(&bars[b % kStagesR], (unsigned)(b / kStagesR) & 1u, err);
+        const RowsR& S = ring[b % kStagesR];
+        const int y0 = stage_y0(b);
+#pragma unroll
+        for (int q = 0; q < kRowsR; ++q) {
+            const int t = TL2D_UR_REVERSE ? kRowsR - 1 - q : q;   // rows in the order of k_cg_r_fused
+            const int j = y0 + t;
+            if (j >= s.j1) continue;
+            if (s.active) {
+                const double rn = S.R[t][tx] - a * S.W[t][tx];
+                r[s.k + (long)j * g.x] = rn;
+                acc[0] += rn * rn;
+            }
+        }
+    }
+    // every issued stage was waited for: no copy in flight
+    tl::grid_sum<1, BX>(acc, rs, bx + by * gridDim.x, block_count(), fin);
+}
+
+// u += alpha_{t-2} p_{t-2} [two], u += alpha_{t-1} p_{t-1}: the updates still due
+// after t trips.
+static __global__ void __launch_bounds__(BX) k_cg_u_close(Geo g, double* __restrict__ u, const double* __restrict__ p2,
+                                                         const double* __restrict__ p1,
+                                                         const double* __restrict__ alphas, int t, int two)
+{
+    Strip s(g);
+    if (!s.active) return;
+    const double a0 = two ? alphas[t - 2] : 0.0, a1 = alphas[t - 1];
+    long i = s.k + (long)s.j0 * g.x;
+    for (int j = s.j0; j < s.j1; ++j, i += g.x) {
+        double v = u[i];
+        if (two) v += a0 * p2[i];
+        u[i] = v + a1 * p1[i];
+    }
 }
 
 // p = beta p + r in place, with the depth-1 halo of p (and of u unless u is

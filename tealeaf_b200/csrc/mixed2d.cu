@@ -497,7 +497,7 @@ extern "C" int tl2d_refine_solve_step(Chunk* chunk, Settings* settings, int tt, 
     flush(s, chunk);
     TL_LAUNCH(s, "k_cg_init", k_cg_init<<<full_grid(s->g), FB, 0, s->stream>>>(
                                   s->g, settings->coefficient, rx, ry, chunk->density, chunk->energy, chunk->u,
-                                  chunk->p, s->alt[ALT_P], chunk->r, chunk->w, chunk->kx, chunk->ky, s->rs,
+                                  chunk->p, s->alt[ALT_P], nullptr, chunk->r, chunk->w, chunk->kx, chunk->ky, s->rs,
                                   FinCgInit{s->d_state, s->d_mirror}));
     s->pend.halo[TL_FIELD_U] = s->pend.halo[TL_FIELD_P] = 1;
     flush(s, chunk);

@@ -610,7 +610,7 @@ void run_cg_init(Chunk* chunk, Settings* settings, double rx, double ry, double*
     TL_LAUNCH(s, "k_cg_init",
               k_cg_init<<<full_grid(s->g), FB, 0, s->stream>>>(
                   s->g, settings->coefficient, rx, ry, chunk->density, chunk->energy, chunk->u, chunk->p,
-                  s->alt[ALT_P], chunk->r, chunk->w, chunk->kx, chunk->ky, s->rs, tl::NoFinish()));
+                  s->alt[ALT_P], nullptr, chunk->r, chunk->w, chunk->kx, chunk->ky, s->rs, tl::NoFinish()));
     double o;
     if (fetch(s, 1, &o)) *rro += o;
 }

@@ -203,12 +203,14 @@ inline const CUtensorMap* tma_lookup(TlSuite2D* s, const void* ptr, int kind, En
 
 // Tensor map of a chunk array for k_cg_w_fused_tma: kind 0 operand rows (box
 // (BX+4) x kRowsT), 1 kx ((BX+2) x kRowsT), 2 ky (BX x kRowsT); for
-// k_cg_ur_fused_tma: kind 3 (BX x kRowsU).
+// k_cg_ur_fused_tma: kind 3 (BX x kRowsU); for k_cg_r_fused_tma: kind 5 (BX x
+// kRowsR).
 inline const CUtensorMap* tma_map(TlSuite2D* s, const double* ptr, int kind)
 {
-    static const unsigned box[4] = {BX + 4, BX + 2, BX, BX};
+    static const unsigned box[6] = {BX + 4, BX + 2, BX, BX, 0, BX};
+    static const unsigned rows[6] = {kRowsT, kRowsT, kRowsT, kRowsU, 0, kRowsR};
     return tma_lookup(s, ptr, kind, [&](CUtensorMap* m) {
-        return tl::tma_encode_3d(m, ptr, s->g.x, s->g.y, 1, box[kind], kind == 3 ? kRowsU : kRowsT, 1);
+        return tl::tma_encode_3d(m, ptr, s->g.x, s->g.y, 1, box[kind], rows[kind], 1);
     });
 }
 
@@ -218,36 +220,40 @@ inline bool tma_usable(const TlSuite2D* s) { return s->tma && s->g.hd % 2 == 0 &
 
 inline bool tma_failed(const TlSuite2D* s) { return s->h_mirror && s->h_mirror[kTmaErrWord2] != 0; }
 
-// The fused CG w sweep (k_cg_w_fused semantics), by TMA where possible.
-// Internal linkage, like the kernels it launches: each translation unit has
-// its own kernel copies, so each keeps its own record of the raised
-// shared-memory limit.
-template <bool F, bool R, typename Finish>
+// The fused CG w sweep (k_cg_w_fused semantics), by TMA where possible; U: with
+// the u updates of the two trips before it. Internal linkage, like the kernels
+// it launches: each translation unit has its own kernel copies, so each keeps
+// its own record of the raised shared-memory limit.
+template <bool F, bool R, bool U = false, typename Finish>
 static void launch_cg_w2(TlSuite2D* s, Chunk* chunk, dim3 grid, const Faces& fc, Scalar beta, const double* p_in,
-                  double* p_out, const double* r, double* w, double* u_halo, int uhd, const int* done, Finish fin)
+                  double* p_out, const double* r, double* w, double* u_halo, int uhd, const int* done, Finish fin,
+                  const CgU& cu = CgU{})
 {
+    const char* name = U ? "k_cg_wu_fused" : "k_cg_w_fused";
     if (tma_usable(s)) {
         const CUtensorMap* a = tma_map(s, p_in, 0);
         const CUtensorMap* b = F ? tma_map(s, r, 0) : a;
         const CUtensorMap* kx = tma_map(s, chunk->kx, 1);
         const CUtensorMap* ky = tma_map(s, chunk->ky, 2);
-        if (a && b && kx && ky) {
-            const Tma2Maps m{*a, *b, *kx, *ky};
+        const CUtensorMap* mu = U ? tma_map(s, cu.u, 2) : a;
+        const CUtensorMap* m2 = U ? tma_map(s, cu.p2, 2) : a;
+        if (a && b && kx && ky && mu && m2) {
+            const Tma2Maps m{*a, *b, *kx, *ky, *mu, *m2};
             static unsigned attr_set = 0;   // devices on which the shared-memory size was raised
             if (!(attr_set & (1u << (s->device & 31)))) {
-                TL_CUDA(cudaFuncSetAttribute(k_cg_w_fused_tma<F, R, Finish>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaRowsBytes));
+                TL_CUDA(cudaFuncSetAttribute(k_cg_w_fused_tma<F, R, U, Finish>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_rows_bytes<U>()));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, "k_cg_w_fused", (k_cg_w_fused_tma<F, R><<<grid, BX, kTmaRowsBytes, s->stream>>>(
-                                             s->g, fc, beta, m, p_in, p_out, r, w, u_halo, uhd, s->rs, done, fin,
-                                             s->d_mirror + kTmaErrWord2)));
+            TL_LAUNCH(s, name, (k_cg_w_fused_tma<F, R, U><<<grid, BX, tma_rows_bytes<U>(), s->stream>>>(
+                                   s->g, fc, beta, cu, m, p_in, p_out, r, w, u_halo, uhd, s->rs, done, fin,
+                                   s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
-    TL_LAUNCH(s, "k_cg_w_fused", (k_cg_w_fused<F, R><<<grid, BX, 0, s->stream>>>(
-                                     s->g, fc, beta, p_in, p_out, r, w, chunk->kx, chunk->ky, u_halo, uhd, s->rs,
-                                     done, fin)));
+    TL_LAUNCH(s, name, (k_cg_w_fused<F, R, U><<<grid, BX, 0, s->stream>>>(
+                           s->g, fc, beta, cu, p_in, p_out, r, w, chunk->kx, chunk->ky, u_halo, uhd, s->rs, done,
+                           fin)));
 }
 
 // The fused CG u/r update (k_cg_ur_fused semantics), by TMA where possible
@@ -276,6 +282,29 @@ static void launch_cg_ur2(TlSuite2D* s, dim3 grid, Scalar alpha, double* u, cons
     }
     TL_LAUNCH(s, "k_cg_ur_fused", (k_cg_ur_fused<<<grid, BX, 0, s->stream>>>(s->g, alpha, u, p, r, w, s->rs, done,
                                                                             fin)));
+}
+// The fused CG r update (k_cg_r_fused semantics), by TMA where possible
+// (internal linkage as launch_cg_w2).
+template <typename Finish>
+static void launch_cg_r2(TlSuite2D* s, dim3 grid, Scalar alpha, double* r, const double* w, const int* done, Finish fin)
+{
+    if (tma_usable(s)) {
+        const CUtensorMap* mr = tma_map(s, r, 5);
+        const CUtensorMap* mw = tma_map(s, w, 5);
+        if (mr && mw) {
+            const TmaRMaps m{*mr, *mw};
+            static unsigned attr_set = 0;   // devices on which the shared-memory size was raised
+            if (!(attr_set & (1u << (s->device & 31)))) {
+                TL_CUDA(cudaFuncSetAttribute(k_cg_r_fused_tma<Finish>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kTmaRBytes));
+                attr_set |= 1u << (s->device & 31);
+            }
+            TL_LAUNCH(s, "k_cg_r_fused", (k_cg_r_fused_tma<<<grid, BX, kTmaRBytes, s->stream>>>(
+                                             s->g, alpha, m, r, s->rs, done, fin, s->d_mirror + kTmaErrWord2)));
+            return;
+        }
+    }
+    TL_LAUNCH(s, "k_cg_r_fused", (k_cg_r_fused<<<grid, BX, 0, s->stream>>>(s->g, alpha, r, w, s->rs, done, fin)));
 }
 // Region boxes (kTW x kTH cells, kind 4) of the TMA-staged blocked kernels.
 inline const CUtensorMap* blocked_map(TlSuite2D* s, const double* ptr)
