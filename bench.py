@@ -55,6 +55,8 @@ KERNEL_BYTES_PER_CELL = {
     "k_blocked<ppcg>": 64,   # per launch of L PPCG inner steps: reads sd, r, u, kx, ky; writes sd, r, u
     "k3_cg_w": 56,           # 3D: reads p_old, r, kx, ky, kz; writes p, w
     "k3_cg_ur": 48,          # 3D: reads u, p, r, w; writes u, r
+    "k3_cg_wu": 80,          # 3D: the same with two trips' u updates: reads u and the p before, writes u
+    "k3_cg_r": 24,           # 3D: reads r, w; writes r
     "k3_cheby_trip": 64,     # 3D: reads u, p, u0, kx, ky, kz; writes u, p
     "k3_ppcg_step": 72,      # 3D: reads sd, r, u, kx, ky, kz; writes sd, r, u
     "k3_blocked<cheby>": 64,  # 3D, per launch of L Chebyshev trips: reads u, p, u0, kx, ky, kz; writes u, p
@@ -421,7 +423,7 @@ def extra_dropin(n: int, dims: int, peak: float, steps: int = 2, warm_cap: int =
     deck; 3D: the 6-box deck of the adjoint configuration): one warm-up
     timestep capped at `warm_cap` iterations, then `steps` full timesteps of
     the device-resident loop to eps 1e-15, timed with CUDA events on the
-    suite stream; the fraction counts 84 (2D) / 104 (3D) algorithmic bytes
+    suite stream; the fraction counts 84 (2D) / 92 (3D) algorithmic bytes
     per cell and iteration."""
     import ctypes as C
 
@@ -453,7 +455,7 @@ def extra_dropin(n: int, dims: int, peak: float, steps: int = 2, warm_cap: int =
         h.finalise()
     cells = n ** dims
     value = sum(per_step) / (ms / 1000.0)
-    bpc = CG_BYTES_PER_CELL_ITER if dims == 2 else 104
+    bpc = CG_BYTES_PER_CELL_ITER if dims == 2 else 92
     gbs = bpc * cells * value / 1e9
     return {"metric": "solver_iterations_per_s", "value": value, "unit": "iter/s", "dtype": "f64",
             "workload": "dropin_%dd_%d_cg" % (dims, n), "cells": cells, "eps": prob.eps, "steps": steps,

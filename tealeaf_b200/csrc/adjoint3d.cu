@@ -15,7 +15,7 @@
 //
 //   A l_N = dJ/du_N ;  A l_n = l_{n+1}   (n = N-1 .. 1)
 //
-// solved by the forward CG sweeps (k3_cg_w, k3_cg_ur), and the gradient
+// solved by the forward CG loops (cg_chip3, cg_deferred3), and the gradient
 //
 //   dJ/drho_c = dJ/drho_c|explicit + l_1,c e_0,c
 //               - sum_n sum_{f at c} (dk_f/drho_c) (l_a - l_b)(u_a - u_b),
@@ -169,11 +169,9 @@ void copy_field(TlSuite3D* s, double* dst, const double* src)
 }
 
 // CG solve A lam = rhs from lam = 0 to r.r <= rel_tol^2 rhs.rhs with the
-// forward sweeps; clobbers the chunk's p, r, w. Returns the iterations.
+// forward loops; clobbers the chunk's p, r, w. Returns the iterations.
 int adjoint_solve(TlSuite3D* s, Chunk* chunk, const double* rhs, double* lam, double rel_tol, int max_iters)
 {
-    const Faces fc = faces_of(chunk);
-    const dim3 gi = interior_grid(s->g), gh = fused_grid(s->g), bl = interior_block();
     s->h_mirror[0] = 0;
     TL3_LAUNCH(s, "k3a_prep", (k3a_prep<<<full_grid(s->g), full_block(), 0, s->stream>>>(
                                   s->g, rhs, chunk->vec_r, chunk->vec_p, lam, s->rs,
@@ -193,28 +191,12 @@ int adjoint_solve(TlSuite3D* s, Chunk* chunk, const double* rhs, double* lam, do
         TL_CUDA(cudaStreamSynchronize(s->stream));
         return st.trip;
     }
-    double* buf[2] = {chunk->vec_p, s->alt[ALT3_P]};
-    tl::FinCgW fin_w{s->d_state, s->d_cg_alphas};
-    tl::FinCgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
-    const Scalar beta{0.0, &s->d_state->beta}, alpha{0.0, &s->d_state->alpha};
-    const int* done = &s->d_state->done;
-    int cur = 0;
-    batched(s, max_iters, [&](int t) {
-        if (t == 0) {
-            launch_cg_w3<false, false>(s, chunk, gh, fc, beta, buf[cur], buf[cur], chunk->vec_r, chunk->vec_w,
-                                       nullptr, 0, done, fin_w);
-        } else {
-            launch_cg_w3<true, true>(s, chunk, gh, fc, beta, buf[cur], buf[cur ^ 1], chunk->vec_r, chunk->vec_w,
-                                     nullptr, 0, done, fin_w);
-            cur ^= 1;
-        }
-        launch_cg_ur3(s, gi, alpha, lam, buf[cur], chunk->vec_r, chunk->vec_w, done, fin_ur);
-    });
-    DevState st{};
-    TL_CUDA(cudaMemcpy(&st, s->d_state, sizeof(DevState), cudaMemcpyDeviceToHost));
-    const int flips = std::max(0, st.trip - 1);
-    if (buf[flips & 1] != chunk->vec_p) swap_alt(s, chunk, ALT3_P);
-    return st.trip;
+    return cg_deferred3(s, chunk, lam, prm, [&](auto&& trip) {
+               batched(s, max_iters, trip);
+               DevState st{};
+               TL_CUDA(cudaMemcpy(&st, s->d_state, sizeof(DevState), cudaMemcpyDeviceToHost));
+               return st;
+           }).trip;
 }
 
 void face_grad(TlSuite3D* s, Chunk* chunk, Settings* settings, const double* lam, const double* u, double* grad)

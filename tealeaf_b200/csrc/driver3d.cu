@@ -133,31 +133,12 @@ struct Run3 {
                                 s->stream));
     }
 
-    // cg_solver_main_step_driver trips until the loop ends; closes the phase.
-    DevState cg_phase(int from, bool fresh)
+    // cg_solver_main_step_driver trips after cg_init until the loop ends;
+    // closes the phase.
+    DevState cg_phase()
     {
-        if (from == 0 && fresh && cg_chip3(s, chunk, chunk->vec_u, prm)) return cg_close(read_state());
-        double* buf[2] = {chunk->vec_p, s->alt[ALT3_P]};
-        tl::FinCgW fin_w{s->d_state, s->d_cg_alphas};
-        tl::FinCgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
-        const Scalar beta{0.0, &s->d_state->beta}, alpha{0.0, &s->d_state->alpha};
-        int cur = 0;
-        auto trip = [&](int t) {
-            if (fresh && t == from) {
-                launch_cg_w3<false, false>(s, chunk, gh, fc, beta, buf[cur], buf[cur], chunk->vec_r, chunk->vec_w,
-                                           nullptr, 0, done(), fin_w);
-            } else {
-                launch_cg_w3<true, true>(s, chunk, gh, fc, beta, buf[cur], buf[cur ^ 1], chunk->vec_r, chunk->vec_w,
-                                         nullptr, 0, done(), fin_w);
-                cur ^= 1;
-            }
-            launch_cg_ur3(s, gi, alpha, chunk->vec_u, buf[cur], chunk->vec_r, chunk->vec_w, done(), fin_ur);
-        };
-        DevState st = loop(from, trip);
-        const int ran = st.trip - from;
-        const int flips = fresh ? std::max(0, ran - 1) : ran;
-        if (buf[flips & 1] != chunk->vec_p) swap_alt(s, chunk, ALT3_P);
-        return cg_close(st);
+        if (cg_chip3(s, chunk, chunk->vec_u, prm)) return cg_close(read_state());
+        return cg_close(cg_deferred3(s, chunk, chunk->vec_u, prm, [&](auto&& trip) { return loop(0, trip); }));
     }
 
     // Closes a CG phase that ended in state st: the last p update, the halos
@@ -494,7 +475,7 @@ void tl3d_solve_step(Chunk* chunk, Settings* settings, int tt, TlStepStats3* sta
     // cg_solver_init_driver (3d/drivers/cg_solver_driver.c:31-63)
     TL3_LAUNCH(s, "k3_cg_init", k3_cg_init<<<full_grid(s->g), full_block(), 0, s->stream>>>(
                                     s->g, settings->coefficient, rx, ry, rz, chunk->density, chunk->energy,
-                                    chunk->vec_u, chunk->vec_p, s->alt[ALT3_P], chunk->vec_r, chunk->vec_w,
+                                    chunk->vec_u, chunk->vec_p, s->alt[ALT3_P], s->alt[ALT3_SD], chunk->vec_r, chunk->vec_w,
                                     chunk->vec_kx, chunk->vec_ky, chunk->vec_kz, s->rs,
                                     tl::FinCgInit{s->d_state, s->d_mirror}));
     for (int f = 0; f < TL3_NUM_FIELDS; ++f) s->pend.halo[f] = 0;
@@ -503,7 +484,7 @@ void tl3d_solve_step(Chunk* chunk, Settings* settings, int tt, TlStepStats3* sta
     TL3_LAUNCH(s, "k3_copy_u", k3_copy_u<<<R.gi, R.bl, 0, s->stream>>>(s->g, chunk->vec_u0, chunk->vec_u));
     R.read_state();
 
-    DevState st = R.cg_phase(0, true);
+    DevState st = R.cg_phase();
     double error = st.error;
     if (st.reason == 2 && settings->solver == TL3_CHEBY_SOLVER) {
         st = R.cheby_phase(st.trip, st_out);

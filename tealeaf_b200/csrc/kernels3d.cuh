@@ -14,6 +14,8 @@
 #include "solver_common.cuh"
 #include "tealeaf_b200_3d.h"
 
+#include <type_traits>
+
 using tl::ReduceSlots;
 
 namespace tl3d {
@@ -168,6 +170,14 @@ __device__ __forceinline__ void halo_duty3(const Geo& g, const Faces& fc, int de
     }
 }
 
+// body(ii, i, centre, smvp), or with the centre's stored A value where it takes one.
+template <typename Body>
+__device__ __forceinline__ void call_body(Body& body, int ii, long i, double c, double v, double raw)
+{
+    if constexpr (std::is_invocable_v<Body&, int, long, double, double, double>) body(ii, i, c, v, raw);
+    else body(ii, i, c, v);
+}
+
 // Operand planes of the fused sweeps, staged in shared memory: the block's
 // BX x BY cells of the two operand arrays A, B with a one-cell ring (x and y
 // neighbours), and the face coefficients kx (one extra column), ky (one extra
@@ -266,7 +276,7 @@ __device__ __forceinline__ void walkc(const Geo& g, const Faces& fc, const Penci
         const double fr = ii == zlast ? ((REFLECT && fc.f) ? c : F.A[cy][cx]) : cell(F, cy, cx);
         const double v = smvp(P.kx[ty][tx], P.kx[ty][tx + 1], P.ky[ty][tx], P.ky[ty + 1][tx], P.kz[ty][tx],
                               F.kz[ty][tx], c, l, r, d, u, bk, fr);
-        body(ii, i, c, v);
+        call_body(body, ii, i, c, v, P.A[cy][cx]);
         bk = c;
     }
     cp_async_wait<0>();
@@ -368,7 +378,7 @@ __device__ __forceinline__ void walkt(const Geo& g, const Faces& fc, const Penci
         const double fr = ii == zlast ? ((REFLECT && fc.f) ? c : F.A[cy][cx]) : cell(F, cy, cx);
         const double v = smvp(P.kx[ty][tx], P.kx[ty][tx + 1], P.ky[ty][tx], P.ky[ty + 1][tx], P.kz[ty][tx],
                               F.kz[ty][tx], c, l, r, d, u, bk, fr);
-        body(ii, i, c, v);
+        call_body(body, ii, i, c, v, P.A[cy][cx]);
         bk = c;
     }
     __syncthreads();   // every issued plane has been waited for: no copy is in flight
@@ -424,9 +434,45 @@ __device__ __forceinline__ void walk(const Geo& g, const Faces& fc, const Pencil
 // [p = beta p + r] ; depth-1 reflective halo of p ; w = A p ; pw = sum(w p)
 // (3d/c_kernels/omp3/cg_solver.c:105-193). Grid: interior blocks plus one
 // z-plane of halo-duty blocks (the reflected halo of p_out, and the pending
-// halo of u when u_halo is given; u is read-only here).
-template <bool FUSE_P, bool REFLECT, typename Finish>
-static __global__ void __launch_bounds__(NT, TL3D_MINB) k3_cg_w(Geo g, Faces fc, Scalar beta,
+// halo of u when u_halo is given; u is read-only here). UPD: the sweep also
+// applies the u updates of the two trips before it, u += alpha_{t-2} p_{t-2} +
+// alpha_{t-1} p_{t-1}, one after the other (p_{t-1} is here anyway): 92 B per
+// cell and trip on average against 104 with u and p moved in each u/r sweep.
+// u and p_{t-2} come one plane ahead by per-thread loads.
+struct CgU {
+    double* u;
+    const double* p2;       // p_{t-2}
+    const double* alphas;   // the trips' alphas
+    int t;                  // this trip
+};
+struct CgUWalk {            // a thread's column of u and p_{t-2}
+    const CgU& cu;
+    const Geo& g;
+    const PencilC& s;
+    double a0, a1, un, pn;
+    __device__ __forceinline__ CgUWalk(const CgU& c, const Geo& geo, const PencilC& pc) : cu(c), g(geo), s(pc)
+    {
+        a0 = cu.alphas[cu.t - 2];
+        a1 = cu.alphas[cu.t - 1];
+        fetch(s.i0, s.k + (long)s.j * g.x + (long)s.i0 * g.xy());
+    }
+    __device__ __forceinline__ void fetch(int ii, long i)
+    {
+        un = pn = 0.0;
+        if (s.active && ii < s.i1) {
+            un = cu.u[i];
+            pn = cu.p2[i];
+        }
+    }
+    __device__ __forceinline__ void step(int ii, long i, double raw)
+    {
+        const double v = (un + a0 * pn) + a1 * raw;
+        fetch(ii + 1, i + g.xy());
+        if (s.active) cu.u[i] = v;
+    }
+};
+template <bool FUSE_P, bool REFLECT, bool UPD, typename Finish>
+static __global__ void __launch_bounds__(NT, TL3D_MINB) k3_cg_w(Geo g, Faces fc, Scalar beta, CgU cu,
                                                                const double* __restrict__ p_in, double* p_out,
                                                                const double* __restrict__ r, double* __restrict__ w,
                                                                const double* __restrict__ kx,
@@ -440,15 +486,29 @@ static __global__ void __launch_bounds__(NT, TL3D_MINB) k3_cg_w(Geo g, Faces fc,
     auto cur = [&](long idx) { return FUSE_P ? bt * p_in[idx] + r[idx] : p_in[idx]; };
     if (blockIdx.z + 1 < gridDim.z) {
         const PencilC s(g);
-        walkc<REFLECT>(g, fc, s, p_in, FUSE_P ? r : nullptr, kx, ky, kz,
-                       [&](double pa, double rb) { return FUSE_P ? bt * pa + rb : pa; },
-                       [&](int, long i, double c, double v) {
-            if (s.active) {
-                w[i] = v;
-                acc[0] += v * c;
-                if (FUSE_P) p_out[i] = c;
-            }
-        });
+        if constexpr (UPD) {
+            CgUWalk uw(cu, g, s);
+            walkc<REFLECT>(g, fc, s, p_in, FUSE_P ? r : nullptr, kx, ky, kz,
+                           [&](double pa, double rb) { return FUSE_P ? bt * pa + rb : pa; },
+                           [&](int ii, long i, double c, double v, double raw) {
+                               if (s.active) {
+                                   w[i] = v;
+                                   acc[0] += v * c;
+                                   p_out[i] = c;
+                               }
+                               uw.step(ii, i, raw);
+                           });
+        } else {
+            walkc<REFLECT>(g, fc, s, p_in, FUSE_P ? r : nullptr, kx, ky, kz,
+                           [&](double pa, double rb) { return FUSE_P ? bt * pa + rb : pa; },
+                           [&](int, long i, double c, double v) {
+                               if (s.active) {
+                                   w[i] = v;
+                                   acc[0] += v * c;
+                                   if (FUSE_P) p_out[i] = c;
+                               }
+                           });
+        }
     } else {
         if (REFLECT) halo_duty3(g, fc, 1, p_out, cur);
         if (u_halo) halo_duty3(g, fc, uhd, u_halo, [&](long idx) { return u_halo[idx]; });
@@ -458,8 +518,8 @@ static __global__ void __launch_bounds__(NT, TL3D_MINB) k3_cg_w(Geo g, Faces fc,
 
 // k3_cg_w with the operand planes brought in by TMA (walkt); the same
 // arithmetic, so the same results. `err`: the bounded barrier waits' flag.
-template <bool FUSE_P, bool REFLECT, typename Finish>
-static __global__ void __launch_bounds__(NT, TL3D_MINB) k3_cg_w_tma(Geo g, Faces fc, Scalar beta,
+template <bool FUSE_P, bool REFLECT, bool UPD, typename Finish>
+static __global__ void __launch_bounds__(NT, TL3D_MINB) k3_cg_w_tma(Geo g, Faces fc, Scalar beta, CgU cu,
                                                                    const __grid_constant__ Tma3Maps maps,
                                                                    const double* __restrict__ p_in, double* p_out,
                                                                    const double* __restrict__ r,
@@ -474,15 +534,29 @@ static __global__ void __launch_bounds__(NT, TL3D_MINB) k3_cg_w_tma(Geo g, Faces
     auto cur = [&](long idx) { return FUSE_P ? bt * p_in[idx] + r[idx] : p_in[idx]; };
     if (blockIdx.z + 1 < gridDim.z) {
         const PencilC s(g);
-        walkt<REFLECT>(g, fc, s, maps, FUSE_P, p_in, FUSE_P ? r : nullptr, t3_raw, err,
-                       [&](double pa, double rb) { return FUSE_P ? bt * pa + rb : pa; },
-                       [&](int, long i, double c, double v) {
-            if (s.active) {
-                w[i] = v;
-                acc[0] += v * c;
-                if (FUSE_P) p_out[i] = c;
-            }
-        });
+        if constexpr (UPD) {
+            CgUWalk uw(cu, g, s);
+            walkt<REFLECT>(g, fc, s, maps, FUSE_P, p_in, FUSE_P ? r : nullptr, t3_raw, err,
+                           [&](double pa, double rb) { return FUSE_P ? bt * pa + rb : pa; },
+                           [&](int ii, long i, double c, double v, double raw) {
+                               if (s.active) {
+                                   w[i] = v;
+                                   acc[0] += v * c;
+                                   p_out[i] = c;
+                               }
+                               uw.step(ii, i, raw);
+                           });
+        } else {
+            walkt<REFLECT>(g, fc, s, maps, FUSE_P, p_in, FUSE_P ? r : nullptr, t3_raw, err,
+                           [&](double pa, double rb) { return FUSE_P ? bt * pa + rb : pa; },
+                           [&](int, long i, double c, double v) {
+                               if (s.active) {
+                                   w[i] = v;
+                                   acc[0] += v * c;
+                                   if (FUSE_P) p_out[i] = c;
+                               }
+                           });
+        }
     } else {
         if (REFLECT) halo_duty3(g, fc, 1, p_out, cur);
         if (u_halo) halo_duty3(g, fc, uhd, u_halo, [&](long idx) { return u_halo[idx]; });
@@ -602,6 +676,123 @@ static __global__ void __launch_bounds__(NT, 4) k3_cg_ur_tma(Geo g, Scalar alpha
         }
     }
     tl::grid_sum<1, NT>(acc, rs, bx + gridDim.x * (by + gridDim.y * bz), block_count(), fin);
+}
+
+// CG sweep 2 where the w sweeps carry u (CgU): r -= alpha w ; rrn = sum(r r).
+// Pencils, planes and sums as k3_cg_ur.
+template <typename Finish>
+static __global__ void __launch_bounds__(NT, 8) k3_cg_r(Geo g, Scalar alpha, double* __restrict__ r,
+                                                        const double* __restrict__ w, ReduceSlots rs,
+                                                        const int* __restrict__ done, Finish fin)
+{
+    if (gate_closed(done)) return;
+    const int bx = ur3_b(blockIdx.x, gridDim.x), by = ur3_b(blockIdx.y, gridDim.y), bz = ur3_b(blockIdx.z, gridDim.z);
+    Pencil s(g, bx, by, bz);
+    double acc[1] = {0.0};
+    if (s.active) {
+        const double a = alpha.get();
+        const long xy = g.xy();
+        const long step = TL3D_UR_REVERSE ? -xy : xy;
+        long i = s.k + (long)s.j * g.x + (long)(TL3D_UR_REVERSE ? s.i1 - 1 : s.i0) * xy;
+        TL3D_PRAGMA_UNROLL(TL3D_UNROLL)
+        for (int n = 0; n < s.i1 - s.i0; ++n, i += step) {
+            const double rn = r[i] - a * w[i];
+            r[i] = rn;
+            acc[0] += rn * rn;
+        }
+    }
+    tl::grid_sum<1, NT>(acc, rs, bx + gridDim.x * (by + gridDim.y * bz), block_count(), fin);
+}
+
+// k3_cg_r with its operands brought in by TMA (as k3_cg_ur_tma): stages of
+// kPlanesU planes of r and w, 6 deep (49 KB, 4 blocks per SM).
+#ifndef TL3D_TMA_STAGES_R
+#define TL3D_TMA_STAGES_R 6
+#endif
+constexpr int kStagesR3 = TL3D_TMA_STAGES_R;
+struct PlanesR {
+    alignas(128) double R[kPlanesU][BY][BX];
+    alignas(128) double W[kPlanesU][BY][BX];
+};
+struct Tma3RMaps {
+    CUtensorMap r, w;
+};
+constexpr size_t kTmaR3Bytes = kStagesR3 * sizeof(PlanesR) + kStagesR3 * 8 + 128;
+
+template <typename Finish>
+static __global__ void __launch_bounds__(NT, 4) k3_cg_r_tma(Geo g, Scalar alpha, const __grid_constant__ Tma3RMaps maps,
+                                                         double* __restrict__ r, ReduceSlots rs,
+                                                         const int* __restrict__ done, Finish fin, int* err)
+{
+    extern __shared__ __align__(128) unsigned char r3_raw[];
+    if (gate_closed(done)) return;
+    unsigned char* base = r3_raw + ((128 - (tl::smem_addr(r3_raw) & 127)) & 127);
+    PlanesR* ring = reinterpret_cast<PlanesR*>(base);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kStagesR3 * sizeof(PlanesR));
+    const int bx = ur3_b(blockIdx.x, gridDim.x), by = ur3_b(blockIdx.y, gridDim.y), bz = ur3_b(blockIdx.z, gridDim.z);
+    Pencil s(g, bx, by, bz);
+    double acc[1] = {0.0};
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const bool leader = tx == 0 && ty == 0;
+    const int kb = g.hd + bx * BX, jb = g.hd + by * BY;
+    const int np = (s.i1 - s.i0 + kPlanesU - 1) / kPlanesU;
+    // stage b holds planes z0(b) .. z0(b) + kPlanesU - 1 (the pencil's last
+    // stage may run past i1; those planes are loaded and not used)
+    auto stage_z0 = [&](int b) { return s.i0 + (TL3D_UR_REVERSE ? np - 1 - b : b) * kPlanesU; };
+    auto issue = [&](int b) {
+        PlanesR& S = ring[b % kStagesR3];
+        unsigned long long* bar = &bars[b % kStagesR3];
+        tl::mbar_expect_tx(bar, 2u * sizeof(double) * kPlanesU * BY * BX);
+        tl::tma_load_3d(&S.R[0][0][0], &maps.r, kb, jb, stage_z0(b), bar);
+        tl::tma_load_3d(&S.W[0][0][0], &maps.w, kb, jb, stage_z0(b), bar);
+    };
+    if (leader) {
+        for (int q = 0; q < kStagesR3; ++q) tl::mbar_init(&bars[q], 1);
+        tl::mbar_fence_init();
+    }
+    __syncthreads();
+    if (leader)
+        for (int b = 0; b < kStagesR3 - 1 && b < np; ++b) issue(b);
+    const double a = alpha.get();
+    const long xy = g.xy();
+    for (int b = 0; b < np; ++b) {
+        __syncthreads();   // every thread is past stage b-1: its slot is free
+        if (leader && b + kStagesR3 - 1 < np) issue(b + kStagesR3 - 1);
+        tl::mbar_wait(&bars[b % kStagesR3], (unsigned)(b / kStagesR3) & 1u, err);
+        const PlanesR& S = ring[b % kStagesR3];
+        const int z0 = stage_z0(b);
+#pragma unroll
+        for (int q = 0; q < kPlanesU; ++q) {
+            const int t = TL3D_UR_REVERSE ? kPlanesU - 1 - q : q;   // planes in the order of k3_cg_r
+            const int ii = z0 + t;
+            if (ii >= s.i1) continue;
+            if (s.active) {
+                const double rn = S.R[t][ty][tx] - a * S.W[t][ty][tx];
+                r[s.k + (long)s.j * g.x + (long)ii * xy] = rn;
+                acc[0] += rn * rn;
+            }
+        }
+    }
+    // every issued stage was waited for: no copy in flight
+    tl::grid_sum<1, NT>(acc, rs, bx + gridDim.x * (by + gridDim.y * bz), block_count(), fin);
+}
+
+// u += alpha_{t-2} p_{t-2} [two], u += alpha_{t-1} p_{t-1}: the updates still due
+// after t trips.
+static __global__ void __launch_bounds__(NT) k3_cg_u_close(Geo g, double* __restrict__ u, const double* __restrict__ p2,
+                                                          const double* __restrict__ p1,
+                                                          const double* __restrict__ alphas, int t, int two)
+{
+    Pencil s(g);
+    if (!s.active) return;
+    const double a0 = two ? alphas[t - 2] : 0.0, a1 = alphas[t - 1];
+    const long xy = g.xy();
+    long i = s.k + (long)s.j * g.x + (long)s.i0 * xy;
+    for (int ii = s.i0; ii < s.i1; ++ii, i += xy) {
+        double v = u[i];
+        if (two) v += a0 * p2[i];
+        u[i] = v + a1 * p1[i];
+    }
 }
 
 // p = beta p + r (APPLY_P) and the depth-1 halos of p and (unless null) u.
@@ -893,7 +1084,7 @@ static __global__ void __launch_bounds__(FBX* FBY) k3_cg_init(Geo g, int coeffic
                                                              const double* __restrict__ density,
                                                              const double* __restrict__ energy, double* __restrict__ u,
                                                              double* __restrict__ p, double* __restrict__ p2,
-                                                             double* __restrict__ r, double* __restrict__ w,
+                                                             double* __restrict__ p3, double* __restrict__ r, double* __restrict__ w,
                                                              double* __restrict__ kx, double* __restrict__ ky,
                                                              double* __restrict__ kz, ReduceSlots rs, Finish fin)
 {
@@ -933,11 +1124,11 @@ static __global__ void __launch_bounds__(FBX* FBY) k3_cg_init(Geo g, int coeffic
             const double rr = uc - v;
             r[i] = rr;
             p[i] = rr;
-            if (p2) p2[i] = rr;
             acc[0] = rr * rr;
         } else {
             p[i] = 0.0;
             if (p2) p2[i] = 0.0;
+            if (p3) p3[i] = 0.0;
             r[i] = 0.0;
             if (ring) w[i] = wc;
         }

@@ -552,7 +552,7 @@ void run_cg_solver_init(Chunk* chunk, Settings* settings, double rx, double ry, 
     TL3_LAUNCH(s, "k3_cg_init",
                k3_cg_init<<<full_grid(s->g), full_block(), 0, s->stream>>>(
                    s->g, settings->coefficient, rx, ry, rz, chunk->density, chunk->energy, chunk->vec_u,
-                   chunk->vec_p, s->alt[ALT3_P], chunk->vec_r, chunk->vec_w, chunk->vec_kx, chunk->vec_ky,
+                   chunk->vec_p, s->alt[ALT3_P], nullptr, chunk->vec_r, chunk->vec_w, chunk->vec_kx, chunk->vec_ky,
                    chunk->vec_kz, s->rs, tl::NoFinish()));
     double o;
     if (fetch(s, 1, &o)) *rro += o;

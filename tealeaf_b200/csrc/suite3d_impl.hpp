@@ -229,14 +229,16 @@ static void launch_blocked3(TlSuite3D* s, Chunk* chunk, Blocked3Args a, const do
                             chunk->vec_kz, done)));
 }
 
-// The fused CG w sweep (k3_cg_w semantics), by TMA where possible.
-// Internal linkage, like the kernels it launches: each translation unit has
+// The fused CG w sweep (k3_cg_w semantics), by TMA where possible; U: with the
+// u updates of the two trips before it. Internal linkage, like the kernels it launches: each translation unit has
 // its own kernel copies, so each keeps its own record of the raised
 // shared-memory limit.
-template <bool F, bool R, typename Finish>
+template <bool F, bool R, bool U = false, typename Finish>
 static void launch_cg_w3(TlSuite3D* s, Chunk* chunk, dim3 grid, const Faces& fc, Scalar beta, const double* p_in,
-                  double* p_out, const double* r, double* w, double* u_halo, int uhd, const int* done, Finish fin)
+                  double* p_out, const double* r, double* w, double* u_halo, int uhd, const int* done, Finish fin,
+                  const CgU& cu = CgU{})
 {
+    const char* name = U ? "k3_cg_wu" : "k3_cg_w";
     const dim3 bl = interior_block();
     if (tma_usable(s)) {
         const CUtensorMap* a = tma_map(s, p_in, 0);
@@ -248,17 +250,17 @@ static void launch_cg_w3(TlSuite3D* s, Chunk* chunk, dim3 grid, const Faces& fc,
             const Tma3Maps m{*a, *b, *kx, *ky, *kz};
             static unsigned attr_set = 0;   // devices on which the shared-memory size was raised
             if (!(attr_set & (1u << (s->device & 31)))) {
-                TL_CUDA(cudaFuncSetAttribute(k3_cg_w_tma<F, R, Finish>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                TL_CUDA(cudaFuncSetAttribute(k3_cg_w_tma<F, R, U, Finish>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)kTmaRingBytes));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL3_LAUNCH(s, "k3_cg_w", (k3_cg_w_tma<F, R><<<grid, bl, kTmaRingBytes, s->stream>>>(
-                                         s->g, fc, beta, m, p_in, p_out, r, w, u_halo, uhd, s->rs, done, fin,
-                                         s->d_mirror + kTmaErrWord)));
+            TL3_LAUNCH(s, name, (k3_cg_w_tma<F, R, U><<<grid, bl, kTmaRingBytes, s->stream>>>(
+                                    s->g, fc, beta, cu, m, p_in, p_out, r, w, u_halo, uhd, s->rs, done, fin,
+                                    s->d_mirror + kTmaErrWord)));
             return;
         }
     }
-    TL3_LAUNCH(s, "k3_cg_w", (k3_cg_w<F, R><<<grid, bl, 0, s->stream>>>(s->g, fc, beta, p_in, p_out, r, w,
+    TL3_LAUNCH(s, name, (k3_cg_w<F, R, U><<<grid, bl, 0, s->stream>>>(s->g, fc, beta, cu, p_in, p_out, r, w,
                                                                       chunk->vec_kx, chunk->vec_ky, chunk->vec_kz,
                                                                       u_halo, uhd, s->rs, done, fin)));
 }
@@ -289,6 +291,71 @@ static void launch_cg_ur3(TlSuite3D* s, dim3 grid, Scalar alpha, double* u, cons
         }
     }
     TL3_LAUNCH(s, "k3_cg_ur", (k3_cg_ur<<<grid, bl, 0, s->stream>>>(s->g, alpha, u, p, r, w, s->rs, done, fin)));
+}
+
+// The fused CG r update (k3_cg_r semantics), by TMA where possible.
+template <typename Finish>
+static void launch_cg_r3(TlSuite3D* s, dim3 grid, Scalar alpha, double* r, const double* w, const int* done, Finish fin)
+{
+    const dim3 bl = interior_block();
+    if (tma_usable(s)) {
+        const CUtensorMap* mr = tma_map(s, r, 4);
+        const CUtensorMap* mw = tma_map(s, w, 4);
+        if (mr && mw) {
+            const Tma3RMaps m{*mr, *mw};
+            static unsigned attr_set = 0;   // devices on which the shared-memory size was raised
+            if (!(attr_set & (1u << (s->device & 31)))) {
+                TL_CUDA(cudaFuncSetAttribute(k3_cg_r_tma<Finish>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kTmaR3Bytes));
+                attr_set |= 1u << (s->device & 31);
+            }
+            TL3_LAUNCH(s, "k3_cg_r", (k3_cg_r_tma<<<grid, bl, kTmaR3Bytes, s->stream>>>(
+                                         s->g, alpha, m, r, s->rs, done, fin, s->d_mirror + kTmaErrWord)));
+            return;
+        }
+    }
+    TL3_LAUNCH(s, "k3_cg_r", (k3_cg_r<<<grid, bl, 0, s->stream>>>(s->g, alpha, r, w, s->rs, done, fin)));
+}
+
+// The CG loop of a mesh that does not fit on chip, its solution in u: the w
+// sweep of every second trip applies the u updates of the two trips before it
+// (CgU), so p goes round three buffers, the third the suite's second sd buffer
+// (unused by CG; cg_init has cleared its halo as p's). loop(trip) launches the
+// trips trip(0), ... and returns the state they end in.
+template <typename Loop>
+static DevState cg_deferred3(TlSuite3D* s, Chunk* chunk, double* u, const DevParams& prm, Loop loop)
+{
+    double* buf[3] = {chunk->vec_p, s->alt[ALT3_P], s->alt[ALT3_SD]};   // trip t's p is buf[t % 3]
+    const Faces fc = faces_of(chunk);
+    const dim3 gi = interior_grid(s->g), gh = fused_grid(s->g);
+    const int* done = &s->d_state->done;
+    const tl::FinCgW fin_w{s->d_state, s->d_cg_alphas};
+    const tl::FinCgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
+    const Scalar beta{0.0, &s->d_state->beta}, alpha{0.0, &s->d_state->alpha};
+    const DevState st = loop([&](int t) {
+        double* const p = buf[t % 3];
+        const double* const p1 = buf[(t + 2) % 3];
+        if (t == 0)
+            launch_cg_w3<false, false>(s, chunk, gh, fc, beta, p, p, chunk->vec_r, chunk->vec_w, nullptr, 0, done,
+                                       fin_w);
+        else if (t % 2 == 0)
+            launch_cg_w3<true, true, true>(s, chunk, gh, fc, beta, p1, p, chunk->vec_r, chunk->vec_w, nullptr, 0, done,
+                                           fin_w, CgU{u, buf[(t + 1) % 3], s->d_cg_alphas, t});
+        else
+            launch_cg_w3<true, true>(s, chunk, gh, fc, beta, p1, p, chunk->vec_r, chunk->vec_w, nullptr, 0, done,
+                                     fin_w);
+        launch_cg_r3(s, gi, alpha, chunk->vec_r, chunk->vec_w, done, fin_ur);
+    });
+    const int t = st.trip;   // trips that ran: t - 1 is the last
+    if (t > 0) {
+        TL3_LAUNCH(s, "k3_cg_u_close", (k3_cg_u_close<<<gi, interior_block(), 0, s->stream>>>(
+                                           s->g, u, buf[(t + 1) % 3], buf[(t + 2) % 3], s->d_cg_alphas, t,
+                                           t % 2 == 0 ? 1 : 0)));
+        chunk->vec_p = buf[(t + 2) % 3];
+        s->alt[ALT3_P] = buf[t % 3];
+        s->alt[ALT3_SD] = buf[(t + 1) % 3];
+    }
+    return st;
 }
 
 // Tensor maps of a stencil sweep over operands a (and b) with the chunk's
