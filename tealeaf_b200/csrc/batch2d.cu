@@ -25,7 +25,11 @@
 // and the largest problems get the whole grid once the small ones have
 // converged. A block holds at most one tile and never waits while holding
 // it; only a block that finds no tile anywhere polls, bounded by a clock
-// limit (a timeout sets an error word and the blocks return). Per-problem
+// limit (a timeout sets an error word and the blocks return). Taking a tile
+// costs two L2 round trips: one load that brings every schedule and its
+// scalar, one atomic that hands out the tile and says of which phase (a poll,
+// a draw, a fence and three loads were 5500 cycles; closing a phase 7700,
+// 5500 with the scalars fetched beside the partials). Per-problem
 // dot products are reduced deterministically: each tile writes its block
 // sum, and the block finishing the problem's last tile of the phase sums
 // the problem's tile partials in tile order and runs the CG scalar update
@@ -49,14 +53,25 @@ using namespace tl2d::rf;
 namespace {
 
 // Arithmetic of the batch's FP32 sweeps (dot products and scalars are FP64
-// either way): FP32 (TL2D_BATCH_MATH_F32 1; 785 against 846 ms for the
+// either way): FP32 (TL2D_BATCH_MATH_F32 1; with plain loads 785 against 846 ms for the
 // 64-problem step, the same iterations) or FP64 on the FP32 values (0).
 #ifndef TL2D_BATCH_MATH_F32
 #define TL2D_BATCH_MATH_F32 1
 #endif
 using BatchM = std::conditional_t<TL2D_BATCH_MATH_F32 != 0, float, double>;
 
-constexpr int kBatchMinB = 8;                    // resident blocks per SM of the persistent kernel
+// The persistent kernel's two forms. A batch whose FP32 arrays fit L2 is bound
+// by the latency of a phase -- a tile's rows, its dot product, the next phase's
+// opening, twice an iteration -- and runs best with few blocks per SM, each with
+// many registers and rows in flight; one that streams from HBM wants as many
+// rows in flight per SM as shared memory holds. One step, 4 x 8 against 6 x 6
+// (blocks per SM x rows): 24 problems of sides 64-768 (66 MB of arrays) 25.5
+// against 28.3 ms, 64-1100 (90 MB) 39.3 / 42.2; 128-1400 (190 MB) 90.8 / 87.8,
+// 200 of 64-400 (180 MB) 40.3 / 36.5, the 64 of 128-2048 (900 MB) 620 / 579;
+// 8 x 6, with 64 registers a thread: 30.0, 49.8, 97.8, 36.1, 582.
+struct Resident { static constexpr int MINB = 4, STAGES = 8; };
+struct Streaming { static constexpr int MINB = 6, STAGES = 6; };
+constexpr int kGroupsPerSm = 8;                  // blocks per SM that the problems' groups are cut for
 constexpr long long kWaitLimit = 4000000000LL;   // default: SM clocks a phase wait may take (~2 s)
 
 enum { BF_KX = 0, BF_KY, BF_P0, BF_P1, BF_W, BF_R, BF_XS, BF_COUNT };
@@ -65,7 +80,7 @@ struct BProb {
     Lay L;
     int tx, ty;      // tiles per row / column
     int tile0;       // first global tile of this problem
-    int g0, gsize;   // the problem's group: blocks g0 .. g0 + gsize - 1
+    int gsize;       // blocks of the problem's group
     int gx, hd;      // FP64 chunk arrays: row length, halo depth
     float* f[BF_COUNT];
     double* u;
@@ -80,53 +95,351 @@ struct BCtl {
     long long limit;  // SM clocks a block may go without a tile before it gives up (kept across steps)
 };
 
-// Per-problem schedule of the persistent kernel. One 64-bit word holds the
-// open phase (high half) and the tiles handed out in it (low half): a block
-// takes tile t with one atomic add and holds a tile of that phase exactly
-// when t < tiles per phase. The block completing the phase's last tile runs
-// the phase's scalar update, writes the next phase's kind and iteration and
-// opens it by swapping in (phase + 1) << 32; a finished problem's low half
-// is kClosed, so every later draw comes back void. A block never waits
-// while it holds a tile: when its problem has no tile left in the open
-// phase it takes one from the problem with the most tiles left, and only
-// when no problem has one does it poll (bounded by the clock limit).
+// Per-problem schedule of the persistent kernel: the open phase (iteration and
+// kind, high half of `word`), the tiles left to hand out in it (low half, above
+// kNone) and the phase's scalar. A block takes a tile with one atomic
+// subtraction and holds tile (left - 1) of that phase exactly when `left` was
+// above kNone; what the phase is comes back with it. The block completing the
+// phase's last tile runs the phase's scalar update, writes the next phase's
+// scalar and opens it by swapping in its word; a finished problem has kind
+// PH_DONE and no tiles. A block never waits while it holds a tile: when its
+// problem has no tile left in the open phase it takes one from the problem with
+// the most tiles left, and only when no problem has one does it poll (bounded by
+// the clock limit). A schedule has a 128-byte line to itself: polls of one and
+// draws from another would serialise on a shared line.
 enum { PH_W = 0, PH_UR = 1, PH_FOLD = 2, PH_RESID = 3, PH_DONE = 4 };
-constexpr unsigned kClosed = 0x40000000u;
-struct PCtl {
-    unsigned long long word;   // open phase << 32 | tiles handed out in it
-    int kind;                  // kind of the open phase
-    int it;                    // CG iteration of the open phase
+constexpr unsigned kNone = 0x40000000u;   // failed draws take the low half below it
+struct alignas(128) PCtl {
+    double coef;               // beta (PH_W) or alpha (PH_UR) of the open phase
+    unsigned long long word;   // (iteration << 3 | kind) << 32 | kNone + tiles left
+};
+__device__ __forceinline__ unsigned long long phase_word(int it, int kind, int tiles)
+{
+    return (unsigned long long)((unsigned)it << 3 | (unsigned)kind) << 32 | (kNone + (unsigned)(kind == PH_DONE ? 0 : tiles));
+}
+__device__ __forceinline__ int tiles_left(unsigned long long word) { return (int)((unsigned)word - kNone); }
+__device__ __forceinline__ unsigned phase_of(unsigned long long word) { return (unsigned)(word >> 32); }
+
+// The scalar and the word of a schedule in one 16-byte load. A draw that then
+// finds the same phase open may use the scalar: the next phase's is written
+// only once every tile of this one has been handed out and completed.
+__device__ __forceinline__ unsigned long long sched_load(const PCtl* s, double& coef)
+{
+    unsigned long long lo, hi;
+    asm volatile(
+        "{\n"
+        ".reg .b128 q;\n"
+        "ld.relaxed.gpu.global.b128 q, [%2];\n"
+        "mov.b128 {%0, %1}, q;\n"
+        "}\n"
+        : "=l"(lo), "=l"(hi)
+        : "l"(s)
+        : "memory");
+    coef = __longlong_as_double((long long)lo);
+    return hi;
+}
+// What the phase's opener published is visible after the draw.
+__device__ __forceinline__ unsigned long long sched_draw(PCtl* s)
+{
+    unsigned long long old;
+    asm volatile("atom.add.acquire.gpu.global.u64 %0, [%1], %2;" : "=l"(old) : "l"(&s->word), "l"(~0ull) : "memory");
+    return old;
+}
+__device__ __forceinline__ void sched_open(PCtl* s, double coef, unsigned long long word)
+{
+    unsigned long long old;
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(&s->coef), "d"(coef) : "memory");
+    asm volatile("atom.exch.release.gpu.global.b64 %0, [%1], %2;" : "=l"(old) : "l"(&s->word), "l"(word) : "memory");
+}
+
+// Rows of a tile on their way from L2 to shared memory: every thread holds two
+// cells of up to four arrays a row; of a pair of lanes the even one copies the
+// pair's 16 bytes of the first two arrays, the odd one those of the other two,
+// so a warp waits for its own copies only. Plain loads waited for L2 row by row
+// (16-row tiles: 18200 cycles for the w sweep, 10500 for the u/r update) because
+// a row's stores, which might alias, hold back the next row's loads; the copies
+// need no registers and are issued STAGES rows ahead (7200 and 4000 cycles on a
+// quiet SM).
+struct alignas(128) RingRow {
+    float2 cell[4][BX];         // [array][thread]
+    float4 edge[3][BX / 16];    // [array][2 * warp + side]: the columns beside a warp's
 };
 
-__device__ __forceinline__ unsigned long long vol_read64(const unsigned long long* p)
+__device__ __forceinline__ unsigned ring_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ring_copy(unsigned to, const float* from)
 {
-    return *(volatile const unsigned long long*)p;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to), "l"(from) : "memory");
+}
+__device__ __forceinline__ Cells<float> ring_read(unsigned at)
+{
+    Cells<float> c;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(c.e[0]), "=f"(c.e[1]) : "r"(at) : "memory");
+    return c;
+}
+__device__ __forceinline__ float ring_read1(unsigned at)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+// Rows are waited for two at a time; each pair commits one group, an empty one
+// past the tile's end, so that a pair has arrived once at most ST / 2 - 1 groups
+// are pending.
+__device__ __forceinline__ void ring_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int ST>
+__device__ __forceinline__ void ring_wait()
+{
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(ST / 2 - 1) : "memory");
+    __syncwarp();
+}
+constexpr unsigned kRow = sizeof(RingRow), kArr = sizeof(float2) * BX, kEdgeArr = sizeof(float4) * (BX / 16);
+template <int ST>
+__device__ __forceinline__ unsigned ring_after(unsigned slot)   // slot: byte offset of a pair of rows
+{
+    return slot == (ST - 2) * kRow ? 0u : slot + 2 * kRow;
+}
+
+// CG sweep 1 over tile (tx, ty): [p = bt p + r], w = A p; returns this thread's
+// share of sum(w p). The arithmetic and its order are rf_w_tile's.
+template <int ST, bool FUSE_P>
+__device__ __forceinline__ double batch_w_tile(RingRow* R, const Lay& L, int tx, int ty, double bt_,
+                                               const float* __restrict__ p_in, float* __restrict__ p_out,
+                                               const float* __restrict__ r, float* __restrict__ w,
+                                               const float* __restrict__ kx, const float* __restrict__ ky)
+{
+    using M = BatchM;
+    constexpr int N = Pack<float>::N;
+    const Span<N> s(L, tx, ty);
+    const M bt = (M)bt_;
+    const unsigned xp = (unsigned)L.xp;
+    const int rows = s.j1 - s.j0;
+    const bool first = s.lane == 0, final = s.lane == 31, odd = s.lane & 1, end = first || final;
+    const bool in0 = s.c0 < L.nx, in1 = s.c0 + 1 < L.nx;
+    const int c4 = min(s.c0 & ~3, L.xp - 4);   // the pair's four columns
+    const int pair = threadIdx.x & ~1;
+    const unsigned to = ring_addr(&R[0].cell[odd ? 2 : 0][pair]);
+    const unsigned me = ring_addr(&R[0].cell[0][pair + ((s.cc - c4) >> 1)]);
+    const unsigned ed = ring_addr(&R[0].edge[0][2 * (threadIdx.x >> 5) + (final ? 1 : 0)]);
+    const unsigned near = ed + (final ? 0u : 12u);   // of the edge's four columns, the neighbour
+    // row k of rows + 2: p, r (and ky from the tile's own first row on) of row
+    // j0 - 1 + k, kx of the row before it, which is the one the operator is at
+    const float* const one = (odd ? ky : p_in) + c4;
+    const float* const two = (odd ? kx : r) + c4;
+    const float* const pe_in = p_in + c4 + (final ? 4 : -4);
+    const float* const re_in = r + c4 + (final ? 4 : -4);
+    const float* const ke_in = kx + c4 + 4;
+    unsigned g = (unsigned)s.j0 * xp;   // of the next row to fill
+    int k = 0;
+    auto fill = [&](unsigned at) {
+        if (k < rows + 2) {
+            if (!odd || k > 0) ring_copy(to + at, one + g);
+            if (odd) {
+                if (k > 1) ring_copy(to + at + kArr, two + (g - xp));
+            } else if (FUSE_P) {
+                ring_copy(to + at + kArr, two + g);
+            }
+            if (end) {
+                if (k > 0 && k <= rows) {   // the tile's own rows only
+                    ring_copy(ed + at, pe_in + g);
+                    if (FUSE_P) ring_copy(ed + at + kEdgeArr, re_in + g);
+                }
+                if (final && k > 1) ring_copy(ed + at + 2 * kEdgeArr, ke_in + (g - xp));
+            }
+        }
+        ++k;
+        g += xp;
+    };
+    auto fill2 = [&](unsigned at) {
+        fill(at);
+        fill(at + kRow);
+        ring_commit();
+    };
+    struct Row {
+        Cells<float> p, q, ky, kx;
+        float pe, qe, ke;
+    };
+    auto read = [&](unsigned at, Row& v) {
+        v.p = ring_read(me + at);
+        if (FUSE_P) v.q = ring_read(me + at + kArr);
+        v.ky = ring_read(me + at + 2 * kArr);
+        v.kx = ring_read(me + at + 3 * kArr);
+        v.pe = v.qe = v.ke = 0.f;
+        if (end) {
+            v.pe = ring_read1(near + at);
+            if (FUSE_P) v.qe = ring_read1(near + at + kEdgeArr);
+            v.ke = ring_read1(near + at + 2 * kEdgeArr);
+        }
+    };
+    auto fold = [&](Row& v) {
+        if (FUSE_P) {
+#pragma unroll
+            for (int m = 0; m < N; ++m) v.p.e[m] = (float)(bt * (M)v.p.e[m] + (M)v.q.e[m]);
+            v.pe = (float)(bt * (M)v.pe + (M)v.qe);
+        }
+    };
+    unsigned slot = 0;
+#pragma unroll
+    for (int c = 0; c < ST; c += 2) fill2(c * kRow);
+    double acc = 0.0;
+    Cells<float> pd{}, pc{}, kyc{};
+    float pe = 0.f;
+    unsigned i = ((unsigned)s.j0 + 1) * xp + s.cc;
+    auto step = [&](const Row& v) {   // the operator at (pc, kyc, pe), v the row above
+        float pl = __shfl_up_sync(kFull, pc.e[N - 1], 1);
+        float pr = __shfl_down_sync(kFull, pc.e[0], 1);
+        float kxr = __shfl_down_sync(kFull, v.kx.e[0], 1);
+        if (first) pl = pe;
+        if (final) {
+            pr = pe;
+            kxr = v.ke;
+        }
+        Cells<float> wv;
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            const M c = (M)pc.e[m];
+            const M l = m == 0 ? (M)pl : (M)pc.e[m - 1];
+            const M rr = m == N - 1 ? (M)pr : (M)pc.e[m + 1];
+            const M kr = m == N - 1 ? (M)kxr : (M)v.kx.e[m + 1];
+            wv.e[m] = (float)smvp_m<M>((M)v.kx.e[m], kr, (M)kyc.e[m], (M)v.ky.e[m], c, l, rr, (M)pd.e[m],
+                                       (M)v.p.e[m]);
+        }
+        if (s.any) {
+            st8(w + i, wv);
+            if (FUSE_P) st8(p_out + i, pc);
+        }
+        if (in0) acc += (double)wv.e[0] * (double)pc.e[0];
+        if (in1) acc += (double)wv.e[1] * (double)pc.e[1];
+        pd = pc;
+        pc = v.p;
+        kyc = v.ky;
+        pe = v.pe;
+        i += xp;
+    };
+    Row a, b;
+    auto take2 = [&]() {
+        ring_wait<ST>();
+        read(slot, a);
+        read(slot + kRow, b);
+        __syncwarp();
+        fill2(slot);
+        slot = ring_after<ST>(slot);
+        fold(a);
+        fold(b);
+    };
+    take2();
+    pd = a.p;
+    pc = b.p;
+    kyc = b.ky;
+    pe = b.pe;
+    for (int j = 0; j < rows; j += 2) {
+        take2();
+        step(a);
+        if (j + 1 < rows) step(b);
+    }
+    return acc;
+}
+
+// CG sweep 2 over tile (tx, ty): xs += a p, r -= a w; returns this thread's
+// share of sum(r r). The arithmetic and its order are rf_ur_tile's.
+template <int ST>
+__device__ __forceinline__ double batch_ur_tile(RingRow* R, const Lay& L, int tx, int ty, double a_,
+                                                float* __restrict__ xs, const float* __restrict__ p,
+                                                float* __restrict__ r, const float* __restrict__ w)
+{
+    using M = BatchM;
+    constexpr int N = Pack<float>::N;
+    const Span<N> s(L, tx, ty);
+    if (!__any_sync(kFull, s.any)) return 0.0;
+    const M al = (M)a_;
+    const unsigned xp = (unsigned)L.xp;
+    const int rows = s.j1 - s.j0;
+    const bool odd = s.lane & 1, in0 = s.c0 < L.nx, in1 = s.c0 + 1 < L.nx;
+    const int pair = threadIdx.x & ~1;
+    const int c4 = min(s.c0 & ~3, L.xp - 4);
+    const unsigned to = ring_addr(&R[0].cell[odd ? 2 : 0][pair]);
+    const unsigned me = ring_addr(&R[0].cell[0][pair + ((s.cc - c4) >> 1)]);
+    const float* const one = (odd ? p : xs) + c4;
+    const float* const two = (odd ? w : r) + c4;
+    unsigned g = ((unsigned)s.j0 + 1) * xp, i = g + s.cc;
+    int k = 0;
+    auto fill2 = [&](unsigned at) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q, ++k, g += xp)
+            if (k < rows) {
+                ring_copy(to + at + q * kRow, one + g);
+                ring_copy(to + at + q * kRow + kArr, two + g);
+            }
+        ring_commit();
+    };
+#pragma unroll
+    for (int c = 0; c < ST; c += 2) fill2(c * kRow);
+    double acc = 0.0;
+    unsigned slot = 0;
+    struct Row {
+        Cells<float> xs, r, p, w;
+    };
+    auto read = [&](unsigned at, Row& v) {
+        v.xs = ring_read(me + at);
+        v.r = ring_read(me + at + kArr);
+        v.p = ring_read(me + at + 2 * kArr);
+        v.w = ring_read(me + at + 3 * kArr);
+    };
+    auto step = [&](Row& v) {
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            v.xs.e[m] = (float)((M)v.xs.e[m] + al * (M)v.p.e[m]);
+            v.r.e[m] = (float)((M)v.r.e[m] - al * (M)v.w.e[m]);
+        }
+        if (s.any) {
+            st8(xs + i, v.xs);
+            st8(r + i, v.r);
+        }
+        if (in0) acc += (double)v.r.e[0] * (double)v.r.e[0];
+        if (in1) acc += (double)v.r.e[1] * (double)v.r.e[1];
+        i += xp;
+    };
+    for (int j = 0; j < rows; j += 2) {
+        Row a, b;
+        ring_wait<ST>();
+        read(slot, a);
+        read(slot + kRow, b);
+        __syncwarp();
+        fill2(slot);
+        slot = ring_after<ST>(slot);
+        step(a);
+        if (j + 1 < rows) step(b);
+    }
+    return acc;
 }
 
 // Block sum of this thread's values; returns true in every thread of the
-// block that completed problem b's last tile of the phase, with the
-// problem's totals (fixed-order sum of its tile partials) in tot (thread 0).
+// block that completed the problem's last tile of the phase, with the
+// problem's totals (fixed-order sum of its tile partials) in tot (thread 0)
+// and its scalars in cp, fetched beside the partials.
 template <int N>
 __device__ bool tile_done(double (&v)[N], int t, const BProb& P, unsigned* ticket, double* partials,
-                          double (&tot)[N])
+                          const MxState* st, MxState& cp, double (&tot)[N])
 {
+    constexpr int kWords = sizeof(MxState) / sizeof(double);
+    static_assert(sizeof(MxState) % sizeof(double) == 0 && kWords <= BX, "one word per thread");
     __shared__ double smem[N][BX / tl::kWarp];
     __shared__ bool last;
+    const int nt = P.tx * P.ty;
     __syncthreads();
     tl::block_sum<N, BX>(v, smem);
     if (threadIdx.x == 0) {
+        unsigned before;
 #pragma unroll
         for (int r = 0; r < N; ++r) partials[(long)t * 2 + r] = v[r];
-        __threadfence();
-        last = atomicAdd(ticket, 1u) == (unsigned)(P.tx * P.ty - 1);
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(ticket) : "memory");
+        last = before == (unsigned)(nt - 1);
     }
     __syncthreads();
     if (!last) return false;
-    __threadfence();
+    if (threadIdx.x < kWords) ((double*)&cp)[threadIdx.x] = __ldcg((const double*)st + threadIdx.x);
     double s[N];
 #pragma unroll
     for (int r = 0; r < N; ++r) s[r] = 0.0;
-    const int nt = P.tx * P.ty;
     // partials k = tid, tid + BX, ... added in that order; four loads in flight
     for (int k0 = threadIdx.x; k0 < nt; k0 += 4 * BX) {
         double q[4][N];
@@ -151,152 +464,155 @@ __device__ bool tile_done(double (&v)[N], int t, const BProb& P, unsigned* ticke
     return true;
 }
 
-// Warp 0: the unfinished problem with the most tiles not yet handed out in
-// its open phase (the lowest index among equals); -1 when every problem has
-// finished, -2 when none has a tile to hand out right now.
-__device__ int find_work(const BProb* __restrict__ P, PCtl* pc, int np)
+// Warp 0: draws a tile of problem b, or, when it has none left in its open
+// phase, of the problem with the most tiles left. 1 with b, t, phase and coef
+// set; 0 when no problem has a tile right now; -1 when every problem has
+// finished. The first 32 problems looked at, b among them, cost one round trip.
+__device__ __forceinline__ int find_tile(PCtl* pc, int np, int& b, int& t, unsigned& phase, double& coef)
 {
+    constexpr int kOwn = 0x3fffffff;
     const int lane = threadIdx.x & 31;
     int best = 0, who = -1;
+    unsigned seen = 0;
+    double c = 0.0;
     bool live = false;
-    for (int b = lane; b < np; b += 32) {
-        const unsigned lo = (unsigned)vol_read64(&pc[b].word);
-        if (lo >= kClosed) continue;
-        live = true;
-        const unsigned nt = (unsigned)(P[b].tx * P[b].ty);
-        if (lo < nt && (int)(nt - lo) > best) {
-            best = (int)(nt - lo);
-            who = b;
+    for (int k0 = 0; k0 < np; k0 += 32) {
+        const int k = k0 + lane, q = b + k < np ? b + k : b + k - np;
+        if (k < np) {
+            double cq;
+            const unsigned long long word = sched_load(&pc[q], cq);
+            live |= (phase_of(word) & 7u) != PH_DONE;
+            int left = tiles_left(word);
+            if (left > 0 && k == 0) left = kOwn;   // its own problem first
+            if (left > best) {
+                best = left;
+                who = q;
+                seen = phase_of(word);
+                c = cq;
+            }
         }
+        if (__any_sync(0xffffffffu, best == kOwn)) break;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const int ob = __shfl_down_sync(0xffffffffu, best, o);
-        const int ow = __shfl_down_sync(0xffffffffu, who, o);
-        if (ob > best || (ob == best && ow >= 0 && (who < 0 || ow < who))) {
-            best = ob;
-            who = ow;
-        }
+    if (!__any_sync(0xffffffffu, live)) return -1;
+    const int most = __reduce_max_sync(0xffffffffu, best);
+    if (most <= 0) return 0;
+    const int from = __ffs(__ballot_sync(0xffffffffu, best == most)) - 1;
+    int got = 0;
+    if (lane == from) {
+        const unsigned long long word = sched_draw(&pc[who]);
+        t = tiles_left(word) - 1;
+        phase = phase_of(word);
+        got = t >= 0;
+        coef = c;
+        if (got && phase != seen) sched_load(&pc[who], coef);
     }
-    who = __shfl_sync(0xffffffffu, who, 0);
-    live = __any_sync(0xffffffffu, live);
-    return who >= 0 ? who : (live ? -2 : -1);
+    got = __shfl_sync(0xffffffffu, got, from);
+    if (got) {
+        b = __shfl_sync(0xffffffffu, who, from);
+        t = __shfl_sync(0xffffffffu, t, from);
+        phase = __shfl_sync(0xffffffffu, phase, from);
+        coef = __shfl_sync(0xffffffffu, coef, from);
+    }
+    return got;
 }
 
-// Thread 0: draws a tile of problem b; true with its index in t and the
-// phase in g when one was left in the open phase.
-__device__ __forceinline__ bool draw(const BProb* __restrict__ P, PCtl* pc, int b, int& t, unsigned& g)
+// K: Resident or Streaming.
+template <typename K>
+__global__ void __launch_bounds__(BX, K::MINB) k_batch_cg(const BProb* __restrict__ P, int np,
+                                                          const int* __restrict__ block_prob, MxState* st,
+                                                          unsigned* tickets, double* partials, PCtl* pc,
+                                                          BCtl* ctl, int max_iters)
 {
-    const unsigned nt = (unsigned)(P[b].tx * P[b].ty);
-    const unsigned long long old = atomicAdd(&pc[b].word, 1ull);
-    if ((unsigned)old >= nt) return false;
-    t = (int)(unsigned)old;
-    g = (unsigned)(old >> 32);
-    return true;
-}
-
-__global__ void __launch_bounds__(BX, kBatchMinB) k_batch_cg(const BProb* __restrict__ P, int np,
-                                                             const int* __restrict__ block_prob, MxState* st,
-                                                             unsigned* tickets, double* partials, PCtl* pc,
-                                                             BCtl* ctl, int max_iters)
-{
-    __shared__ int sh_go, sh_b, sh_t, sh_kind, sh_it;
-    __shared__ unsigned sh_g;
+    // 128-byte lines: the copies of a warp take a third longer across them
+    extern __shared__ __align__(128) unsigned char ring_bytes[];
+    RingRow* const ring = reinterpret_cast<RingRow*>(ring_bytes);
+    __shared__ int sh_go, sh_b, sh_t;
+    __shared__ unsigned sh_phase;
     __shared__ double sh_coef;
-    int b = block_prob[blockIdx.x];
+    __shared__ BProb Q;       // the problem of the block's tile
+    __shared__ MxState cp;
+    int b = block_prob[blockIdx.x], have = -1;
+    const long long limit = ctl->limit;
     long long idle0 = clock64();
     for (;;) {
         if (threadIdx.x < 32) {
-            int go = 0, t = 0;   // 1: a tile of problem b, 0: none right now, -1: leave
-            unsigned g = 0;
-            if (threadIdx.x == 0 && (unsigned)vol_read64(&pc[b].word) < (unsigned)(P[b].tx * P[b].ty))
-                go = draw(P, pc, b, t, g) ? 1 : 0;
-            go = __shfl_sync(0xffffffffu, go, 0);
-            if (go == 0) {
-                const int nb = find_work(P, pc, np);
-                if (threadIdx.x == 0) {
-                    if (nb == -1) {
-                        go = -1;
-                    } else if (nb >= 0 && draw(P, pc, nb, t, g)) {
-                        go = 1;
-                        b = nb;
-                    }
+            int t = 0;
+            unsigned phase = 0;
+            double coef = 0.0;
+            const int err = vol_read(&ctl->err);   // under way beside the schedules
+            int go = find_tile(pc, np, b, t, phase, coef);
+            if (go == 1) {
+                idle0 = clock64();
+            } else if (go == 0) {
+                if (err) {
+                    go = -1;
+                } else if (clock64() - idle0 > limit) {
+                    if (threadIdx.x == 0) atomicExch(&ctl->err, 1);
+                    go = -1;
+                } else {
+                    __nanosleep(64);
                 }
+                go = __shfl_sync(0xffffffffu, go, 0);
             }
             if (threadIdx.x == 0) {
-                if (go == 1) {
-                    __threadfence();   // the phase's kind, scalars and fields are those its opener published
-                    idle0 = clock64();
-                    const int kind = vol_read(&pc[b].kind);
-                    sh_kind = kind;
-                    sh_it = vol_read(&pc[b].it);
-                    sh_coef = kind == PH_W ? __ldcg(&st[b].beta) : kind == PH_UR ? __ldcg(&st[b].alpha) : 0.0;
-                } else if (go == 0) {
-                    if (vol_read(&ctl->err)) {
-                        go = -1;
-                    } else if (clock64() - idle0 > ctl->limit) {
-                        atomicExch(&ctl->err, 1);
-                        go = -1;
-                    } else {
-                        __nanosleep(64);
-                    }
-                }
                 sh_go = go;
                 sh_b = b;
                 sh_t = t;
-                sh_g = g;
+                sh_phase = phase;
+                sh_coef = coef;
             }
         }
         __syncthreads();
-        const int go = sh_go, lt = sh_t, kind = sh_kind, it = sh_it;
-        const unsigned g = sh_g;
+        const int go = sh_go, lt = sh_t, kind = sh_phase & 7u, it = sh_phase >> 3;
         const double coef = sh_coef;
         b = sh_b;
+        if (go == 1 && b != have) {
+            static_assert(sizeof(BProb) % sizeof(int) == 0 && sizeof(BProb) / sizeof(int) <= BX, "one word per thread");
+            if (threadIdx.x < sizeof(BProb) / sizeof(int)) ((int*)&Q)[threadIdx.x] = ((const int*)&P[b])[threadIdx.x];
+            have = b;
+        }
         __syncthreads();   // sh_* are rewritten by the next pass
         if (go < 0) return;
         if (go == 0) continue;
-        const BProb& Q = P[b];
         const int tx = lt % Q.tx, ty = lt / Q.tx;
         double v[2] = {0.0, 0.0};
         if (kind == PH_W) {
             float* pin = Q.f[it == 0 ? BF_P0 : (((it - 1) & 1) ? BF_P1 : BF_P0)];
             float* pout = Q.f[(it & 1) ? BF_P1 : BF_P0];
-            v[0] = it == 0 ? rf_w_tile<float, false, true, BatchM>(Q.L, tx, ty, 0.0, pin, pin, Q.f[BF_R],
-                                                                    Q.f[BF_W], Q.f[BF_KX], Q.f[BF_KY])
-                           : rf_w_tile<float, true, true, BatchM>(Q.L, tx, ty, coef, pin, pout, Q.f[BF_R],
-                                                                   Q.f[BF_W], Q.f[BF_KX], Q.f[BF_KY]);
+            v[0] = it == 0 ? batch_w_tile<K::STAGES, false>(ring, Q.L, tx, ty, 0.0, pin, pin, Q.f[BF_R], Q.f[BF_W],
+                                                  Q.f[BF_KX], Q.f[BF_KY])
+                           : batch_w_tile<K::STAGES, true>(ring, Q.L, tx, ty, coef, pin, pout, Q.f[BF_R], Q.f[BF_W],
+                                                 Q.f[BF_KX], Q.f[BF_KY]);
         } else if (kind == PH_UR) {
-            v[0] = rf_ur_tile<float, true, BatchM>(Q.L, tx, ty, coef, Q.f[BF_XS], Q.f[(it & 1) ? BF_P1 : BF_P0],
-                                                   Q.f[BF_R], Q.f[BF_W]);
+            v[0] = batch_ur_tile<K::STAGES>(ring, Q.L, tx, ty, coef, Q.f[BF_XS], Q.f[(it & 1) ? BF_P1 : BF_P0], Q.f[BF_R],
+                                 Q.f[BF_W]);
         } else if (kind == PH_FOLD) {
             rf_fold_tile<float, true>(Q.L, tx, ty, Q.gx, Q.hd, Q.u, Q.f[BF_XS]);
         } else {
             rf_resid_tile<float, true>(Q.L, tx, ty, Q.gx, Q.hd, Q.u, Q.u0, Q.kx, Q.ky, Q.f[BF_R], v);
         }
         double tot[2];
-        if (tile_done<2>(v, Q.tile0 + lt, Q, &tickets[b], partials, tot) && threadIdx.x == 0) {
+        if (tile_done<2>(v, Q.tile0 + lt, Q, &tickets[b], partials, &st[b], cp, tot) && threadIdx.x == 0) {
             // the phase is complete: its scalar update, then open the next phase
             int next = PH_W, nit = it;
             if (kind == PH_W) {
-                FinMxW{&st[b]}(tot);
+                FinMxW{&cp}(tot);
                 next = PH_UR;
             } else if (kind == PH_UR) {
-                FinMxUr{&st[b], nullptr}(tot);
-                if (st[b].upd) next = PH_FOLD;
+                FinMxUr{&cp, nullptr}(tot);
+                if (cp.upd) next = PH_FOLD;
                 else nit = it + 1;
             } else if (kind == PH_FOLD) {
                 next = PH_RESID;
             } else {
-                FinMxRes{&st[b], nullptr}(tot);
+                FinMxRes{&cp, nullptr}(tot);
                 nit = it + 1;
-                if (st[b].done) next = PH_DONE;
+                if (cp.done) next = PH_DONE;
             }
             if (next == PH_W && nit >= max_iters) next = PH_DONE;
             if (next == PH_DONE) atomicMax(&ctl->iters, nit);
-            pc[b].it = nit;
-            pc[b].kind = next;
-            __threadfence();
-            atomicExch(&pc[b].word, ((unsigned long long)(g + 1u) << 32) | (next == PH_DONE ? kClosed : 0u));
+            st[b] = cp;
+            sched_open(&pc[b], next == PH_W ? cp.beta : cp.alpha, phase_word(nit, next, Q.tx * Q.ty));
         }
     }
 }
@@ -304,14 +620,14 @@ __global__ void __launch_bounds__(BX, kBatchMinB) k_batch_cg(const BProb* __rest
 // Clears the per-problem tile tickets and schedules (a step that gave up may
 // have left them mid-phase) and the step's control words; the clock limit is
 // kept. A problem the setup already converged starts closed.
-__global__ void k_batch_reset(const MxState* st, int np, BCtl* ctl, unsigned* tickets, PCtl* pc)
+__global__ void k_batch_reset(const BProb* __restrict__ P, const MxState* st, int np, BCtl* ctl, unsigned* tickets,
+                              PCtl* pc)
 {
     for (int b = threadIdx.x; b < np; b += blockDim.x) {
         const bool done = st[b].done != 0;
         tickets[b] = 0u;
-        pc[b].word = done ? kClosed : 0ull;
-        pc[b].kind = done ? PH_DONE : PH_W;
-        pc[b].it = 0;
+        pc[b].coef = 0.0;
+        pc[b].word = phase_word(0, done ? PH_DONE : PH_W, P[b].tx * P[b].ty);
     }
     if (threadIdx.x == 0) {
         ctl->err = 0;
@@ -349,9 +665,12 @@ struct TlBatch {
     int max_tiles = 0;               // capacity of the tile tables
     int ntiles = 0;
     int tile_rows = 0;
-    int grid_blocks = 0;             // blocks the groups share (co-resident limit at most)
-    int launch_blocks = 0;           // blocks launched: the sum of the group sizes
-    int max_grid = 0;
+    int grid_blocks = 0;             // blocks the groups share
+    int launch_blocks = 0;           // blocks launched: the sum of the group sizes, the co-resident limit at most
+    int max_grid = 0;                // most blocks the groups may share
+    int resident = 0;                // co-resident blocks of the persistent kernel
+    const void* kernel = nullptr;    // its form
+    size_t smem = 0;                 // bytes of its row ring
     int max_iters = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -442,7 +761,6 @@ bool batch_layout(TlBatch* B, int tile_rows)
         Q.ty = (int)t.y;
         Q.tile0 = tiles;
         tiles += Q.tx * Q.ty;
-        Q.g0 = (int)bp.size();
         Q.gsize = std::min(size[b], Q.tx * Q.ty);
         for (int k = 0; k < Q.gsize; ++k) bp.push_back(b);
         Q.gx = B->suites[b]->g.x;
@@ -461,6 +779,14 @@ bool batch_layout(TlBatch* B, int tile_rows)
     }
     B->ntiles = tiles;
     B->tile_rows = tile_rows;
+    // more group blocks than fit the chip at once: an even selection of them is
+    // launched (a problem left without a block of its own is served by those of
+    // the others, which take work wherever most is left)
+    const size_t want = bp.size();
+    if (want > (size_t)B->resident) {
+        for (size_t k = 0; k < (size_t)B->resident; ++k) bp[k] = bp[k * want / B->resident];
+        bp.resize(B->resident);
+    }
     B->launch_blocks = (int)bp.size();
     if (!TL_CUDA(cudaMemcpyAsync(B->d_prob, P.data(), sizeof(BProb) * P.size(), cudaMemcpyHostToDevice, B->stream)))
         return false;
@@ -504,19 +830,20 @@ void issue_step(TlBatch* B, int iter_cap, bool finish)
             s->g.x, s->g.hd, B->lay[b], c->r, c->u0, c->kx, c->ky, f[BF_KX], f[BF_KY], f[BF_R], f[BF_P0], f[BF_P1],
             f[BF_W], f[BF_XS], B->rs, FinMxInit{&B->d_st[b], 0.0, st->eps, st->max_iters, nullptr});
     }
-    k_batch_reset<<<1, 128, 0, B->stream>>>(B->d_st, B->count, B->d_ctl, B->d_tickets, B->d_pctl);
+    k_batch_reset<<<1, 128, 0, B->stream>>>(B->d_prob, B->d_st, B->count, B->d_ctl, B->d_tickets, B->d_pctl);
     void* args[] = {&B->d_prob, &B->count, &B->d_block_prob, &B->d_st, &B->d_tickets, &B->d_partials, &B->d_pctl,
                     &B->d_ctl, &iter_cap};
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(B->launch_blocks);
     cfg.blockDim = dim3(BX);
+    cfg.dynamicSmemBytes = B->smem;
     cfg.stream = B->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelExC(&cfg, (const void*)k_batch_cg, args);
+    cudaLaunchKernelExC(&cfg, B->kernel, args);
     if (!finish) return;
     for (int b = 0; b < B->count; ++b) {
         TlSuite2D* s = B->suites[b];
@@ -624,9 +951,17 @@ TlBatch* tl2d_batch_create(Chunk** chunks, Settings** settings, int count, int t
     TL_CUDA(cudaMemsetAsync(B->d_ctl, 0, sizeof(BCtl), B->stream));
     static const long long default_limit = kWaitLimit;
     TL_CUDA(cudaMemcpyAsync(&B->d_ctl->limit, &default_limit, sizeof(long long), cudaMemcpyHostToDevice, B->stream));
+    // Resident when the FP32 arrays fit L2 (see Resident)
+    int l2 = 0;
+    TL_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, B->device));
+    const bool resident = total <= (size_t)l2;
+    B->kernel = resident ? (const void*)k_batch_cg<Resident> : (const void*)k_batch_cg<Streaming>;
+    B->smem = (resident ? Resident::STAGES : Streaming::STAGES) * sizeof(RingRow);
     int per_sm = 0;
-    TL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_cg, BX, 0));
-    B->max_grid = std::max(1, per_sm) * B->sm_count;
+    TL_CUDA(cudaFuncSetAttribute(B->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B->smem));
+    TL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, B->kernel, BX, B->smem));
+    B->resident = std::max(1, per_sm) * B->sm_count;
+    B->max_grid = kGroupsPerSm * B->sm_count;
     B->grid_blocks = grid_blocks > 0 ? std::min(grid_blocks, B->max_grid) : B->max_grid;
     if (!TL_CUDA(cudaMalloc(&B->d_block_prob, sizeof(int) * B->max_grid))) {
         batch_free(B);

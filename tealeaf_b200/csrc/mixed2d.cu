@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(BX, Pack<T>::MINB) k_rf_w(Lay L, const MxState
     T* const p_out = st->trip & 1 ? p1 : p0;
     const T* const p_in = FUSE_P ? (st->trip & 1 ? p0 : p1) : p_out;
     const double bt = FUSE_P ? st->beta : 0.0;
-    double acc[1] = {rf_w_tile<T, FUSE_P, false, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, bt, p_in, p_out,
+    double acc[1] = {rf_w_tile<T, FUSE_P, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, bt, p_in, p_out,
                                                                          r, w, kx, ky)};
     tl::grid_sum<1, BX>(acc, rs, block_id(), block_count(), fin);
 }
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(BX, Pack<T>::MINB) k_rf_ur(Lay L, const MxStat
 {
     if (mx_idle(st)) return;
     const T* const p = st->trip & 1 ? p1 : p0;
-    double acc[1] = {rf_ur_tile<T, false, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, st->alpha, xs, p, r, w)};
+    double acc[1] = {rf_ur_tile<T, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, st->alpha, xs, p, r, w)};
     tl::grid_sum<1, BX>(acc, rs, block_id(), block_count(), fin);
 }
 

@@ -247,14 +247,6 @@ __device__ __forceinline__ Cells<T> ld(const T* p)
 // between phases: CG = true reads through L2 (ld.global.cg), never from a
 // stale L1 line or the read-only path; false is a plain load.
 template <bool CG, typename T>
-__device__ __forceinline__ Cells<T> ldc(const T* p)
-{
-    if (!CG) return ld(p);
-    Cells<T> c;
-    c.v = __ldcg(reinterpret_cast<const typename Pack<T>::V*>(p));
-    return c;
-}
-template <bool CG, typename T>
 __device__ __forceinline__ T ldc1(const T* p)
 {
     return CG ? __ldcg(p) : *p;
@@ -348,7 +340,7 @@ __global__ void __launch_bounds__(256) k_rf_init(int gx, int hd, Lay L, const do
 // CG sweep 1 over tile (tx, ty), arithmetic in M: [p = beta p + r] (rounded
 // to T as stored), w = A p; returns this thread's share of sum(w p) over the
 // stored values. All threads of the block take part (warp shuffles).
-template <typename T, bool FUSE_P, bool CG = false, typename M = double>
+template <typename T, bool FUSE_P, typename M = double>
 __device__ __forceinline__ double rf_w_tile(const Lay& L, int tx, int ty, double bt_, const T* __restrict__ p_in,
                                             T* __restrict__ p_out, const T* __restrict__ r, T* __restrict__ w,
                                             const T* __restrict__ kx, const T* __restrict__ ky)
@@ -358,30 +350,30 @@ __device__ __forceinline__ double rf_w_tile(const Lay& L, int tx, int ty, double
     const Span<N> s(L, tx, ty);
     const M bt = (M)bt_;
     auto cur = [&](long idx) -> Cells<T> {
-        Cells<T> c = ldc<CG>(p_in + idx);
+        Cells<T> c = ld(p_in + idx);
         if (FUSE_P) {
-            const Cells<T> q = ldc<CG>(r + idx);
+            const Cells<T> q = ld(r + idx);
 #pragma unroll
             for (int m = 0; m < N; ++m) c.e[m] = (T)(bt * (M)c.e[m] + (M)q.e[m]);
         }
         return c;
     };
     auto cur1 = [&](long idx) -> T {
-        return FUSE_P ? (T)(bt * (M)ldc1<CG>(p_in + idx) + (M)ldc1<CG>(r + idx)) : ldc1<CG>(p_in + idx);
+        return FUSE_P ? (T)(bt * (M)p_in[idx] + (M)r[idx]) : p_in[idx];
     };
     const long xp = L.xp;
     long i = (long)(s.j0 + 1) * xp + s.cc;
-    Cells<T> pc = cur(i), pd = cur(i - xp), kyc = ldc<CG>(ky + i);
+    Cells<T> pc = cur(i), pd = cur(i - xp), kyc = ld(ky + i);
 TL2D_PRAGMA_UNROLL(TL2D_UNROLL)
     for (int j = s.j0; j < s.j1; ++j, i += xp) {
-        const Cells<T> pu = cur(i + xp), kyu = ldc<CG>(ky + i + xp), kxc = ldc<CG>(kx + i);
+        const Cells<T> pu = cur(i + xp), kyu = ld(ky + i + xp), kxc = ld(kx + i);
         T pl = __shfl_up_sync(kFull, pc.e[N - 1], 1);
         T pr = __shfl_down_sync(kFull, pc.e[0], 1);
         T kxr = __shfl_down_sync(kFull, kxc.e[0], 1);
         if (s.lane == 0) pl = cur1(i - 1);
         if (s.lane == 31) {
             pr = cur1(i + N);
-            kxr = ldc1<CG>(kx + i + N);
+            kxr = kx[i + N];
         }
         Cells<T> wv;
 #pragma unroll
@@ -408,7 +400,7 @@ TL2D_PRAGMA_UNROLL(TL2D_UNROLL)
 
 // CG sweep 2 over tile (tx, ty): xs += alpha p ; r -= alpha w ; returns this
 // thread's share of sum(r r).
-template <typename T, bool CG = false, typename M = double>
+template <typename T, typename M = double>
 __device__ __forceinline__ double rf_ur_tile(const Lay& L, int tx, int ty, double a_, T* __restrict__ xs,
                                              const T* __restrict__ p, T* __restrict__ r, const T* __restrict__ w)
 {
@@ -420,8 +412,8 @@ __device__ __forceinline__ double rf_ur_tile(const Lay& L, int tx, int ty, doubl
         long i = (long)(s.j0 + 1) * L.xp + s.c0;
 TL2D_PRAGMA_UNROLL(TL2D_UNROLL)
         for (int j = s.j0; j < s.j1; ++j, i += L.xp) {
-            Cells<T> xv = ldc<CG>(xs + i), rv = ldc<CG>(r + i);
-            const Cells<T> pv = ldc<CG>(p + i), wv = ldc<CG>(w + i);
+            Cells<T> xv = ld(xs + i), rv = ld(r + i);
+            const Cells<T> pv = ld(p + i), wv = ld(w + i);
 #pragma unroll
             for (int m = 0; m < N; ++m) {
                 xv.e[m] = (T)((M)xv.e[m] + a * (M)pv.e[m]);
