@@ -587,9 +587,9 @@ __global__ void __launch_bounds__(BX, K::MINB) k_batch_cg(const BProb* __restric
             v[0] = batch_ur_tile<K::STAGES>(ring, Q.L, tx, ty, coef, Q.f[BF_XS], Q.f[(it & 1) ? BF_P1 : BF_P0], Q.f[BF_R],
                                  Q.f[BF_W]);
         } else if (kind == PH_FOLD) {
-            rf_fold_tile<float, true>(Q.L, tx, ty, Q.gx, Q.hd, Q.u, Q.f[BF_XS]);
+            rf_fold_tile<float>(Q.L, tx, ty, Q.gx, Q.hd, Q.u, Q.f[BF_XS]);
         } else {
-            rf_resid_tile<float, true>(Q.L, tx, ty, Q.gx, Q.hd, Q.u, Q.u0, Q.kx, Q.ky, Q.f[BF_R], v);
+            rf_resid_tile<float>(Q.L, tx, ty, Q.gx, Q.hd, Q.u, Q.u0, Q.kx, Q.ky, Q.f[BF_R], v);
         }
         double tot[2];
         if (tile_done<2>(v, Q.tile0 + lt, Q, &tickets[b], partials, &st[b], cp, tot) && threadIdx.x == 0) {
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(BX, K::MINB) k_batch_cg(const BProb* __restric
                 FinMxW{&cp}(tot);
                 next = PH_UR;
             } else if (kind == PH_UR) {
-                FinMxUr{&cp, nullptr}(tot);
+                FinMxUr{&cp}(tot);
                 if (cp.upd) next = PH_FOLD;
                 else nit = it + 1;
             } else if (kind == PH_FOLD) {

@@ -36,10 +36,11 @@ __global__ void __launch_bounds__(BX, Pack<T>::MINB) k_rf_w(Lay L, const MxState
                                                             T* __restrict__ w, const T* __restrict__ kx,
                                                             const T* __restrict__ ky, ReduceSlots rs, FinMxW fin)
 {
-    if (mx_idle(st)) return;
-    T* const p_out = st->trip & 1 ? p1 : p0;
-    const T* const p_in = FUSE_P ? (st->trip & 1 ? p0 : p1) : p_out;
-    const double bt = FUSE_P ? st->beta : 0.0;
+    const MxState& h = mx_read(st);
+    if (mx_idle(h)) return;
+    T* const p_out = h.trip & 1 ? p1 : p0;
+    const T* const p_in = FUSE_P ? (h.trip & 1 ? p0 : p1) : p_out;
+    const double bt = FUSE_P ? h.beta : 0.0;
     double acc[1] = {rf_w_tile<T, FUSE_P, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, bt, p_in, p_out,
                                                                          r, w, kx, ky)};
     tl::grid_sum<1, BX>(acc, rs, block_id(), block_count(), fin);
@@ -51,9 +52,10 @@ __global__ void __launch_bounds__(BX, Pack<T>::MINB) k_rf_ur(Lay L, const MxStat
                                                              T* __restrict__ r, const T* __restrict__ w,
                                                              ReduceSlots rs, FinMxUr fin)
 {
-    if (mx_idle(st)) return;
-    const T* const p = st->trip & 1 ? p1 : p0;
-    double acc[1] = {rf_ur_tile<T, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, st->alpha, xs, p, r, w)};
+    const MxState& h = mx_read(st);
+    if (mx_idle(h)) return;
+    const T* const p = h.trip & 1 ? p1 : p0;
+    double acc[1] = {rf_ur_tile<T, typename RfMath<T>::M>(L, blockIdx.x, blockIdx.y, h.alpha, xs, p, r, w)};
     tl::grid_sum<1, BX>(acc, rs, block_id(), block_count(), fin);
 }
 
@@ -69,7 +71,8 @@ __global__ void __launch_bounds__(BX, Pack<T>::MINB - 2) k_rf_pc(Lay L, const Mx
                                                                T* __restrict__ z, const T* __restrict__ kx,
                                                                const T* __restrict__ ky)
 {
-    if (mx_idle(st)) return;
+    const MxState& h = mx_read(st);
+    if (mx_idle(h)) return;
     const double fa = FOLD == 2 ? alphas[pp - 1] : 0.0, fb = FOLD == 2 ? betas[pp - 1] : 0.0;
     rf_pc_tile<T, FOLD, FOLD == 2>(L, blockIdx.x, blockIdx.y, theta, fa, fb, sd_in, sd_out, s_in, s_out, z, kx, ky);
 }
@@ -84,7 +87,8 @@ __global__ void __launch_bounds__(BX, Pack<T>::MINB - 2) k_rf_pc_last(Lay L, con
                                                                   const T* __restrict__ r, ReduceSlots rs,
                                                                   FinPcgZ fin)
 {
-    if (mx_idle(st)) return;
+    const MxState& h = mx_read(st);
+    if (mx_idle(h)) return;
     const double fa = FOLD == 2 ? alphas[pp - 1] : 0.0, fb = FOLD == 2 ? betas[pp - 1] : 0.0;
     double acc[1] = {rf_pc_last_tile<T, FOLD>(L, blockIdx.x, blockIdx.y, theta, fa, fb, sd, s_in, z, r)};
     tl::grid_sum<1, BX>(acc, rs, block_id(), block_count(), fin);
@@ -103,7 +107,9 @@ template <typename T>
 __global__ void __launch_bounds__(BX) k_rf_fold(Lay L, const MxState* __restrict__ st, int gx, int hd,
                                                 double* __restrict__ u, T* __restrict__ xs)
 {
-    if (mx_no_update(st)) return;
+    tl::chain_start();
+    tl::chain_wait();
+    if (mx_no_update(mx_read(st))) return;
     rf_fold_tile<T>(L, blockIdx.x, blockIdx.y, gx, hd, u, xs);
 }
 
@@ -113,7 +119,9 @@ __global__ void __launch_bounds__(BX) k_rf_resid(Lay L, const MxState* __restric
                                                  const double* __restrict__ kx, const double* __restrict__ ky,
                                                  T* __restrict__ rT, ReduceSlots rs, FinMxRes fin)
 {
-    if (mx_no_update(st)) return;
+    tl::chain_start();
+    tl::chain_wait();
+    if (mx_no_update(mx_read(st))) return;
     double acc[2] = {0.0, 0.0};
     rf_resid_tile<T>(L, blockIdx.x, blockIdx.y, gx, hd, u, u0, kx, ky, rT, acc);
     tl::grid_sum<2, BX>(acc, rs, block_id(), block_count(), fin);
@@ -172,6 +180,16 @@ const CUtensorMap* rf_map(TlSuite2D* s, const Lay& L, const T* ptr, bool ring)
     });
 }
 
+// The sums of a trip stay on the device: a kernel that writes to mapped host
+// memory ends when the write has crossed the bus (83.1 against 75.8 ms for 3376
+// trips of two sweeps at 1536^2).
+ReduceSlots device_slots(const TlSuite2D* s)
+{
+    ReduceSlots rs = s->rs;
+    rs.out_host = nullptr;
+    return rs;
+}
+
 // The refinement w sweep (k_rf_w semantics), by TMA where the maps encode; r:
 // the field folded into p. Internal linkage with the kernels, as the drop-in
 // helpers.
@@ -193,14 +211,15 @@ void rf_w(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, const 
                                              (int)smem));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, name, (k_rf_w_tma<T, FUSE_P><<<gl, BX, smem, s->stream>>>(
-                                   b.L, b.st, m, b.f[RF_P0], b.f[RF_P1], b.f[RF_W], s->rs, fin,
+            TL_LAUNCH(s, name, (tl::launch_chained(k_rf_w_tma<T, FUSE_P>, gl, dim3(BX), smem, s->stream,
+                                   b.L, b.st, m, b.f[RF_P0], b.f[RF_P1], b.f[RF_W], device_slots(s), fin,
                                    s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
     TL_LAUNCH(s, name, (k_rf_w<T, FUSE_P><<<gl, BX, 0, s->stream>>>(b.L, b.st, b.f[RF_P0], b.f[RF_P1], r, b.f[RF_W],
-                                                                     b.f[RF_KX], b.f[RF_KY], s->rs, fin)));
+                                                                     b.f[RF_KX], b.f[RF_KY], device_slots(s),
+                                                                     fin)));
 }
 
 // The refinement u/r update (k_rf_ur semantics), by TMA where the maps encode.
@@ -221,13 +240,14 @@ void rf_ur(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, FinMx
                                              (int)smem));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, name, (k_rf_ur_tma<T><<<gl, BX, smem, s->stream>>>(b.L, b.st, m, b.f[RF_XS], b.f[RF_R],
-                                                                           s->rs, fin, s->d_mirror + kTmaErrWord2)));
+            TL_LAUNCH(s, name, (tl::launch_chained(k_rf_ur_tma<T>, gl, dim3(BX), smem, s->stream, b.L, b.st, m,
+                                                   b.f[RF_XS], b.f[RF_R], device_slots(s), fin,
+                                                   s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
     TL_LAUNCH(s, name, (k_rf_ur<T><<<gl, BX, 0, s->stream>>>(b.L, b.st, b.f[RF_XS], b.f[RF_P0], b.f[RF_P1], b.f[RF_R],
-                                                              b.f[RF_W], s->rs, fin)));
+                                                              b.f[RF_W], device_slots(s), fin)));
 }
 
 // Launches groups of up to kGroup trips, each followed by `update`, looking at
@@ -288,12 +308,12 @@ int solve_refined(TlSuite2D* s, Chunk* chunk, int max_iters, double rel_tol, int
     batched(s, max_iters, [&](int t) {
         if (t == 0) rf_w<T, false>(s, b, gl, nm[1], b.f[RF_R], FinMxW{b.st});
         else rf_w<T, true>(s, b, gl, nm[1], b.f[RF_R], FinMxW{b.st});
-        rf_ur<T>(s, b, gl, nm[2], FinMxUr{b.st, s->d_mirror});
+        rf_ur<T>(s, b, gl, nm[2], FinMxUr{b.st});
     }, [&] {
-        TL_LAUNCH(s, nm[3], (k_rf_fold<T><<<gl, BX, 0, s->stream>>>(L, b.st, s->g.x, s->g.hd, chunk->u,
-                                                                     b.f[RF_XS])));
-        TL_LAUNCH(s, nm[4], (k_rf_resid<T><<<gl, BX, 0, s->stream>>>(L, b.st, s->g.x, s->g.hd, chunk->u,
-                                                                      chunk->u0, chunk->kx, chunk->ky, b.f[RF_R],
+        TL_LAUNCH(s, nm[3], (tl::launch_chained(k_rf_fold<T>, gl, dim3(BX), 0, s->stream, L, b.st, s->g.x,
+                                                s->g.hd, chunk->u, b.f[RF_XS])));
+        TL_LAUNCH(s, nm[4], (tl::launch_chained(k_rf_resid<T>, gl, dim3(BX), 0, s->stream, L, b.st, s->g.x,
+                                                s->g.hd, chunk->u, chunk->u0, chunk->kx, chunk->ky, b.f[RF_R],
                                                                       s->rs, FinMxRes{b.st, s->d_mirror})));
     });
     MxState st{};
@@ -356,16 +376,16 @@ int solve_refined_ppcg(TlSuite2D* s, Chunk* chunk, Settings* settings, double re
     T* const r = b.f[RF_R];
     T* const z = b.f[RF_Z];
     auto fold_resid = [&](double* betas) {
-        TL_LAUNCH(s, nm[3], (k_rf_fold<T><<<gl, BX, 0, s->stream>>>(L, b.st, s->g.x, s->g.hd, chunk->u,
-                                                                     b.f[RF_XS])));
-        TL_LAUNCH(s, nm[4], (k_rf_resid<T><<<gl, BX, 0, s->stream>>>(L, b.st, s->g.x, s->g.hd, chunk->u,
-                                                                      chunk->u0, chunk->kx, chunk->ky, r, s->rs,
+        TL_LAUNCH(s, nm[3], (tl::launch_chained(k_rf_fold<T>, gl, dim3(BX), 0, s->stream, L, b.st, s->g.x,
+                                                s->g.hd, chunk->u, b.f[RF_XS])));
+        TL_LAUNCH(s, nm[4], (tl::launch_chained(k_rf_resid<T>, gl, dim3(BX), 0, s->stream, L, b.st, s->g.x,
+                                                s->g.hd, chunk->u, chunk->u0, chunk->kx, chunk->ky, r, s->rs,
                                                                       FinMxRes{b.st, s->d_mirror, betas})));
     };
     // CG trips up to the switch (2d/shared.h:41-42 for the constants)
     const FinMxUr cg_fin = settings->error_switch
-                               ? FinMxUr{b.st, s->d_mirror, s->d_cg_betas, 20, settings->eps_lim}
-                               : FinMxUr{b.st, s->d_mirror, s->d_cg_betas, settings->presteps, 1.0};
+                               ? FinMxUr{b.st, s->d_cg_betas, 20, settings->eps_lim}
+                               : FinMxUr{b.st, s->d_cg_betas, settings->presteps, 1.0};
     batched(s, max_iters, [&](int t) {
         if (t == 0) rf_w<T, false>(s, b, gl, nm[1], r, FinMxW{b.st, s->d_cg_alphas});
         else rf_w<T, true>(s, b, gl, nm[1], r, FinMxW{b.st, s->d_cg_alphas});
@@ -431,7 +451,7 @@ int solve_refined_ppcg(TlSuite2D* s, Chunk* chunk, Settings* settings, double re
             }
             // p = z + beta p, w = A p, alpha = r.z / p.w
             rf_w<T, true>(s, b, gl, nm[1], z, FinMxW{b.st, nullptr, true});
-            rf_ur<T>(s, b, gl, nm[2], FinMxUr{b.st, s->d_mirror});
+            rf_ur<T>(s, b, gl, nm[2], FinMxUr{b.st});
         }, [&] { fold_resid(nullptr); });
         TL_CUDA(cudaMemcpy(&st, b.st, sizeof(MxState), cudaMemcpyDeviceToHost));
     }

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kPcThreads, sizeof(T) == 4 ? 2 : 1)
     extern __shared__ __align__(16) unsigned char pc_raw[];
     T* const A0 = reinterpret_cast<T*>(pc_raw);
     T* const A1 = A0 + kPcH * kPcW;
-    if (mx_idle(st)) return;
+    if (mx_idle(mx_read(st))) return;
     const int tid = threadIdx.x, cx = tid % kPcW, cy = tid / kPcW, lane = tid & 31;
     const int X0 = blockIdx.x * kPcX, Y0 = blockIdx.y * kPcY;
     const int gx = X0 - kPcMax + cx;   // interior column of this thread

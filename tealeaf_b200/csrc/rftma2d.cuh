@@ -87,24 +87,31 @@ constexpr size_t rf_u_tma_bytes()
 // rows j0-1+4b ..): the rows of interior rows j0+4b .. j0+4b+3 and their
 // upper neighbours are in stages b and b+1.
 template <typename T, bool FUSE_P>
-__global__ void __launch_bounds__(BX, 4) k_rf_w_tma(Lay L, const MxState* __restrict__ st,
+__global__ void __launch_bounds__(BX, 4) k_rf_w_tma(Lay L, const MxState* st,
                                                     const __grid_constant__ RfWMaps m, T* p0, T* p1,
                                                     T* __restrict__ w, ReduceSlots rs, FinMxW fin, int* err)
 {
     extern __shared__ __align__(128) unsigned char rw_raw[];
     using S = RfRowsW<T>;
     constexpr int N = Pack<T>::N, W = S::W, H = S::H;
-    if (mx_idle(st)) return;
-    const int par = st->trip & 1, in = FUSE_P ? par ^ 1 : par;
-    T* const p_out = par ? p1 : p0;
+    tl::chain_start();
     unsigned char* base = rw_raw + ((128 - (tl::smem_addr(rw_raw) & 127)) & 127);
     S* ring = reinterpret_cast<S*>(base);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kRfStages * sizeof(S));
-    const double bt = FUSE_P ? st->beta : 0.0;
     const Span<N> s(L, blockIdx.x, blockIdx.y);
     const int tid = threadIdx.x;
     const int cb = blockIdx.x * W;
     const int np = (s.j1 - s.j0 + 2 + kRfRows - 1) / kRfRows;
+    if (tid == 0) {
+        for (int q = 0; q < kRfStages; ++q) tl::mbar_init(&bars[q], 1);
+        tl::mbar_fence_init();
+    }
+    tl::chain_wait();
+    const MxState& h = mx_read(st);
+    if (mx_idle(h)) return;
+    const double bt = FUSE_P ? h.beta : 0.0;
+    const int par = h.trip & 1, in = FUSE_P ? par ^ 1 : par;
+    T* const p_out = par ? p1 : p0;
     constexpr unsigned kMain = sizeof(T) * kRfRows * W, kRing = sizeof(T) * kRfRows * H;
     auto issue = [&](int b) {
         S& Q = ring[b % kRfStages];
@@ -123,11 +130,6 @@ __global__ void __launch_bounds__(BX, 4) k_rf_w_tma(Lay L, const MxState* __rest
         tl::tma_load_3d(&Q.KXR[0][0], &m.kxh, cb + W, y0, 0, bar);
         tl::tma_load_3d(&Q.KY[0][0], &m.ky, cb, y0, 0, bar);
     };
-    if (tid == 0) {
-        for (int q = 0; q < kRfStages; ++q) tl::mbar_init(&bars[q], 1);
-        tl::mbar_fence_init();
-    }
-    __syncthreads();
     if (tid == 0)
         for (int b = 0; b < kRfStages - 1 && b < np; ++b) issue(b);
     // t: T-layout row - j0
@@ -215,15 +217,14 @@ __global__ void __launch_bounds__(BX, 4) k_rf_w_tma(Lay L, const MxState* __rest
 // k_rf_ur by TMA: stage b holds T-layout rows j0+1+4b .. (interior rows
 // j0+4b ..).
 template <typename T>
-__global__ void __launch_bounds__(BX, 4) k_rf_ur_tma(Lay L, const MxState* __restrict__ st,
+__global__ void __launch_bounds__(BX, 4) k_rf_ur_tma(Lay L, const MxState* st,
                                                      const __grid_constant__ RfUMaps m, T* __restrict__ xs,
                                                      T* __restrict__ r, ReduceSlots rs, FinMxUr fin, int* err)
 {
     extern __shared__ __align__(128) unsigned char ru_raw[];
     using S = RfRowsU<T>;
     constexpr int N = Pack<T>::N, W = S::W;
-    if (mx_idle(st)) return;
-    const int par = st->trip & 1;
+    tl::chain_start();
     unsigned char* base = ru_raw + ((128 - (tl::smem_addr(ru_raw) & 127)) & 127);
     S* ring = reinterpret_cast<S*>(base);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kRfStagesU * sizeof(S));
@@ -231,6 +232,14 @@ __global__ void __launch_bounds__(BX, 4) k_rf_ur_tma(Lay L, const MxState* __res
     const int tid = threadIdx.x;
     const int cb = blockIdx.x * W;
     const int np = (s.j1 - s.j0 + kRfRows - 1) / kRfRows;
+    if (tid == 0) {
+        for (int q = 0; q < kRfStagesU; ++q) tl::mbar_init(&bars[q], 1);
+        tl::mbar_fence_init();
+    }
+    tl::chain_wait();
+    const MxState& h = mx_read(st);
+    if (mx_idle(h)) return;
+    const int par = h.trip & 1;
     auto issue = [&](int b) {
         S& Q = ring[b % kRfStagesU];
         unsigned long long* bar = &bars[b % kRfStagesU];
@@ -241,15 +250,10 @@ __global__ void __launch_bounds__(BX, 4) k_rf_ur_tma(Lay L, const MxState* __res
         tl::tma_load_3d(&Q.R[0][0], &m.r, cb, y0, 0, bar);
         tl::tma_load_3d(&Q.Wv[0][0], &m.w, cb, y0, 0, bar);
     };
-    if (tid == 0) {
-        for (int q = 0; q < kRfStagesU; ++q) tl::mbar_init(&bars[q], 1);
-        tl::mbar_fence_init();
-    }
-    __syncthreads();
     if (tid == 0)
         for (int b = 0; b < kRfStagesU - 1 && b < np; ++b) issue(b);
     using M = typename RfMath<T>::M;
-    const M a = (M)st->alpha;
+    const M a = (M)h.alpha;
     double acc = 0.0;
     long i = (long)(s.j0 + 1) * L.xp + s.c0;
     for (int b = 0; b < np; ++b) {
