@@ -292,7 +292,8 @@ static __global__ void __launch_bounds__(kTBThreads, 1) k_blocked_tma(Geo g, Blo
     double* const S1 = S0 + kBlockedFieldDoubles;
     double* const stg = S1 + kBlockedFieldDoubles;
     unsigned long long* const bar = reinterpret_cast<unsigned long long*>(stg + 5 * kBlockedFieldDoubles);
-    if (gate_closed(done)) return;
+    __shared__ SweepHead head;
+    tl::chain_start();
     const int ntx = (g.x - 2 * g.hd + Blk<MODE>::TX - 1) / Blk<MODE>::TX;
     const int ntiles = ntx * ((g.y - 2 * g.hd + Blk<MODE>::TY - 1) / Blk<MODE>::TY);
     const int tid = threadIdx.x;
@@ -309,7 +310,10 @@ static __global__ void __launch_bounds__(kTBThreads, 1) k_blocked_tma(Geo g, Blo
         tl::mbar_init(bar, 1);
         tl::mbar_fence_init();
     }
+    tl::chain_wait();
+    if (tid == 0) head.gate(done);
     __syncthreads();
+    if (head.closed) return;
     if (tid == 0 && (int)blockIdx.x < ntiles) issue(blockIdx.x);
     unsigned phase = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, phase ^= 1u) {
@@ -328,12 +332,20 @@ template <typename Finish>
 static __global__ void __launch_bounds__(BX) k_norm2_fin(Geo g, const double* __restrict__ b, ReduceSlots rs,
                                                        const int* __restrict__ done, Finish fin)
 {
-    if (gate_closed(done)) return;
+    __shared__ SweepHead head;
+    tl::chain_start();
+    tl::chain_wait();
+    if (threadIdx.x == 0) head.gate(done);
+    __syncthreads();
+    if (head.closed) return;
     Strip s(g);
     double acc[1] = {0.0};
     if (s.active) {
         long i = s.k + (long)s.j0 * g.x;
-        for (int j = s.j0; j < s.j1; ++j, i += g.x) acc[0] += b[i] * b[i];
+        for (int j = s.j0; j < s.j1; ++j, i += g.x) {
+            const double v = __ldcg(b + i);
+            acc[0] += v * v;
+        }
     }
     tl::grid_sum<1, BX>(acc, rs, block_id(), block_count(), fin);
 }
@@ -342,6 +354,8 @@ static __global__ void __launch_bounds__(BX) k_norm2_fin(Geo g, const double* __
 template <typename Finish>
 static __global__ void k_finish_only(const int* __restrict__ done, Finish fin)
 {
+    tl::chain_start();
+    tl::chain_wait();
     if (gate_closed(done) || threadIdx.x != 0) return;
     const double t[1] = {0.0};
     fin(t);

@@ -304,12 +304,13 @@ struct Run {
             if (mu && mp && mr && mw && mm && my) {
                 const PcgMaps m{*mu, *mp, *mr, *mw, *mm, *my};
                 TL_LAUNCH(s, "k_pcg_ur", (k_pcg_ur_tma<BS><<<gbi, BX, kPcgTmaBytes, s->stream>>>(
-                                             gb, alpha, m, chunk->u, chunk->r, z, s->rs, done(), fin_ur,
+                                             gb, alpha, m, chunk->u, chunk->r, z, loop_slots(s, done()), done(), fin_ur,
                                              s->d_mirror + kTmaErrWord2)));
             } else {
                 TL_LAUNCH(s, "k_pcg_ur", (k_pcg_ur<BS><<<gbi, BX, 0, s->stream>>>(gb, alpha, chunk->u, p, chunk->r,
                                                                                   chunk->w, chunk->ky, chunk->mi, z,
-                                                                                  s->rs, done(), fin_ur)));
+                                                                                  loop_slots(s, done()), done(),
+                                                                                  fin_ur)));
             }
         });
     }
@@ -393,10 +394,11 @@ struct Run {
                                       chunk->u0, nullptr, chunk->w, chunk->r, chunk->kx, chunk->ky, done());
                     const FinChebyBlock fin{s->d_state, pc, s->d_mirror, L, norm};
                     if (norm)
-                        TL_LAUNCH(s, "k_norm2_fin", (k_norm2_fin<<<gi, BX, 0, s->stream>>>(s->g, chunk->r, s->rs,
-                                                                                            done(), fin)));
+                        TL_LAUNCH(s, "k_norm2_fin", (chain(s, k_norm2_fin<FinChebyBlock>, gi, BX, 0, s->g, chunk->r,
+                                                           loop_slots(s, done()), done(), fin)));
                     else
-                        TL_LAUNCH(s, "k_finish_only", (k_finish_only<<<1, 32, 0, s->stream>>>(done(), fin)));
+                        TL_LAUNCH(s, "k_finish_only", (chain(s, k_finish_only<FinChebyBlock>, 1, 32, 0, done(),
+                                                             fin)));
                     cur ^= 1;
                     return L;
                 }, starts);
@@ -469,8 +471,8 @@ struct Run {
                     sc ^= 1;
                     rc ^= 1;
                     if (last)
-                        TL_LAUNCH(s, "k_norm2_fin", (k_norm2_fin<<<gi, BX, 0, s->stream>>>(s->g, rb[rc], s->rs,
-                                                                                            done(), fin_n)));
+                        TL_LAUNCH(s, "k_norm2_fin", (chain(s, k_norm2_fin<FinPpcgNorm>, gi, BX, 0, s->g, rb[rc],
+                                                           loop_slots(s, done()), done(), fin_n)));
                 }
                 return;
             }
@@ -479,7 +481,7 @@ struct Run {
                 if (pp == 0 && last)
                     TL_LAUNCH(s, "k_ppcg_step", (k_ppcg_step<1, true><<<gh, BX, 0, s->stream>>>(
                                   s->g, fc, chunk->theta, coef, 0, sb[sc], sb[sc ^ 1], rb[rc], rb[rc ^ 1], chunk->u,
-                                  chunk->kx, chunk->ky, s->rs, done(), fin_n)));
+                                  chunk->kx, chunk->ky, loop_slots(s, done()), done(), fin_n)));
                 else if (pp == 0)
                     TL_LAUNCH(s, "k_ppcg_step", (k_ppcg_step<1, false><<<gh, BX, 0, s->stream>>>(
                                   s->g, fc, chunk->theta, coef, 0, sb[sc], sb[sc ^ 1], rb[rc], rb[rc ^ 1], chunk->u,
@@ -487,7 +489,7 @@ struct Run {
                 else if (last)
                     TL_LAUNCH(s, "k_ppcg_step", (k_ppcg_step<2, true><<<gh, BX, 0, s->stream>>>(
                                   s->g, fc, chunk->theta, coef, pp - 1, sb[sc], sb[sc ^ 1], rb[rc], rb[rc ^ 1],
-                                  chunk->u, chunk->kx, chunk->ky, s->rs, done(), fin_n)));
+                                  chunk->u, chunk->kx, chunk->ky, loop_slots(s, done()), done(), fin_n)));
                 else
                     TL_LAUNCH(s, "k_ppcg_step", (k_ppcg_step<2, false><<<gh, BX, 0, s->stream>>>(
                                   s->g, fc, chunk->theta, coef, pp - 1, sb[sc], sb[sc ^ 1], rb[rc], rb[rc ^ 1],

@@ -236,8 +236,8 @@ struct Run3 {
                                       chunk->vec_w, chunk->vec_r);
                     const tl::FinChebyBlock fin{s->d_state, pc, s->d_mirror, L, nrm};
                     if (nrm)
-                        TL3_LAUNCH(s, "k3_norm2_fin", (k3_norm2_fin<<<gh, bl, 0, s->stream>>>(s->g, chunk->vec_r,
-                                                                                             s->rs, done(), fin)));
+                        TL3_LAUNCH(s, "k3_norm2_fin", (k3_norm2_fin<<<gh, bl, 0, s->stream>>>(
+                                                         s->g, chunk->vec_r, loop_slots(s, done()), done(), fin)));
                     else
                         TL3_LAUNCH(s, "k3_finish_only", (k3_finish_only<<<1, 32, 0, s->stream>>>(done(), fin)));
                     cur ^= 1;
@@ -309,8 +309,8 @@ struct Run3 {
                     sc ^= 1;
                     rc ^= 1;
                     if (pp0 + L == ni)
-                        TL3_LAUNCH(s, "k3_norm2_fin", (k3_norm2_fin<<<gh, bl, 0, s->stream>>>(s->g, rb[rc], s->rs,
-                                                                                             done(), fin_n)));
+                        TL3_LAUNCH(s, "k3_norm2_fin", (k3_norm2_fin<<<gh, bl, 0, s->stream>>>(
+                                                         s->g, rb[rc], loop_slots(s, done()), done(), fin_n)));
                 }
                 return;
             }

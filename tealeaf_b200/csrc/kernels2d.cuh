@@ -31,6 +31,7 @@ using tl::FinCgUr;
 using tl::FinCgW;
 using tl::FinPcgUr;
 using tl::FinChebyBlock;
+using tl::SweepHead;
 using tl::FinChebyTrip;
 using tl::FinPpcgNorm;
 using tl::FinPpcgW;
@@ -775,16 +776,29 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc
                                                                       int* err)
 {
     extern __shared__ __align__(128) unsigned char t2_raw[];
-    if (gate_closed(done)) return;
-    double acc[1] = {0.0};
     using Rows = RowsT<UPD>;
-    const double bt = FUSE_P ? beta.get() : 0.0;
-    const double a0 = UPD ? cu.alphas[cu.t - 2] : 0.0, a1 = UPD ? cu.alphas[cu.t - 1] : 0.0;
-    auto cur = [&](long idx) { return FUSE_P ? bt * p_in[idx] + r[idx] : p_in[idx]; };
+    __shared__ SweepHead head;
+    tl::chain_start();
+    unsigned char* base = t2_raw + ((128 - (tl::smem_addr(t2_raw) & 127)) & 127);
+    Rows* ring = reinterpret_cast<Rows*>(base);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kStagesT * sizeof(Rows));
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < kStagesT; ++q) tl::mbar_init(&bars[q], 1);
+        tl::mbar_fence_init();
+    }
+    tl::chain_wait();
+    if (threadIdx.x == 0) {
+        head.gate(done);
+        head.s[0] = FUSE_P ? beta.fresh() : 0.0;
+        head.s[1] = UPD ? __ldcg(cu.alphas + (cu.t - 2)) : 0.0;
+        head.s[2] = UPD ? __ldcg(cu.alphas + (cu.t - 1)) : 0.0;
+    }
+    __syncthreads();
+    if (head.closed) return;
+    double acc[1] = {0.0};
+    const double bt = head.s[0], a0 = head.s[1], a1 = head.s[2];
+    auto cur = [&](long idx) { return FUSE_P ? bt * __ldcg(p_in + idx) + __ldcg(r + idx) : __ldcg(p_in + idx); };
     if (blockIdx.y + 1 < gridDim.y) {
-        unsigned char* base = t2_raw + ((128 - (tl::smem_addr(t2_raw) & 127)) & 127);
-        Rows* ring = reinterpret_cast<Rows*>(base);
-        unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kStagesT * sizeof(Rows));
         const StripC s(g);
         const int x = g.x, tx = threadIdx.x;
         const int k0 = g.hd + blockIdx.x * BX;
@@ -807,11 +821,6 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc
                 tl::tma_load_3d(&S.P2[0][0], &maps.p2, k0, y0, 0, bar);
             }
         };
-        if (tx == 0) {
-            for (int q = 0; q < kStagesT; ++q) tl::mbar_init(&bars[q], 1);
-            tl::mbar_fence_init();
-        }
-        __syncthreads();
         if (tx == 0)
             for (int b = 0; b < kStagesT - 1 && b < np; ++b) issue(b);
         // row j of the strip: stage (j - jb) / 4, row (j - jb) % 4
@@ -872,7 +881,7 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_w_fused_tma(Geo g, Faces fc
         // every issued stage was waited for (the last rows read stage np-1): no copy in flight
     } else {
         if (REFLECT) halo_duty(g, fc, 1, p_out, cur);
-        if (u_halo) halo_duty(g, fc, uhd, u_halo, [&](long idx) { return u_halo[idx]; });
+        if (u_halo) halo_duty(g, fc, uhd, u_halo, [&](long idx) { return __ldcg(u_halo + idx); });
     }
     tl::grid_sum<1, BX>(acc, rs, block_id(), block_count(), fin);
 }
@@ -939,7 +948,8 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_ur_fused_tma(Geo g, Scalar 
                                                                Finish fin, int* err)
 {
     extern __shared__ __align__(128) unsigned char tu_raw[];
-    if (gate_closed(done)) return;
+    __shared__ SweepHead head;
+    tl::chain_start();
     unsigned char* base = tu_raw + ((128 - (tl::smem_addr(tu_raw) & 127)) & 127);
     RowsU* ring = reinterpret_cast<RowsU*>(base);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kStagesU * sizeof(RowsU));
@@ -966,10 +976,16 @@ static __global__ void __launch_bounds__(BX, 4) k_cg_ur_fused_tma(Geo g, Scalar 
         for (int q = 0; q < kStagesU; ++q) tl::mbar_init(&bars[q], 1);
         tl::mbar_fence_init();
     }
+    tl::chain_wait();
+    if (tx == 0) {
+        head.gate(done);
+        head.s[0] = alpha.fresh();
+    }
     __syncthreads();
+    if (head.closed) return;
     if (tx == 0)
         for (int b = 0; b < kStagesU - 1 && b < np; ++b) issue(b);
-    const double a = alpha.get();
+    const double a = head.s[0];
     for (int b = 0; b < np; ++b) {
         __syncthreads();   // every thread is past stage b-1: its slot is free
         if (tx == 0 && b + kStagesU - 1 < np) issue(b + kStagesU - 1);
@@ -1048,7 +1064,8 @@ static __global__ void __launch_bounds__(BX, TL2D_MINB_R) k_cg_r_fused_tma(Geo g
                                                                  const int* __restrict__ done, Finish fin, int* err)
 {
     extern __shared__ __align__(128) unsigned char tr_raw[];
-    if (gate_closed(done)) return;
+    __shared__ SweepHead head;
+    tl::chain_start();
     unsigned char* base = tr_raw + ((128 - (tl::smem_addr(tr_raw) & 127)) & 127);
     RowsR* ring = reinterpret_cast<RowsR*>(base);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(base + kStagesR * sizeof(RowsR));
@@ -1071,10 +1088,16 @@ static __global__ void __launch_bounds__(BX, TL2D_MINB_R) k_cg_r_fused_tma(Geo g
         for (int q = 0; q < kStagesR; ++q) tl::mbar_init(&bars[q], 1);
         tl::mbar_fence_init();
     }
+    tl::chain_wait();
+    if (tx == 0) {
+        head.gate(done);
+        head.s[0] = alpha.fresh();
+    }
     __syncthreads();
+    if (head.closed) return;
     if (tx == 0)
         for (int b = 0; b < kStagesR - 1 && b < np; ++b) issue(b);
-    const double a = alpha.get();
+    const double a = head.s[0];
     for (int b = 0; b < np; ++b) {
         __syncthreads();   // every thread is past stage b-1: its slot is free
         if (tx == 0 && b + kStagesR - 1 < np) issue(b + kStagesR - 1);

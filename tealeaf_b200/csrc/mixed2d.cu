@@ -180,16 +180,6 @@ const CUtensorMap* rf_map(TlSuite2D* s, const Lay& L, const T* ptr, bool ring)
     });
 }
 
-// The sums of a trip stay on the device: a kernel that writes to mapped host
-// memory ends when the write has crossed the bus (83.1 against 75.8 ms for 3376
-// trips of two sweeps at 1536^2).
-ReduceSlots device_slots(const TlSuite2D* s)
-{
-    ReduceSlots rs = s->rs;
-    rs.out_host = nullptr;
-    return rs;
-}
-
 // The refinement w sweep (k_rf_w semantics), by TMA where the maps encode; r:
 // the field folded into p. Internal linkage with the kernels, as the drop-in
 // helpers.
@@ -211,14 +201,13 @@ void rf_w(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, const 
                                              (int)smem));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, name, (tl::launch_chained(k_rf_w_tma<T, FUSE_P>, gl, dim3(BX), smem, s->stream,
-                                   b.L, b.st, m, b.f[RF_P0], b.f[RF_P1], b.f[RF_W], device_slots(s), fin,
-                                   s->d_mirror + kTmaErrWord2)));
+            TL_LAUNCH(s, name, (chain(s, k_rf_w_tma<T, FUSE_P>, gl, BX, smem, b.L, b.st, m, b.f[RF_P0], b.f[RF_P1],
+                                      b.f[RF_W], loop_slots(s, &b.st->done), fin, s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
     TL_LAUNCH(s, name, (k_rf_w<T, FUSE_P><<<gl, BX, 0, s->stream>>>(b.L, b.st, b.f[RF_P0], b.f[RF_P1], r, b.f[RF_W],
-                                                                     b.f[RF_KX], b.f[RF_KY], device_slots(s),
+                                                                     b.f[RF_KX], b.f[RF_KY], loop_slots(s, &b.st->done),
                                                                      fin)));
 }
 
@@ -240,14 +229,13 @@ void rf_ur(TlSuite2D* s, const RfBuffers<T>& b, dim3 gl, const char* name, FinMx
                                              (int)smem));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, name, (tl::launch_chained(k_rf_ur_tma<T>, gl, dim3(BX), smem, s->stream, b.L, b.st, m,
-                                                   b.f[RF_XS], b.f[RF_R], device_slots(s), fin,
-                                                   s->d_mirror + kTmaErrWord2)));
+            TL_LAUNCH(s, name, (chain(s, k_rf_ur_tma<T>, gl, BX, smem, b.L, b.st, m, b.f[RF_XS], b.f[RF_R],
+                                      loop_slots(s, &b.st->done), fin, s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
     TL_LAUNCH(s, name, (k_rf_ur<T><<<gl, BX, 0, s->stream>>>(b.L, b.st, b.f[RF_XS], b.f[RF_P0], b.f[RF_P1], b.f[RF_R],
-                                                              b.f[RF_W], device_slots(s), fin)));
+                                                              b.f[RF_W], loop_slots(s, &b.st->done), fin)));
 }
 
 // Launches groups of up to kGroup trips, each followed by `update`, looking at
@@ -310,11 +298,9 @@ int solve_refined(TlSuite2D* s, Chunk* chunk, int max_iters, double rel_tol, int
         else rf_w<T, true>(s, b, gl, nm[1], b.f[RF_R], FinMxW{b.st});
         rf_ur<T>(s, b, gl, nm[2], FinMxUr{b.st});
     }, [&] {
-        TL_LAUNCH(s, nm[3], (tl::launch_chained(k_rf_fold<T>, gl, dim3(BX), 0, s->stream, L, b.st, s->g.x,
-                                                s->g.hd, chunk->u, b.f[RF_XS])));
-        TL_LAUNCH(s, nm[4], (tl::launch_chained(k_rf_resid<T>, gl, dim3(BX), 0, s->stream, L, b.st, s->g.x,
-                                                s->g.hd, chunk->u, chunk->u0, chunk->kx, chunk->ky, b.f[RF_R],
-                                                                      s->rs, FinMxRes{b.st, s->d_mirror})));
+        TL_LAUNCH(s, nm[3], (chain(s, k_rf_fold<T>, gl, BX, 0, L, b.st, s->g.x, s->g.hd, chunk->u, b.f[RF_XS])));
+        TL_LAUNCH(s, nm[4], (chain(s, k_rf_resid<T>, gl, BX, 0, L, b.st, s->g.x, s->g.hd, chunk->u, chunk->u0,
+                                   chunk->kx, chunk->ky, b.f[RF_R], s->rs, FinMxRes{b.st, s->d_mirror})));
     });
     MxState st{};
     TL_CUDA(cudaMemcpy(&st, b.st, sizeof(MxState), cudaMemcpyDeviceToHost));
@@ -376,11 +362,9 @@ int solve_refined_ppcg(TlSuite2D* s, Chunk* chunk, Settings* settings, double re
     T* const r = b.f[RF_R];
     T* const z = b.f[RF_Z];
     auto fold_resid = [&](double* betas) {
-        TL_LAUNCH(s, nm[3], (tl::launch_chained(k_rf_fold<T>, gl, dim3(BX), 0, s->stream, L, b.st, s->g.x,
-                                                s->g.hd, chunk->u, b.f[RF_XS])));
-        TL_LAUNCH(s, nm[4], (tl::launch_chained(k_rf_resid<T>, gl, dim3(BX), 0, s->stream, L, b.st, s->g.x,
-                                                s->g.hd, chunk->u, chunk->u0, chunk->kx, chunk->ky, r, s->rs,
-                                                                      FinMxRes{b.st, s->d_mirror, betas})));
+        TL_LAUNCH(s, nm[3], (chain(s, k_rf_fold<T>, gl, BX, 0, L, b.st, s->g.x, s->g.hd, chunk->u, b.f[RF_XS])));
+        TL_LAUNCH(s, nm[4], (chain(s, k_rf_resid<T>, gl, BX, 0, L, b.st, s->g.x, s->g.hd, chunk->u, chunk->u0,
+                                   chunk->kx, chunk->ky, r, s->rs, FinMxRes{b.st, s->d_mirror, betas})));
     };
     // CG trips up to the switch (2d/shared.h:41-42 for the constants)
     const FinMxUr cg_fin = settings->error_switch

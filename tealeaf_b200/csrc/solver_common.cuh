@@ -17,6 +17,7 @@ struct Scalar {
     double v;
     const double* dev;
     __device__ __forceinline__ double get() const { return dev ? *dev : v; }
+    __device__ __forceinline__ double fresh() const { return dev ? __ldcg(dev) : v; }   // in a chained kernel
 };
 
 // Control block of the device-resident solver loops (device memory).
@@ -64,7 +65,9 @@ __device__ __forceinline__ void end_of_trip(DevState* st, const DevParams& prm, 
         st->done = 1;
         st->reason = reason;
     }
-    if (host_mirror) {
+    // the host only looks for the end, and a kernel that writes to its memory ends
+    // when the write has crossed the bus (1 us)
+    if (host_mirror && st->done) {
         host_mirror[0] = st->done;
         host_mirror[1] = st->trip;
         host_mirror[2] = st->reason;
@@ -137,6 +140,15 @@ struct FinPcgUr {          // preconditioned CG: t = (r.r, r.z); beta = r.z / rr
 };
 
 __device__ __forceinline__ bool gate_closed(const int* done) { return done && *(volatile const int*)done; }
+
+// The same for a chained kernel, past chain_wait(): one thread of the block reads
+// the gate and the trip's scalars (every warp of a thousand blocks reading the
+// one line they are in queue up for it) and the block's next barrier hands them on.
+struct SweepHead {
+    int closed;
+    double s[3];
+    __device__ __forceinline__ void gate(const int* done) { closed = done && *(volatile const int*)done; }
+};
 
 // Chebyshev coefficients of the current trip: host values, or the device
 // tables indexed by the trip counter.

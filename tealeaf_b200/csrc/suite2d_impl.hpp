@@ -220,6 +220,23 @@ inline bool tma_usable(const TlSuite2D* s) { return s->tma && s->g.hd % 2 == 0 &
 
 inline bool tma_failed(const TlSuite2D* s) { return s->h_mirror && s->h_mirror[kTmaErrWord2] != 0; }
 
+// One of a run of sweeps on the suite's stream (tl::launch_chained).
+template <typename... P, typename... A>
+inline void chain(TlSuite2D* s, void (*kernel)(P...), dim3 grid, int block, size_t smem, A... args)
+{
+    tl::launch_chained(s->sm_count, kernel, grid, dim3(block), smem, s->stream, args...);
+}
+
+// Where the sums of a sweep go: a device-resident loop (done) keeps them on the
+// device, a call of the kernel interface has the host read them. A kernel that
+// writes to mapped host memory ends when the write has crossed the bus (1 us).
+inline ReduceSlots loop_slots(const TlSuite2D* s, const int* done)
+{
+    ReduceSlots rs = s->rs;
+    if (done) rs.out_host = nullptr;
+    return rs;
+}
+
 // The fused CG w sweep (k_cg_w_fused semantics), by TMA where possible; U: with
 // the u updates of the two trips before it. Internal linkage, like the kernels
 // it launches: each translation unit has its own kernel copies, so each keeps
@@ -245,15 +262,15 @@ static void launch_cg_w2(TlSuite2D* s, Chunk* chunk, dim3 grid, const Faces& fc,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_rows_bytes<U>()));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, name, (k_cg_w_fused_tma<F, R, U><<<grid, BX, tma_rows_bytes<U>(), s->stream>>>(
-                                   s->g, fc, beta, cu, m, p_in, p_out, r, w, u_halo, uhd, s->rs, done, fin,
-                                   s->d_mirror + kTmaErrWord2)));
+            TL_LAUNCH(s, name, (chain(s, k_cg_w_fused_tma<F, R, U, Finish>, grid, BX, tma_rows_bytes<U>(), s->g, fc,
+                                      beta, cu, m, p_in, p_out, r, w, u_halo, uhd, loop_slots(s, done), done, fin,
+                                      s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
     TL_LAUNCH(s, name, (k_cg_w_fused<F, R, U><<<grid, BX, 0, s->stream>>>(
-                           s->g, fc, beta, cu, p_in, p_out, r, w, chunk->kx, chunk->ky, u_halo, uhd, s->rs, done,
-                           fin)));
+                           s->g, fc, beta, cu, p_in, p_out, r, w, chunk->kx, chunk->ky, u_halo, uhd,
+                           loop_slots(s, done), done, fin)));
 }
 
 // The fused CG u/r update (k_cg_ur_fused semantics), by TMA where possible
@@ -275,13 +292,14 @@ static void launch_cg_ur2(TlSuite2D* s, dim3 grid, Scalar alpha, double* u, cons
                                              (int)kTmaUrBytes));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, "k_cg_ur_fused", (k_cg_ur_fused_tma<<<grid, BX, kTmaUrBytes, s->stream>>>(
-                                              s->g, alpha, m, u, r, s->rs, done, fin, s->d_mirror + kTmaErrWord2)));
+            TL_LAUNCH(s, "k_cg_ur_fused", (chain(s, k_cg_ur_fused_tma<Finish>, grid, BX, kTmaUrBytes, s->g, alpha,
+                                                 m, u, r, loop_slots(s, done), done, fin,
+                                                 s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
-    TL_LAUNCH(s, "k_cg_ur_fused", (k_cg_ur_fused<<<grid, BX, 0, s->stream>>>(s->g, alpha, u, p, r, w, s->rs, done,
-                                                                            fin)));
+    TL_LAUNCH(s, "k_cg_ur_fused", (k_cg_ur_fused<<<grid, BX, 0, s->stream>>>(
+                                      s->g, alpha, u, p, r, w, loop_slots(s, done), done, fin)));
 }
 // The fused CG r update (k_cg_r_fused semantics), by TMA where possible
 // (internal linkage as launch_cg_w2).
@@ -299,12 +317,13 @@ static void launch_cg_r2(TlSuite2D* s, dim3 grid, Scalar alpha, double* r, const
                                              (int)kTmaRBytes));
                 attr_set |= 1u << (s->device & 31);
             }
-            TL_LAUNCH(s, "k_cg_r_fused", (k_cg_r_fused_tma<<<grid, BX, kTmaRBytes, s->stream>>>(
-                                             s->g, alpha, m, r, s->rs, done, fin, s->d_mirror + kTmaErrWord2)));
+            TL_LAUNCH(s, "k_cg_r_fused", (chain(s, k_cg_r_fused_tma<Finish>, grid, BX, kTmaRBytes, s->g, alpha, m,
+                                                r, loop_slots(s, done), done, fin, s->d_mirror + kTmaErrWord2)));
             return;
         }
     }
-    TL_LAUNCH(s, "k_cg_r_fused", (k_cg_r_fused<<<grid, BX, 0, s->stream>>>(s->g, alpha, r, w, s->rs, done, fin)));
+    TL_LAUNCH(s, "k_cg_r_fused", (k_cg_r_fused<<<grid, BX, 0, s->stream>>>(s->g, alpha, r, w, loop_slots(s, done),
+                                                                            done, fin)));
 }
 // Region boxes (kTW x kTH cells, kind 4) of the TMA-staged blocked kernels.
 inline const CUtensorMap* blocked_map(TlSuite2D* s, const double* ptr)
@@ -352,8 +371,8 @@ static void launch_blocked(TlSuite2D* s, const char* name, const BlockedArgs& a,
                 const BlockedMaps m{*ma, *mb, *mc, *mx, *my};
                 const long tiles = (long)gb.x * gb.y;
                 const unsigned grid = (unsigned)std::min<long>(tiles, s->sm_count);
-                TL_LAUNCH(s, name, (k_blocked_tma<MODE><<<grid, kTBThreads, kBlockedTmaBytes, s->stream>>>(
-                                       s->g, a, m, A_out, B_out, u, w, r, done, s->d_mirror + kTmaErrWord2)));
+                TL_LAUNCH(s, name, (chain(s, k_blocked_tma<MODE>, grid, kTBThreads, kBlockedTmaBytes, s->g, a, m,
+                                          A_out, B_out, u, w, r, done, s->d_mirror + kTmaErrWord2)));
                 return;
             }
         }

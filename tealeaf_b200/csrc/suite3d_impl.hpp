@@ -229,6 +229,16 @@ static void launch_blocked3(TlSuite3D* s, Chunk* chunk, Blocked3Args a, const do
                             chunk->vec_kz, done)));
 }
 
+// Where the sums of a sweep go: a device-resident loop (done) keeps them on the
+// device, a call of the kernel interface has the host read them. A kernel that
+// writes to mapped host memory ends when the write has crossed the bus (1 us).
+inline tl::ReduceSlots loop_slots(const TlSuite3D* s, const int* done)
+{
+    tl::ReduceSlots rs = s->rs;
+    if (done) rs.out_host = nullptr;
+    return rs;
+}
+
 // The fused CG w sweep (k3_cg_w semantics), by TMA where possible; U: with the
 // u updates of the two trips before it. Internal linkage, like the kernels it launches: each translation unit has
 // its own kernel copies, so each keeps its own record of the raised
@@ -255,14 +265,15 @@ static void launch_cg_w3(TlSuite3D* s, Chunk* chunk, dim3 grid, const Faces& fc,
                 attr_set |= 1u << (s->device & 31);
             }
             TL3_LAUNCH(s, name, (k3_cg_w_tma<F, R, U><<<grid, bl, kTmaRingBytes, s->stream>>>(
-                                    s->g, fc, beta, cu, m, p_in, p_out, r, w, u_halo, uhd, s->rs, done, fin,
+                                    s->g, fc, beta, cu, m, p_in, p_out, r, w, u_halo, uhd, loop_slots(s, done), done,
+                                    fin,
                                     s->d_mirror + kTmaErrWord)));
             return;
         }
     }
     TL3_LAUNCH(s, name, (k3_cg_w<F, R, U><<<grid, bl, 0, s->stream>>>(s->g, fc, beta, cu, p_in, p_out, r, w,
                                                                       chunk->vec_kx, chunk->vec_ky, chunk->vec_kz,
-                                                                      u_halo, uhd, s->rs, done, fin)));
+                                                                      u_halo, uhd, loop_slots(s, done), done, fin)));
 }
 
 // The fused CG u/r update (k3_cg_ur semantics), by TMA where possible
@@ -286,11 +297,13 @@ static void launch_cg_ur3(TlSuite3D* s, dim3 grid, Scalar alpha, double* u, cons
                 attr_set |= 1u << (s->device & 31);
             }
             TL3_LAUNCH(s, "k3_cg_ur", (k3_cg_ur_tma<<<grid, bl, kTmaUr3Bytes, s->stream>>>(
-                                          s->g, alpha, m, u, r, s->rs, done, fin, s->d_mirror + kTmaErrWord)));
+                                          s->g, alpha, m, u, r, loop_slots(s, done), done, fin,
+                                          s->d_mirror + kTmaErrWord)));
             return;
         }
     }
-    TL3_LAUNCH(s, "k3_cg_ur", (k3_cg_ur<<<grid, bl, 0, s->stream>>>(s->g, alpha, u, p, r, w, s->rs, done, fin)));
+    TL3_LAUNCH(s, "k3_cg_ur", (k3_cg_ur<<<grid, bl, 0, s->stream>>>(s->g, alpha, u, p, r, w,
+                                                                           loop_slots(s, done), done, fin)));
 }
 
 // The fused CG r update (k3_cg_r semantics), by TMA where possible.
@@ -310,11 +323,11 @@ static void launch_cg_r3(TlSuite3D* s, dim3 grid, Scalar alpha, double* r, const
                 attr_set |= 1u << (s->device & 31);
             }
             TL3_LAUNCH(s, "k3_cg_r", (k3_cg_r_tma<<<grid, bl, kTmaR3Bytes, s->stream>>>(
-                                         s->g, alpha, m, r, s->rs, done, fin, s->d_mirror + kTmaErrWord)));
+                                         s->g, alpha, m, r, loop_slots(s, done), done, fin, s->d_mirror + kTmaErrWord)));
             return;
         }
     }
-    TL3_LAUNCH(s, "k3_cg_r", (k3_cg_r<<<grid, bl, 0, s->stream>>>(s->g, alpha, r, w, s->rs, done, fin)));
+    TL3_LAUNCH(s, "k3_cg_r", (k3_cg_r<<<grid, bl, 0, s->stream>>>(s->g, alpha, r, w, loop_slots(s, done), done, fin)));
 }
 
 // The CG loop of a mesh that does not fit on chip, its solution in u: the w
