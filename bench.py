@@ -800,7 +800,7 @@ def precond_object(n: int, peak: float, steps: int = 1, warm_cap: int = 50) -> d
     from tealeaf_b200 import problems
     from tealeaf_b200.host import Host
     out = {"workload": "dropin_2d_%d_cg, preconditioner none / jac_diag / jac_block" % n, "cells": n * n,
-           "bytes_per_cell_iteration": {"none": 96, "jac_diag": 112, "jac_block": 120}}
+           "bytes_per_cell_iteration": {"none": CG_BYTES_PER_CELL_ITER, "jac_diag": 112, "jac_block": 120}}
     for pc in ("none", "jac_diag", "jac_block"):
         prob = problems.dropin_2d(n, seed=2, steps=steps, solver="cg").with_(preconditioner=pc)
         w = Host(prob.tea_in(), dims=2)

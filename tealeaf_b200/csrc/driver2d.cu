@@ -10,7 +10,8 @@
 // Lanczos eigenvalue bounds (tridiagonal QL), the Chebyshev tables and the
 // iteration estimate (single-precision logf/roundf, as cheby_driver.c:146-160).
 //
-// The fused sweeps of kernels2d.cuh do the CG iteration in 96 B/cell, a
+// The fused sweeps of kernels2d.cuh do the CG iteration in 84 B/cell (u every
+// second trip; none on a mesh that fits on chip, cgchip2d.cuh), a
 // Chebyshev trip in 56-72 B/cell and a PPCG inner step in 64 B/cell. Memory
 // ends each solve in the state the reference leaves it in: pending updates
 // and halo reflections are closed at the end of every phase, following the
