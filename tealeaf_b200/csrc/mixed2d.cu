@@ -174,7 +174,7 @@ template <typename T>
 const CUtensorMap* rf_map(TlSuite2D* s, const Lay& L, const T* ptr, bool ring)
 {
     const int kind = 16 + (sizeof(T) == 4 ? 0 : 8) + (ring ? 1 : 0);
-    return tma_lookup(s, ptr, kind, [&](CUtensorMap* m) {
+    return s->tma_cache.lookup(ptr, kind, [&](CUtensorMap* m) {
         return tl::tma_encode_3d(m, ptr, L.xp, L.ny + 2, 1, ring ? RfRowsW<T>::H : RfRowsW<T>::W, kRfRows, 1,
                                  (int)sizeof(T));
     });

@@ -6,6 +6,7 @@
 #include "blocked2d.cuh"
 #include "gridsum.cuh"
 #include "summary.cuh"
+#include "tmacache.hpp"
 
 #include <cuda_runtime.h>
 
@@ -95,14 +96,7 @@ struct TlSuite2D {
     // CG w sweep fed by TMA where the layout allows (tl2d_set_tma); tensor
     // maps encoded once per array.
     bool tma = true;
-    struct TmaEntry {
-        const void* ptr;
-        int kind;
-        CUtensorMap map;
-    };
-    TmaEntry tma_cache[48];
-    int tma_n = 0;
-    int tma_next = 0;
+    tl::TmaCache<CUtensorMap, 48> tma_cache;
 };
 
 // Index of the int, in the mapped mirror words, that the bounded TMA barrier
@@ -182,25 +176,6 @@ FieldBufferType* field_slot(Chunk* chunk, AltField f);
 void swap_alt(TlSuite2D* s, Chunk* chunk, AltField f);
 
 
-// A cached tensor map: (ptr, kind) -> map, encoded by `encode` on a miss; a
-// full cache recycles its entries in turn (arrays of released buffers).
-template <typename Encode>
-inline const CUtensorMap* tma_lookup(TlSuite2D* s, const void* ptr, int kind, Encode encode)
-{
-    for (int i = 0; i < s->tma_n; ++i)
-        if (s->tma_cache[i].ptr == ptr && s->tma_cache[i].kind == kind) return &s->tma_cache[i].map;
-    const int cap = (int)(sizeof(s->tma_cache) / sizeof(s->tma_cache[0]));
-    const int slot = s->tma_n < cap ? s->tma_n : (s->tma_next++ % cap);
-    CUtensorMap m;
-    if (!encode(&m)) return nullptr;
-    TlSuite2D::TmaEntry& e = s->tma_cache[slot];
-    e.map = m;
-    e.ptr = ptr;
-    e.kind = kind;
-    if (s->tma_n < cap) ++s->tma_n;
-    return &e.map;
-}
-
 // Tensor map of a chunk array for k_cg_w_fused_tma: kind 0 operand rows (box
 // (BX+4) x kRowsT), 1 kx ((BX+2) x kRowsT), 2 ky (BX x kRowsT); for
 // k_cg_ur_fused_tma: kind 3 (BX x kRowsU); for k_cg_r_fused_tma: kind 5 (BX x
@@ -209,7 +184,7 @@ inline const CUtensorMap* tma_map(TlSuite2D* s, const double* ptr, int kind)
 {
     static const unsigned box[6] = {BX + 4, BX + 2, BX, BX, 0, BX};
     static const unsigned rows[6] = {kRowsT, kRowsT, kRowsT, kRowsU, 0, kRowsR};
-    return tma_lookup(s, ptr, kind, [&](CUtensorMap* m) {
+    return s->tma_cache.lookup(ptr, kind, [&](CUtensorMap* m) {
         return tl::tma_encode_3d(m, ptr, s->g.x, s->g.y, 1, box[kind], rows[kind], 1);
     });
 }
@@ -328,7 +303,7 @@ static void launch_cg_r2(TlSuite2D* s, dim3 grid, Scalar alpha, double* r, const
 // Region boxes (kTW x kTH cells, kind 4) of the TMA-staged blocked kernels.
 inline const CUtensorMap* blocked_map(TlSuite2D* s, const double* ptr)
 {
-    return tma_lookup(s, ptr, 4, [&](CUtensorMap* m) {
+    return s->tma_cache.lookup(ptr, 4, [&](CUtensorMap* m) {
         return tl::tma_encode_3d(m, ptr, s->g.x, s->g.y, 1, kTW, kTH, 1);
     });
 }

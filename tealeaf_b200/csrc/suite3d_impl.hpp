@@ -7,6 +7,7 @@
 #include "gridsum.cuh"
 #include "kernels3d.cuh"
 #include "summary.cuh"
+#include "tmacache.hpp"
 
 #include <cuda_runtime.h>
 
@@ -60,14 +61,7 @@ struct TlSuite3D {
         std::vector<double> a, b;
     };
     Queue cq, pq;
-    struct TmaEntry {
-        const double* ptr;
-        int kind;
-        CUtensorMap map;
-    };
-    TmaEntry tma_cache[40];
-    int tma_n = 0;
-    int tma_next = 0;
+    tl::TmaCache<CUtensorMap, 40> tma_cache;   // tensor maps encoded once per array
 };
 
 // Index of the int, in the mapped mirror words, that the bounded TMA barrier
@@ -159,22 +153,11 @@ void swap_alt(TlSuite3D* s, Chunk* chunk, AltField3 f);
 // array.
 inline const CUtensorMap* tma_map(TlSuite3D* s, const double* ptr, int kind)
 {
-    for (int i = 0; i < s->tma_n; ++i)
-        if (s->tma_cache[i].ptr == ptr && s->tma_cache[i].kind == kind) return &s->tma_cache[i].map;
-    // a full cache recycles its entries in turn (arrays of released buffers)
-    const int cap = (int)(sizeof(s->tma_cache) / sizeof(s->tma_cache[0]));
-    const int slot = s->tma_n < cap ? s->tma_n : (s->tma_next++ % cap);
     static const unsigned box[6][3] = {{BX + 4, BY + 2, 1}, {BX + 2, BY, 1}, {BX, BY + 1, 1}, {BX, BY, 1},
                                        {BX, BY, kPlanesU}, {kRX, kRYT, 1}};
-    CUtensorMap m;
-    if (!tl::tma_encode_3d(&m, ptr, s->g.x, s->g.y, s->g.z, box[kind][0], box[kind][1], box[kind][2]))
-        return nullptr;
-    TlSuite3D::TmaEntry& e = s->tma_cache[slot];
-    e.map = m;
-    e.ptr = ptr;
-    e.kind = kind;
-    if (s->tma_n < cap) ++s->tma_n;
-    return &e.map;
+    return s->tma_cache.lookup(ptr, kind, [&](CUtensorMap* m) {
+        return tl::tma_encode_3d(m, ptr, s->g.x, s->g.y, s->g.z, box[kind][0], box[kind][1], box[kind][2]);
+    });
 }
 
 // The TMA boxes start at x = hd - 2 + 32 bx: an even halo depth and an even
