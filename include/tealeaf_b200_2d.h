@@ -365,6 +365,14 @@ int tl2d_calculate_2norm_noalloc(const double* field, int x, int y, int halo_dep
  * (2d/shared.c:97-111); this exists to test the error path of the waits. */
 int tl2d_check_bounded_wait(Chunk* chunk, long long polls);
 
+/* No counterpart in the reference. How many polls (1 .. 2^22; 0: the default,
+ * 2^22, seconds) a block of the CG loop that runs as one persistent launch waits
+ * for another block's sums and edge cells before it gives up. A wait that gives
+ * up makes every block return and the solve report an error; the chunk's solver
+ * fields are then invalid until the next solve. For testing that path. Returns
+ * 0, or error 36 for a limit out of range. */
+int tl2d_set_chip_wait_limit(Chunk* chunk, int polls);
+
 /* The four field-summary totals from a parallel tree reduction: one sweep at
  * full bandwidth instead of run_field_summary's serial reference order, so
  * the last bits differ from the reference (accumulated like run_field_summary). */

@@ -271,6 +271,14 @@ void tl3d_set_temporal_blocking(Chunk* chunk, int on);
  * device fields by other means. Asynchronous on the chunk's stream. */
 void tl3d_flush(Chunk* chunk);
 
+/* No counterpart in the reference. How many polls (1 .. 2^22; 0: the default,
+ * 2^22, seconds) a block of the CG loop that runs as one persistent launch waits
+ * for another block's sums and edge cells before it gives up. A wait that gives
+ * up makes every block return and the solve report an error; the chunk's solver
+ * fields are then invalid until the next solve. For testing that path. Returns
+ * 0, or error 36 for a limit out of range. */
+int tl3d_set_chip_wait_limit(Chunk* chunk, int polls);
+
 /* Field ids for the host-buffer staging calls (x*y*z values each). */
 #define TL3D_DENSITY0 0
 #define TL3D_DENSITY 1

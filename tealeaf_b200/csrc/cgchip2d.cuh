@@ -52,6 +52,7 @@ struct ChipArgs {
     int* host_mirror;
     int* err;                  // device word: a wait gave up
     int* err_host;             // its mapped copy for the host
+    int polls;                 // polls of a wait before it gives up
 };
 
 // Where a block keeps the arrays other than p, r and w: registers while 128 a
@@ -279,9 +280,9 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
             const bool gs = !ghost || word_load(a.words + side_r, tag - 1, r_s);
 #pragma unroll
             for (int q = 0; q < R; ++q) p[q] = beta * p[q] + fold(q);
-            if (!gd) r_d = tl::word_wait(a.words + down_r, tag - 1, a.err, &sums.bad);
-            if (!gu) r_u = tl::word_wait(a.words + up_r, tag - 1, a.err, &sums.bad);
-            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, a.err, &sums.bad);
+            if (!gd) r_d = tl::word_wait(a.words + down_r, tag - 1, a.err, &sums.bad, a.polls);
+            if (!gu) r_u = tl::word_wait(a.words + up_r, tag - 1, a.err, &sums.bad, a.polls);
+            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, a.err, &sums.bad, a.polls);
             p_s = beta * p_s + r_s;
             p_d = beta * p_d + r_d;
             p_u = beta * p_u + r_u;
@@ -291,8 +292,8 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
         if (full) sweep_w(std::true_type(), aw[0]);
         else sweep_w(std::false_type(), aw[0]);
         if (!active) aw[0][0] = aw[0][1] = 0.0;
-        ok = tl::strip_sum<BX, 2, 1>(aw, has ? pair : -1, strips, 2 * pairs, sums, a.words, tag, a.err, [] {},
-                              [&](const double* t) { return rro / t[0]; }, pw, alpha);
+        ok = tl::strip_sum<BX, 2, 1>(aw, has ? pair : -1, strips, 2 * pairs, sums, a.words, tag, a.err, a.polls,
+                              [] {}, [&](const double* t) { return rro / t[0]; }, pw, alpha);
         if (!ok) break;
         double ar[NV][2] = {};
         if (BS) {
@@ -318,7 +319,7 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
             tl::word_store(a.words + row_w + BX, top, tag);
         }
         ok = tl::strip_sum<BX, 2, NV>(ar, has ? pair : -1, strips, 2 * pairs, sums, a.words + 2 * pairs, tag, a.err,
-                               [&] {
+                               a.polls, [&] {
 #pragma unroll
                                    for (int q = 0; q < R; ++q) {
                                        if (kRegU) u[kRegU ? q : 0] += alpha * p[q];

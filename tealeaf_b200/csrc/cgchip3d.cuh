@@ -36,6 +36,7 @@ struct Chip3Args {
     int* host_mirror;
     int* err;                  // device word: a wait gave up
     int* err_host;             // its mapped copy for the host
+    int polls;                 // polls of a wait before it gives up
 };
 
 template <int ZR, int T>
@@ -205,9 +206,9 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
             }
 #pragma unroll
             for (int q = 0; q < R; ++q) p[q] = beta * p[q] + r[q];
-            if (!gb) r_k = tl::word_wait(a.words + back_r, tag - 1, a.err, &sums.bad);
-            if (!gf) r_f = tl::word_wait(a.words + front_r, tag - 1, a.err, &sums.bad);
-            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, a.err, &sums.bad);
+            if (!gb) r_k = tl::word_wait(a.words + back_r, tag - 1, a.err, &sums.bad, a.polls);
+            if (!gf) r_f = tl::word_wait(a.words + front_r, tag - 1, a.err, &sums.bad, a.polls);
+            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, a.err, &sums.bad, a.polls);
             p_s = beta * p_s + r_s;
             p_k = beta * p_k + r_k;
             p_f = beta * p_f + r_f;
@@ -217,7 +218,7 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
                 if (!gy[m])
                     r_y[m] = tl::word_wait(a.words + rows_w +
                                                (side ? a.gx * 2 * R * 32 + q * 32 : (R + q - 2 * a.gx * R) * 32) + lane,
-                                           tag - 1, a.err, &sums.bad);
+                                           tag - 1, a.err, &sums.bad, a.polls);
                 if (n < 2 * R && q < nr && (side ? above : below)) YG[n * 32] = beta * YG[n * 32] + r_y[m];
             }
         }
@@ -231,8 +232,8 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
 #pragma unroll
             for (int h = 0; h < T; ++h) acc[0][h] = 0.0;
         // nothing to publish: every ghost was read before its reader's partial was formed
-        ok = tl::strip_sum<NT, T, 1>(acc, has ? unit : -1, strips, TW * units, sums, a.words, tag, a.err, [] {},
-                                     [&](const double* t) { return rro / t[0]; }, pw, alpha);
+        ok = tl::strip_sum<NT, T, 1>(acc, has ? unit : -1, strips, TW * units, sums, a.words, tag, a.err, a.polls,
+                                     [] {}, [&](const double* t) { return rro / t[0]; }, pw, alpha);
         if (!ok) break;
 #pragma unroll
         for (int h = 0; h < T; ++h) acc[0][h] = 0.0;
@@ -259,7 +260,7 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
             tl::word_store(a.words + ends_w + NT, top, tag);
         }
         ok = tl::strip_sum<NT, T, 1>(acc, has ? unit : -1, strips, TW * units, sums, a.words + TW * units, tag, a.err,
-                                     [&] {
+                                     a.polls, [&] {
 #pragma unroll
                                          for (int q = 0; q < R; ++q) {
                                              if (P::kRegU) u[P::kRegU ? q : 0] += alpha * p[q];
@@ -332,7 +333,7 @@ static bool cg_chip3(TlSuite3D* s, Chunk* chunk, double* u, const DevParams& prm
     Chip3Args a{chunk->vec_p, chunk->vec_r, u, chunk->vec_w, chunk->vec_kx, chunk->vec_ky, chunk->vec_kz,
                 s->chip_words, s->chip_tag, (int)grid.x, (int)grid.y, (int)grid.z,
                 tl::ceil_div(units, s->sm_count), s->d_state, s->d_cg_alphas, s->d_cg_betas, prm, s->d_mirror,
-                s->chip_err, s->d_mirror + kTmaErrWord};
+                s->chip_err, s->d_mirror + kTmaErrWord, s->chip_polls};
     s->chip_tag += (unsigned long long)prm.max_iters;
     switch (s->g.zr * 8 + c.tiles) {
         case 4 * 8 + 1: launch_chip3<4, 1>(s, a, units); break;

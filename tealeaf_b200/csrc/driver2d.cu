@@ -188,7 +188,8 @@ struct Run {
         const int pairs = chip_pairs(g, s->sm_count);
         ChipArgs a{chunk->p, chunk->r, chunk->u, chunk->w, z, chunk->kx, chunk->ky, chunk->mi, s->chip_words,
                    s->chip_tag, (int)grid.x, (int)grid.y, tl::ceil_div(pairs, s->sm_count), s->d_state,
-                   s->d_cg_alphas, s->d_cg_betas, prm, s->d_mirror, s->chip_err, s->d_mirror + kTmaErrWord2};
+                   s->d_cg_alphas, s->d_cg_betas, prm, s->d_mirror, s->chip_err,
+                   s->d_mirror + kTmaErrWord2, s->chip_polls};
         s->chip_tag += (unsigned long long)prm.max_iters;
         switch (g.rows) {
             case 2: launch_chip<2, BS>(g, a, pairs); break;

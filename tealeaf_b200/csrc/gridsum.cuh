@@ -13,15 +13,17 @@
 // each other up (6200 cycles). A word is reused with the
 // next tag; the callers see to it that it is rewritten only after all its
 // readers have taken the old value. Waits are bounded: a word that has not
-// come after kWordPolls polls raises the error word, which the other waits
-// look at every kWordErrPoll polls.
+// come after `polls` polls raises the error word, which the other waits
+// look at every kWordErrPoll polls. A block in which a wait gave up leaves the
+// loop as one, at the end of the sum it is in (StripSumSmem::ok): its threads
+// meet at barriers, so none may leave before the others.
 #pragma once
 
 #include "common.cuh"
 
 namespace tl {
 
-constexpr int kWordPolls = 1 << 22;    // each at least one L2 round trip: seconds
+constexpr int kWordPolls = 1 << 22;    // default limit: each at least one L2 round trip, so seconds
 constexpr int kWordErrPoll = 1 << 10;
 
 struct alignas(16) TagWord {
@@ -57,10 +59,10 @@ __device__ __forceinline__ bool word_load(const TagWord* s, unsigned long long t
 }
 
 // Waits for the word; sets *bad when the wait gave up (err raised).
-static __device__ __noinline__ double word_wait(const TagWord* s, unsigned long long tag, int* err, int* bad)
+static __device__ __noinline__ double word_wait(const TagWord* s, unsigned long long tag, int* err, int* bad, int polls)
 {
     double v = 0.0;
-    for (int n = 0; n < kWordPolls; ++n) {
+    for (int n = 0; n < polls; ++n) {
         if (word_load(s, tag, v)) return v;
         if ((n & (kWordErrPoll - 1)) == kWordErrPoll - 1 && *(volatile int*)err) break;
     }
@@ -81,7 +83,8 @@ struct StripSumSmem {
     double warp[NV][NH][16];   // warp sums of this block's strips
     double fin[NV][8];         // warp sums of the final pass
     double out[NV + 1];
-    int bad;
+    int bad;                   // a wait of this block gave up
+    int ok;                    // as the last sum found it: the same for every thread
 };
 
 // The values of NT / 32 warps in the order of tl::block_sum's second stage.
@@ -103,11 +106,12 @@ __device__ __forceinline__ double warps_sum(const double* q)
 // then thread t < NT adds the sums of strips t, t + NT, ... in turn and the NT
 // results go through the same tree. `between` runs after the block's words
 // are stored, before the wait. `scalar(totals)` runs in NT threads; every
-// thread gets the totals and its value. False when a wait gave up.
+// thread gets the totals and its value. False, in every thread of the block, when a
+// wait of the block gave up in this sum or before it.
 template <int NT, int NH, int NV, int NS, typename Between, typename Scalar_>
 __device__ __forceinline__ bool strip_sum(double (&v)[NV][NH], int unit, int strips, int words,
                                           StripSumSmem<NH, NS>& sm, TagWord* slots, unsigned long long tag, int* err,
-                                          Between between, Scalar_ scalar, double (&total)[NV], double& derived)
+                                          int polls, Between between, Scalar_ scalar, double (&total)[NV], double& derived)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
 #pragma unroll
@@ -143,7 +147,7 @@ __device__ __forceinline__ bool strip_sum(double (&v)[NV][NH], int unit, int str
 #pragma unroll
             for (int n = 0; n < NV; ++n)
                 if (strip_of[m] >= 0) {
-                    if (!got[m * NV + n]) x[m * NV + n] = word_wait(slots + n * words + tid + m * T, tag, err, &sm.bad);
+                    if (!got[m * NV + n]) x[m * NV + n] = word_wait(slots + n * words + tid + m * T, tag, err, &sm.bad, polls);
                     sm.vals[n][strip_of[m]] = x[m * NV + n];
                 }
     }
@@ -176,13 +180,14 @@ __device__ __forceinline__ bool strip_sum(double (&v)[NV][NH], int unit, int str
 #pragma unroll
             for (int n = 0; n < NV; ++n) sm.out[n] = t[n];
             sm.out[NV] = d;
+            sm.ok = sm.bad == 0;
         }
     }
     __syncthreads();
 #pragma unroll
     for (int n = 0; n < NV; ++n) total[n] = sm.out[n];
     derived = sm.out[NV];
-    return sm.bad == 0;
+    return sm.ok != 0;   // (not sm.bad, which a thread already past this sum may set)
 }
 
 }  // namespace tl

@@ -283,6 +283,17 @@ void tl2d_set_tma(Chunk* chunk, int on)
     TlSuite2D* s = suite_of(chunk);
     if (s) s->tma = on != 0;
 }
+int tl2d_set_chip_wait_limit(Chunk* chunk, int polls)
+{
+    TlSuite2D* s = suite_of(chunk);
+    if (!s) return tl::error_state().code;
+    if (polls < 0 || polls > tl::kWordPolls) {
+        tl::fail(36, "tl2d_set_chip_wait_limit: polls must be in [0, %d]", tl::kWordPolls);
+        return 36;
+    }
+    s->chip_polls = polls ? polls : tl::kWordPolls;
+    return 0;
+}
 void tl2d_flush(Chunk* chunk) { ready(chunk); }
 
 int tl2d_set_preconditioner(Chunk* chunk, int type)

@@ -289,6 +289,17 @@ void tl3d_set_temporal_blocking(Chunk* chunk, int on)
     TlSuite3D* s = suite_of(chunk);
     if (s) s->temporal_blocking = on != 0;
 }
+int tl3d_set_chip_wait_limit(Chunk* chunk, int polls)
+{
+    TlSuite3D* s = suite_of(chunk);
+    if (!s) return tl::error_state().code;
+    if (polls < 0 || polls > tl::kWordPolls) {
+        tl::fail(36, "tl3d_set_chip_wait_limit: polls must be in [0, %d]", tl::kWordPolls);
+        return 36;
+    }
+    s->chip_polls = polls ? polls : tl::kWordPolls;
+    return 0;
+}
 void tl3d_flush(Chunk* chunk) { ready(chunk); }
 long long tl3d_launch_count(Chunk* chunk)
 {
