@@ -313,7 +313,9 @@ template <int ZR, int T>
 static void launch_chip3(TlSuite3D* s, Chip3Args& a, int units)
 {
     const int threads = a.groups * NT, smem = a.groups * Chip3Place<ZR, T>::bytes;
-    TL_CUDA(cudaFuncSetAttribute(k3_cg_chip<ZR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // the limit of both group counts, so that a thread that launches the other one at the same time sets the same
+    TL_CUDA(cudaFuncSetAttribute(k3_cg_chip<ZR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 2 * Chip3Place<ZR, T>::bytes));
     void* args[] = {&s->g, &a};
     TL3_LAUNCH(s, "k3_cg_chip",
                TL_CUDA(cudaLaunchCooperativeKernel((const void*)k3_cg_chip<ZR, T>, dim3(tl::ceil_div(units, a.groups)),
