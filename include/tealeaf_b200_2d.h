@@ -368,7 +368,7 @@ int tl2d_check_bounded_wait(Chunk* chunk, long long polls);
 /* No counterpart in the reference. How many polls (1 .. 2^22; 0: the default,
  * 2^22, seconds) a block of the CG loop that runs as one persistent launch waits
  * for another block's sums and edge cells before it gives up. A wait that gives
- * up makes every block return and the solve report an error; the chunk's solver
+ * up makes every block return and the solve report error 38; the chunk's solver
  * fields are then invalid until the next solve. For testing that path. Returns
  * 0, or error 36 for a limit out of range. */
 int tl2d_set_chip_wait_limit(Chunk* chunk, int polls);

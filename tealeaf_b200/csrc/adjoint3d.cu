@@ -189,6 +189,7 @@ int adjoint_solve(TlSuite3D* s, Chunk* chunk, const double* rhs, double* lam, do
         DevState st{};
         TL_CUDA(cudaMemcpyAsync(&st, s->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
         TL_CUDA(cudaStreamSynchronize(s->stream));
+        check_chip(s);
         return st.trip;
     }
     return cg_deferred3(s, chunk, lam, prm, [&](auto&& trip) {
@@ -245,6 +246,7 @@ extern "C" int tl3d_solve_step_backward(Chunk* chunk, Settings* settings, const 
     face_grad(s, chunk, settings, lam, u, grad);
     TL_CUDA(cudaStreamSynchronize(s->stream));
     if (iterations) *iterations = it;
+    if (tma_failed(s)) tl::fail(35, "a TMA plane load of the w sweep did not complete (bounded barrier wait gave up)");
     return tl::failed() ? tl::error_state().code : 0;
 }
 

@@ -358,6 +358,7 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
             }
         }
     }
+    if (!ok && tid == 0) *(volatile int*)a.err_host = 1;   // whichever block it is
     if (blockIdx.x == 0 && tid == 0) {
         DevState* st = a.st;
         st->pw = pw[0];
@@ -368,7 +369,6 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
         st->trip = trip;
         st->done = 1;
         st->reason = reason;
-        if (!ok) *(volatile int*)a.err_host = 1;
         a.host_mirror[0] = 1;
         a.host_mirror[1] = trip;
         a.host_mirror[2] = reason;

@@ -292,6 +292,7 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
             }
         }
     }
+    if (!ok && tid == 0) *(volatile int*)a.err_host = 1;   // whichever block it is
     if (blockIdx.x == 0 && tid == 0) {
         DevState* st = a.st;
         st->pw = pw[0];
@@ -302,7 +303,6 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
         st->trip = trip;
         st->done = 1;
         st->reason = reason;
-        if (!ok) *(volatile int*)a.err_host = 1;
         a.host_mirror[0] = 1;
         a.host_mirror[1] = trip;
         a.host_mirror[2] = reason;
@@ -325,7 +325,8 @@ static void launch_chip3(TlSuite3D* s, Chip3Args& a, int units)
 // The whole CG loop in one launch, for a chunk with chip words: p, r, w of the
 // chunk, the solution in `u`, stopped as `prm` says; the state is left as the
 // two-launch loop leaves it, p in the buffer it was in. False (nothing done)
-// where the mesh does not fit.
+// where the mesh does not fit. The caller waits for the stream and calls
+// check_chip.
 static bool cg_chip3(TlSuite3D* s, Chunk* chunk, double* u, const DevParams& prm)
 {
     if (!s->chip_words || prm.max_iters <= 0) return false;
@@ -335,7 +336,7 @@ static bool cg_chip3(TlSuite3D* s, Chunk* chunk, double* u, const DevParams& prm
     Chip3Args a{chunk->vec_p, chunk->vec_r, u, chunk->vec_w, chunk->vec_kx, chunk->vec_ky, chunk->vec_kz,
                 s->chip_words, s->chip_tag, (int)grid.x, (int)grid.y, (int)grid.z,
                 tl::ceil_div(units, s->sm_count), s->d_state, s->d_cg_alphas, s->d_cg_betas, prm, s->d_mirror,
-                s->chip_err, s->d_mirror + kTmaErrWord, s->chip_polls};
+                s->chip_err, s->d_mirror + kChipErrWord, s->chip_polls};
     s->chip_tag += (unsigned long long)prm.max_iters;
     switch (s->g.zr * 8 + c.tiles) {
         case 4 * 8 + 1: launch_chip3<4, 1>(s, a, units); break;

@@ -189,7 +189,7 @@ struct Run {
         ChipArgs a{chunk->p, chunk->r, chunk->u, chunk->w, z, chunk->kx, chunk->ky, chunk->mi, s->chip_words,
                    s->chip_tag, (int)grid.x, (int)grid.y, tl::ceil_div(pairs, s->sm_count), s->d_state,
                    s->d_cg_alphas, s->d_cg_betas, prm, s->d_mirror, s->chip_err,
-                   s->d_mirror + kTmaErrWord2, s->chip_polls};
+                   s->d_mirror + kChipErrWord2, s->chip_polls};
         s->chip_tag += (unsigned long long)prm.max_iters;
         switch (g.rows) {
             case 2: launch_chip<2, BS>(g, a, pairs); break;
@@ -200,7 +200,9 @@ struct Run {
             case 7: launch_chip<7, BS>(g, a, pairs); break;
             default: launch_chip<kChipRows, BS>(g, a, pairs); break;
         }
-        return read_state();
+        read_state();
+        check_chip(s);
+        return host_state;
     }
     template <int H, int BS>
     void launch_chip(Geo& g, ChipArgs& a, int pairs)

@@ -137,7 +137,11 @@ struct Run3 {
     // closes the phase.
     DevState cg_phase()
     {
-        if (cg_chip3(s, chunk, chunk->vec_u, prm)) return cg_close(read_state());
+        if (cg_chip3(s, chunk, chunk->vec_u, prm)) {
+            read_state();
+            check_chip(s);
+            return cg_close(host_state);
+        }
         return cg_close(cg_deferred3(s, chunk, chunk->vec_u, prm, [&](auto&& trip) { return loop(0, trip); }));
     }
 

@@ -103,6 +103,8 @@ struct TlSuite2D {
 // Index of the int, in the mapped mirror words, that the bounded TMA barrier
 // waits set when one gives up.
 constexpr int kTmaErrWord2 = 15;
+// The same for the waits of the CG loop on chip.
+constexpr int kChipErrWord2 = 14;
 
 // Launch on the suite stream, bracketed by profiler events when enabled.
 #define TL_LAUNCH(s, name, ...)                \
@@ -195,6 +197,19 @@ inline const CUtensorMap* tma_map(TlSuite2D* s, const double* ptr, int kind)
 inline bool tma_usable(const TlSuite2D* s) { return s->tma && s->g.hd % 2 == 0 && s->g.x % 2 == 0; }
 
 inline bool tma_failed(const TlSuite2D* s) { return s->h_mirror && s->h_mirror[kTmaErrWord2] != 0; }
+
+// After a CG loop on chip has run and the stream was waited for: reports a wait
+// that gave up in it and clears its words, so that the chunk's next solve is on
+// its own.
+inline void check_chip(TlSuite2D* s)
+{
+    const int word = kChipErrWord2;
+    if (!s->h_mirror[word]) return;
+    s->h_mirror[word] = 0;
+    TL_CUDA(cudaMemsetAsync(s->chip_err, 0, sizeof(int), s->stream));
+    tl::fail(38, "the CG loop on chip did not complete: a wait for another block's sums or edge cells gave up after "
+                 "%d polls", s->chip_polls);
+}
 
 // One of a run of sweeps on the suite's stream (tl::launch_chained).
 template <typename... P, typename... A>

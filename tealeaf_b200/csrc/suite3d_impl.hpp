@@ -68,6 +68,8 @@ struct TlSuite3D {
 // Index of the int, in the mapped mirror words, that the bounded TMA barrier
 // waits set when one gives up.
 constexpr int kTmaErrWord = 15;
+// The same for the waits of the CG loop on chip.
+constexpr int kChipErrWord = 14;
 
 #define TL3_LAUNCH(s, name, ...)               \
     do {                                       \
@@ -166,6 +168,19 @@ inline const CUtensorMap* tma_map(TlSuite3D* s, const double* ptr, int kind)
 inline bool tma_usable(const TlSuite3D* s) { return s->tma && s->g.hd % 2 == 0 && s->g.x % 2 == 0; }
 
 inline bool tma_failed(const TlSuite3D* s) { return s->h_mirror && s->h_mirror[kTmaErrWord] != 0; }
+
+// After a CG loop on chip has run and the stream was waited for: reports a wait
+// that gave up in it and clears its words, so that the chunk's next solve is on
+// its own.
+inline void check_chip(TlSuite3D* s)
+{
+    const int word = kChipErrWord;
+    if (!s->h_mirror[word]) return;
+    s->h_mirror[word] = 0;
+    TL_CUDA(cudaMemsetAsync(s->chip_err, 0, sizeof(int), s->stream));
+    tl::fail(38, "the CG loop on chip did not complete: a wait for another block's sums or edge cells gave up after "
+                 "%d polls", s->chip_polls);
+}
 
 // One launch of the temporally blocked Chebyshev (MODE 0) / PPCG (MODE 1)
 // steps: region planes by TMA where the boxes can start on 16-byte

@@ -6,6 +6,7 @@ blocks' threads meet at barriers, so a block may only be left by all of its
 threads at once."""
 import ctypes as C
 
+import numpy as np
 import pytest
 
 from tealeaf_b200 import abi, problems
@@ -48,5 +49,51 @@ def test_a_limit_out_of_range_is_refused(dims, polls):
         with pytest.raises(abi.SuiteError, match="polls must be"):
             abi.check(h.lib, dims)
         h.solve_device(0)
+    finally:
+        h.finalise()
+
+
+@pytest.mark.parametrize("dims,cells,pc", MESHES)
+def test_the_error_names_the_loop_and_the_chunk_recovers(dims, cells, pc):
+    """The report is the loop's own, not that of the TMA loads, and stays with
+    the solve it belongs to: the same chunk's next solve equals a fresh one's."""
+    a, b = host(dims, cells, pc), host(dims, cells, pc)
+    try:
+        assert set_limit(a, 1) == 0
+        with pytest.raises(abi.SuiteError, match="error 38: the CG loop on chip did not complete.*after 1 polls"):
+            a.solve_device(0)
+        assert set_limit(a, 0) == 0
+        ra, rb = a.solve_device(0), b.solve_device(0)
+        assert ra.iterations == rb.iterations and ra.error == rb.error and ra.summary == rb.summary
+        for f in ("u", "p", "r", "w", "energy"):
+            assert np.array_equal(a.download(f), b.download(f)), f
+    finally:
+        a.finalise()
+        b.finalise()
+
+
+def test_the_adjoint_reports_it_too():
+    import torch
+    h = host(3, (48, 47, 50), "none")
+    try:
+        box = [2.0, 8.0, 2.0, 8.0, 2.0, 8.0]
+        h.solve_device(0)
+        n = h.shape[0] * h.shape[1] * h.shape[2]
+        g, lam, grad = (torch.ones(n, dtype=torch.float64, device="cuda") for _ in range(3))
+        its = C.c_int(0)
+
+        def backward():
+            return h.lib.tl3d_solve_step_backward(C.byref(h.chunk), C.byref(h.settings), g.data_ptr(), h.chunk.vec_u,
+                                                  lam.data_ptr(), grad.data_ptr(), 1e-8, C.byref(its))
+
+        torch.cuda.synchronize()
+        set_limit(h, 1)
+        assert backward() == 38
+        with pytest.raises(abi.SuiteError, match="error 38"):
+            abi.check(h.lib, 3)
+        with pytest.raises(abi.SuiteError, match="error 38"):
+            h.adjoint_gradient(1, 1, box, 1e-8)
+        set_limit(h, 0)
+        assert backward() == 0 and its.value > 0
     finally:
         h.finalise()
