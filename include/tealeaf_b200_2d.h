@@ -365,6 +365,15 @@ int tl2d_calculate_2norm_noalloc(const double* field, int x, int y, int halo_dep
  * (2d/shared.c:97-111); this exists to test the error path of the waits. */
 int tl2d_check_bounded_wait(Chunk* chunk, long long polls);
 
+/* No counterpart in the reference. Run the device-resident CG loop as one
+ * persistent launch where the mesh fits on chip (1, the default) or as two
+ * launches per trip (0), which larger meshes always take: the same results bit
+ * for bit (with jac_block, up to rounding of the dot products unless the mesh
+ * is cut into strips of a multiple of 4 rows).
+ * Where the process has fewer SMs than the device, the persistent launch may be
+ * refused; the solve then takes the two launches. 2 asks for a launch that is
+ * refused, to test that. Returns 0, or error 39 for another mode. */
+int tl2d_set_chip_loop(Chunk* chunk, int mode);
 /* No counterpart in the reference. How many polls (1 .. 2^22; 0: the default,
  * 2^22, seconds) a block of the CG loop that runs as one persistent launch waits
  * for another block's sums and edge cells before it gives up. A wait that gives

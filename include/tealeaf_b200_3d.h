@@ -271,6 +271,14 @@ void tl3d_set_temporal_blocking(Chunk* chunk, int on);
  * device fields by other means. Asynchronous on the chunk's stream. */
 void tl3d_flush(Chunk* chunk);
 
+/* No counterpart in the reference. Run the device-resident CG loop (of a
+ * timestep or an adjoint solve) as one persistent launch where the mesh fits on
+ * chip (1, the default) or as two launches per trip (0), which larger meshes
+ * always take: the same results bit for bit.
+ * Where the process has fewer SMs than the device, the persistent launch may be
+ * refused; the solve then takes the two launches. 2 asks for a launch that is
+ * refused, to test that. Returns 0, or error 39 for another mode. */
+int tl3d_set_chip_loop(Chunk* chunk, int mode);
 /* No counterpart in the reference. How many polls (1 .. 2^22; 0: the default,
  * 2^22, seconds) a block of the CG loop that runs as one persistent launch waits
  * for another block's sums and edge cells before it gives up. A wait that gives

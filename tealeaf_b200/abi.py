@@ -244,10 +244,11 @@ def load(dims: int) -> C.CDLL:
         f = getattr(lib, pre + "check_bounded_wait")
         f.argtypes = [C.POINTER(chunk_t), C.c_longlong]
         f.restype = _i
-    if hasattr(lib, pre + "set_chip_wait_limit"):  # 2D and 3D
-        f = getattr(lib, pre + "set_chip_wait_limit")
-        f.argtypes = [C.POINTER(chunk_t), _i]
-        f.restype = _i
+    for name in ("set_chip_loop", "set_chip_wait_limit"):  # 2D and 3D
+        if hasattr(lib, pre + name):
+            f = getattr(lib, pre + name)
+            f.argtypes = [C.POINTER(chunk_t), _i]
+            f.restype = _i
     if hasattr(lib, pre + "adjoint_gradient"):
         f = getattr(lib, pre + "adjoint_gradient")
         f.argtypes = head + [_i, _i, C.POINTER(_d), _d, _p, C.POINTER(AdjointStats)]

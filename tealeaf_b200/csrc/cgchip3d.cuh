@@ -310,26 +310,25 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
 }
 
 template <int ZR, int T>
-static void launch_chip3(TlSuite3D* s, Chip3Args& a, int units)
+static bool launch_chip3(TlSuite3D* s, Chip3Args& a, int units)
 {
     const int threads = a.groups * NT, smem = a.groups * Chip3Place<ZR, T>::bytes;
     // the limit of both group counts, so that a thread that launches the other one at the same time sets the same
     TL_CUDA(cudaFuncSetAttribute(k3_cg_chip<ZR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  2 * Chip3Place<ZR, T>::bytes));
     void* args[] = {&s->g, &a};
-    TL3_LAUNCH(s, "k3_cg_chip",
-               TL_CUDA(cudaLaunchCooperativeKernel((const void*)k3_cg_chip<ZR, T>, dim3(tl::ceil_div(units, a.groups)),
-                                                   dim3(threads), args, smem, s->stream)));
+    return tl::launch_persistent(s, "k3_cg_chip", (const void*)k3_cg_chip<ZR, T>, tl::ceil_div(units, a.groups), threads,
+                                 args, smem);
 }
 
 // The whole CG loop in one launch, for a chunk with chip words: p, r, w of the
 // chunk, the solution in `u`, stopped as `prm` says; the state is left as the
 // two-launch loop leaves it, p in the buffer it was in. False (nothing done)
-// where the mesh does not fit. The caller waits for the stream and calls
-// check_chip.
+// where it does not run: the mesh does not fit, or not all its blocks do. The
+// caller waits for the stream and calls check_chip.
 static bool cg_chip3(TlSuite3D* s, Chunk* chunk, double* u, const DevParams& prm)
 {
-    if (!s->chip_words || prm.max_iters <= 0) return false;
+    if (!s->chip_words || !s->chip_loop || prm.max_iters <= 0) return false;
     const dim3 grid = interior_grid(s->g);
     const Chip3Cut c = chip3_cut(s->g, s->sm_count);
     const int units = (int)(grid.x * grid.y) * tl::ceil_div(grid.z, c.tiles);
@@ -339,17 +338,16 @@ static bool cg_chip3(TlSuite3D* s, Chunk* chunk, double* u, const DevParams& prm
                 s->chip_err, s->d_mirror + kChipErrWord, s->chip_polls};
     s->chip_tag += (unsigned long long)prm.max_iters;
     switch (s->g.zr * 8 + c.tiles) {
-        case 4 * 8 + 1: launch_chip3<4, 1>(s, a, units); break;
-        case 4 * 8 + 2: launch_chip3<4, 2>(s, a, units); break;
-        case 4 * 8 + 3: launch_chip3<4, 3>(s, a, units); break;
-        case 4 * 8 + 4: launch_chip3<4, 4>(s, a, units); break;
-        case 5 * 8 + 1: launch_chip3<5, 1>(s, a, units); break;
-        case 5 * 8 + 2: launch_chip3<5, 2>(s, a, units); break;
-        case 5 * 8 + 3: launch_chip3<5, 3>(s, a, units); break;
-        case 6 * 8 + 1: launch_chip3<6, 1>(s, a, units); break;
-        default: launch_chip3<6, 2>(s, a, units); break;
+        case 4 * 8 + 1: return launch_chip3<4, 1>(s, a, units);
+        case 4 * 8 + 2: return launch_chip3<4, 2>(s, a, units);
+        case 4 * 8 + 3: return launch_chip3<4, 3>(s, a, units);
+        case 4 * 8 + 4: return launch_chip3<4, 4>(s, a, units);
+        case 5 * 8 + 1: return launch_chip3<5, 1>(s, a, units);
+        case 5 * 8 + 2: return launch_chip3<5, 2>(s, a, units);
+        case 5 * 8 + 3: return launch_chip3<5, 3>(s, a, units);
+        case 6 * 8 + 1: return launch_chip3<6, 1>(s, a, units);
+        default: return launch_chip3<6, 2>(s, a, units);
     }
-    return true;
 }
 
 }  // namespace tl3d

@@ -116,6 +116,36 @@ inline void launch_chained(int sm_count, void (*kernel)(P...), dim3 grid, dim3 b
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Whether a chunk's CG loop runs as one persistent launch where its mesh fits on
+// chip (set_chip_loop).
+enum ChipLoop {
+    kChipOff = 0,       // never
+    kChipOn = 1,        // the default
+    kChipRefused = 2,   // asked for with more blocks than any device holds at once, which the driver refuses
+};
+constexpr int kChipTooMany = 1 << 20;
+
+// Cooperative launch of a persistent loop on the suite's stream. False, with
+// nothing done, where the blocks cannot all be resident: a process that was
+// given part of the device's SMs may still see their full number, and only the
+// launch tells. The caller then runs its launched loop.
+template <typename Suite>
+inline bool launch_persistent(Suite* s, const char* name, const void* kernel, int blocks, int threads, void** args,
+                              size_t smem)
+{
+    if (s->chip_loop == kChipRefused) blocks += kChipTooMany;
+    s->prof.begin(s->stream, name);
+    const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(threads), args, smem, s->stream);
+    s->prof.end(s->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        --s->prof.launches;
+        return false;
+    }
+    TL_CUDA(e);
+    return true;
+}
+
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
 // -------------------------------------------------------------- profiler --

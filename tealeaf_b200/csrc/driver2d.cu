@@ -140,7 +140,7 @@ struct Run {
     // of u and p.
     DevState cg_phase()
     {
-        if (s->chip_words && prm.max_iters > 0) return cg_close(cg_chip<0>(s->g, nullptr), chunk->r);
+        if (cg_chip<0>(s->g, nullptr)) return cg_close(host_state, chunk->r);
         return cg_deferred();
     }
 
@@ -180,42 +180,46 @@ struct Run {
 
     // The whole loop in one launch (k_cg_chip) for a mesh whose state fits on
     // the SMs, in strips of g.rows rows; its strip pairs spread over as many
-    // SMs as there are. BS, z: the preconditioned CG's block and field.
+    // SMs as there are. BS, z: the preconditioned CG's block and field. The
+    // state it ends in is read back; false (nothing done) where it does not run.
     template <int BS>
-    DevState cg_chip(Geo g, double* z)
+    bool cg_chip(Geo g, double* z)
     {
         const dim3 grid = interior_grid(g);
         const int pairs = chip_pairs(g, s->sm_count);
+        if (!s->chip_words || !s->chip_loop || pairs == 0 || prm.max_iters <= 0) return false;
         ChipArgs a{chunk->p, chunk->r, chunk->u, chunk->w, z, chunk->kx, chunk->ky, chunk->mi, s->chip_words,
                    s->chip_tag, (int)grid.x, (int)grid.y, tl::ceil_div(pairs, s->sm_count), s->d_state,
                    s->d_cg_alphas, s->d_cg_betas, prm, s->d_mirror, s->chip_err,
                    s->d_mirror + kChipErrWord2, s->chip_polls};
         s->chip_tag += (unsigned long long)prm.max_iters;
+        bool ran = false;
         switch (g.rows) {
-            case 2: launch_chip<2, BS>(g, a, pairs); break;
-            case 3: launch_chip<3, BS>(g, a, pairs); break;
-            case 4: launch_chip<4, BS>(g, a, pairs); break;
-            case 5: launch_chip<5, BS>(g, a, pairs); break;
-            case 6: launch_chip<6, BS>(g, a, pairs); break;
-            case 7: launch_chip<7, BS>(g, a, pairs); break;
-            default: launch_chip<kChipRows, BS>(g, a, pairs); break;
+            case 2: ran = launch_chip<2, BS>(g, a, pairs); break;
+            case 3: ran = launch_chip<3, BS>(g, a, pairs); break;
+            case 4: ran = launch_chip<4, BS>(g, a, pairs); break;
+            case 5: ran = launch_chip<5, BS>(g, a, pairs); break;
+            case 6: ran = launch_chip<6, BS>(g, a, pairs); break;
+            case 7: ran = launch_chip<7, BS>(g, a, pairs); break;
+            default: ran = launch_chip<kChipRows, BS>(g, a, pairs); break;
         }
+        if (!ran) return false;
         read_state();
         check_chip(s);
-        return host_state;
+        return true;
     }
     template <int H, int BS>
-    void launch_chip(Geo& g, ChipArgs& a, int pairs)
+    bool launch_chip(Geo& g, ChipArgs& a, int pairs)
     {
         if constexpr (BS == 0 || H % BS == 0) {
             const int threads = a.groups * BX;
             constexpr size_t smem = ChipPlace<H, BS>::bytes;
             TL_CUDA(cudaFuncSetAttribute(k_cg_chip<H, BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             void* args[] = {&g, &a};
-            TL_LAUNCH(s, "k_cg_chip", TL_CUDA(cudaLaunchCooperativeKernel((const void*)k_cg_chip<H, BS>,
-                                                                          dim3(tl::ceil_div(pairs, a.groups)),
-                                                                          dim3(threads), args, smem, s->stream)));
+            return tl::launch_persistent(s, "k_cg_chip", (const void*)k_cg_chip<H, BS>,
+                                         tl::ceil_div(pairs, a.groups), threads, args, smem);
         }
+        return false;
     }
 
     // The CG loop with `fold` the field of the p update p = beta p + fold (r
@@ -283,8 +287,7 @@ struct Run {
                                        gb, fc, chunk->r, chunk->kx, chunk->ky, chunk->mi, z, chunk->p, s->rs,
                                        FinCgInit{s->d_state, s->d_mirror})));
         read_state();
-        if (s->chip_words && chip_pairs(gb, s->sm_count) > 0 && prm.max_iters > 0)
-            return cg_close(cg_chip<BS>(gb, z), z);
+        if (cg_chip<BS>(gb, z)) return cg_close(host_state, z);
         FinPcgUr fin_ur{s->d_state, s->d_cg_betas, prm, s->d_mirror};
         const Scalar alpha{0.0, &s->d_state->alpha};
         if (tma_usable(s)) {

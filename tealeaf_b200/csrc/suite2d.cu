@@ -283,6 +283,17 @@ void tl2d_set_tma(Chunk* chunk, int on)
     TlSuite2D* s = suite_of(chunk);
     if (s) s->tma = on != 0;
 }
+int tl2d_set_chip_loop(Chunk* chunk, int mode)
+{
+    TlSuite2D* s = suite_of(chunk);
+    if (!s) return tl::error_state().code;
+    if (mode < tl::kChipOff || mode > tl::kChipRefused) {
+        tl::fail(39, "tl2d_set_chip_loop: mode %d is not 0 (off), 1 (on) or 2 (refused)", mode);
+        return 39;
+    }
+    s->chip_loop = mode;
+    return 0;
+}
 int tl2d_set_chip_wait_limit(Chunk* chunk, int polls)
 {
     TlSuite2D* s = suite_of(chunk);

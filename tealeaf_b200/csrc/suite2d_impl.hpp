@@ -62,6 +62,7 @@ struct TlSuite2D {
     tl::TagWord* chip_words = nullptr;
     unsigned long long chip_tag = 0;
     int* chip_err = nullptr;
+    int chip_loop = tl::kChipOn;       // whether that loop is used (tl2d_set_chip_loop)
     int chip_polls = tl::kWordPolls;   // polls of a wait before it gives up (tl2d_set_chip_wait_limit)
 
     // Device-resident driver: Chebyshev trips / PPCG inner steps temporally

@@ -289,6 +289,17 @@ void tl3d_set_temporal_blocking(Chunk* chunk, int on)
     TlSuite3D* s = suite_of(chunk);
     if (s) s->temporal_blocking = on != 0;
 }
+int tl3d_set_chip_loop(Chunk* chunk, int mode)
+{
+    TlSuite3D* s = suite_of(chunk);
+    if (!s) return tl::error_state().code;
+    if (mode < tl::kChipOff || mode > tl::kChipRefused) {
+        tl::fail(39, "tl3d_set_chip_loop: mode %d is not 0 (off), 1 (on) or 2 (refused)", mode);
+        return 39;
+    }
+    s->chip_loop = mode;
+    return 0;
+}
 int tl3d_set_chip_wait_limit(Chunk* chunk, int polls)
 {
     TlSuite3D* s = suite_of(chunk);

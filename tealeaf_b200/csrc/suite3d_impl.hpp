@@ -52,6 +52,7 @@ struct TlSuite3D {
     tl::TagWord* chip_words = nullptr;
     unsigned long long chip_tag = 0;
     int* chip_err = nullptr;
+    int chip_loop = tl::kChipOn;       // whether that loop is used (tl3d_set_chip_loop)
     int chip_polls = tl::kWordPolls;   // polls of a wait before it gives up (tl3d_set_chip_wait_limit)
     bool tma = true;   // feed the CG w sweep by TMA where the layout allows (tl3d_set_tma)
     bool temporal_blocking = true;   // Chebyshev / PPCG blocks (tl3d_set_temporal_blocking)
