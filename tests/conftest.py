@@ -21,6 +21,19 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200) and the built suite libraries")
 
 
+def pytest_collection_modifyitems(items):
+    """The reference's multi-rank host linked with the B200 library is built
+    from the reference's own sources (build() leaves it out where they are
+    absent): without it its test skips, as those of the reference's other
+    programs do."""
+    from oracle.oracle import REF_DIR
+    if (REF_DIR / "harness2d_b200_mpi").exists():
+        return
+    for item in items:
+        if getattr(item, "originalname", "") == "test_reference_multi_rank_host_on_the_b200_library":
+            item.add_marker(pytest.mark.skip(reason="oracle/_ref/harness2d_b200_mpi not built"))
+
+
 @pytest.fixture(scope="session")
 def oracle_lib():
     from oracle.oracle import OracleLib
