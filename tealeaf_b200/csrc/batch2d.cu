@@ -80,7 +80,6 @@ struct BProb {
     Lay L;
     int tx, ty;      // tiles per row / column
     int tile0;       // first global tile of this problem
-    int gsize;       // blocks of the problem's group
     int gx, hd;      // FP64 chunk arrays: row length, halo depth
     float* f[BF_COUNT];
     double* u;
@@ -761,8 +760,7 @@ bool batch_layout(TlBatch* B, int tile_rows)
         Q.ty = (int)t.y;
         Q.tile0 = tiles;
         tiles += Q.tx * Q.ty;
-        Q.gsize = std::min(size[b], Q.tx * Q.ty);
-        for (int k = 0; k < Q.gsize; ++k) bp.push_back(b);
+        bp.insert(bp.end(), std::min(size[b], Q.tx * Q.ty), b);
         Q.gx = B->suites[b]->g.x;
         Q.hd = B->suites[b]->g.hd;
         char* base = (char*)B->slab + B->field_off[b];

@@ -222,35 +222,25 @@ struct Run {
         return false;
     }
 
-    // The CG loop with `fold` the field of the p update p = beta p + fold (r
-    // for CG, z for the preconditioned CG) and ur(p) launching the second
-    // sweep of a trip on the current p buffer.
+    // The preconditioned CG loop in two launches per trip: z folded into p by
+    // the w sweep, ur(p) launching the trip's second sweep on its p buffer.
     template <typename Ur>
-    DevState cg_trips(int from, bool fresh, const double* fold, Ur&& ur)
+    DevState pcg_trips(const double* z, Ur&& ur)
     {
-        double* buf[2] = {chunk->p, s->alt[ALT_P]};
+        double* buf[2] = {chunk->p, s->alt[ALT_P]};   // trip t's p is buf[t & 1]
         FinCgW fin_w{s->d_state, s->d_cg_alphas};
         const Scalar beta{0.0, &s->d_state->beta};
-        // parity of the current p buffer: trip t (t > from or !fresh) writes buf[(t - from + base) & 1]
-        int cur = 0;
-        auto trip = [&](int t) {
-            if (fresh && t == from) {
-                launch_cg_w2<false, false>(s, chunk, gh, fc, beta, buf[cur], buf[cur], fold, chunk->w, nullptr,
-                                           0, done(), fin_w);
-            } else {
-                launch_cg_w2<true, true>(s, chunk, gh, fc, beta, buf[cur], buf[cur ^ 1], fold, chunk->w,
-                                         nullptr, 0, done(), fin_w);
-                cur ^= 1;
-            }
-            ur(buf[cur]);
-        };
-        DevState st = loop(from, trip);
-        // Trips from..st.trip-1 ran; the fused ones flipped the current buffer.
-        const int ran = st.trip - from;
-        const int flips = fresh ? std::max(0, ran - 1) : ran;
-        double* pcur = buf[flips & 1];
-        if (pcur != chunk->p) swap_alt(s, chunk, ALT_P);
-        return cg_close(st, fold);
+        DevState st = loop(0, [&](int t) {
+            double* const p = buf[t & 1];
+            if (t == 0)
+                launch_cg_w2<false, false>(s, chunk, gh, fc, beta, p, p, z, chunk->w, nullptr, 0, done(), fin_w);
+            else
+                launch_cg_w2<true, true>(s, chunk, gh, fc, beta, buf[(t + 1) & 1], p, z, chunk->w, nullptr, 0, done(),
+                                         fin_w);
+            ur(p);
+        });
+        if (st.trip > 0 && st.trip % 2 == 0) swap_alt(s, chunk, ALT_P);   // the last trip's is the second buffer
+        return cg_close(st, z);
     }
 
     // Closes a CG phase that ended in state st: the last p update, the halos
@@ -298,7 +288,7 @@ struct Run {
                 attr_set |= 1u << (s->device & 31);
             }
         }
-        return cg_trips(0, true, z, [&](double* p) {
+        return pcg_trips(z, [&](double* p) {
             const CUtensorMap *mu = nullptr, *mp = nullptr, *mr = nullptr, *mw = nullptr, *mm = nullptr, *my = nullptr;
             if (tma_usable(s)) {
                 mu = tma_map(s, chunk->u, 3);
