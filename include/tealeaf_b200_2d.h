@@ -374,12 +374,12 @@ int tl2d_check_bounded_wait(Chunk* chunk, long long polls);
  * refused; the solve then takes the two launches. 2 asks for a launch that is
  * refused, to test that. Returns 0, or error 39 for another mode. */
 int tl2d_set_chip_loop(Chunk* chunk, int mode);
-/* No counterpart in the reference. How many polls (1 .. 2^22; 0: the default,
- * 2^22, seconds) a block of the CG loop that runs as one persistent launch waits
- * for another block's sums and edge cells before it gives up. A wait that gives
- * up makes every block return and the solve report error 38; the chunk's solver
- * fields are then invalid until the next solve. For testing that path. Returns
- * 0, or error 36 for a limit out of range. */
+/* No counterpart in the reference. How many polls (1 .. 2^22, in steps of 1024
+ * from there on; 0: the default, 2^22, seconds) a block of the CG loop that runs
+ * as one persistent launch waits for another block's sums and edge cells before
+ * it gives up. A wait that gives up makes every block return and the solve
+ * report error 38; the chunk's solver fields are then invalid until the next
+ * solve. For testing that path. Returns 0, or error 36 for a limit out of range. */
 int tl2d_set_chip_wait_limit(Chunk* chunk, int polls);
 
 /* The four field-summary totals from a parallel tree reduction: one sweep at

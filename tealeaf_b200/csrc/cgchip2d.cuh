@@ -100,7 +100,7 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
         const int row = (n >> 1) / a.gx * 2 + (n & 1);
         sums.strip_of[n] = (short)(row < a.gy ? (n >> 1) % a.gx + row * a.gx : -1);
     }
-    if (tid == 0) sums.bad = 0;
+    if (tid == 0) sums.waits = {a.err, a.polls, max(0, tl::kWordErrPoll - a.polls), 0};
     const int k = g.hd + bx * BX + tid % BX;
     const int j0 = has ? g.hd + by * g.rows : g.hd, j1 = min(j0 + 2 * g.rows, g.y - g.hd);
     const int nr = has ? j1 - j0 : 1;
@@ -280,9 +280,9 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
             const bool gs = !ghost || word_load(a.words + side_r, tag - 1, r_s);
 #pragma unroll
             for (int q = 0; q < R; ++q) p[q] = beta * p[q] + fold(q);
-            if (!gd) r_d = tl::word_wait(a.words + down_r, tag - 1, a.err, &sums.bad, a.polls);
-            if (!gu) r_u = tl::word_wait(a.words + up_r, tag - 1, a.err, &sums.bad, a.polls);
-            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, a.err, &sums.bad, a.polls);
+            if (!gd) r_d = tl::word_wait(a.words + down_r, tag - 1, &sums.waits);
+            if (!gu) r_u = tl::word_wait(a.words + up_r, tag - 1, &sums.waits);
+            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, &sums.waits);
             p_s = beta * p_s + r_s;
             p_d = beta * p_d + r_d;
             p_u = beta * p_u + r_u;
@@ -292,8 +292,8 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
         if (full) sweep_w(std::true_type(), aw[0]);
         else sweep_w(std::false_type(), aw[0]);
         if (!active) aw[0][0] = aw[0][1] = 0.0;
-        ok = tl::strip_sum<BX, 2, 1>(aw, has ? pair : -1, strips, 2 * pairs, sums, a.words, tag, a.err, a.polls,
-                              [] {}, [&](const double* t) { return rro / t[0]; }, pw, alpha);
+        ok = tl::strip_sum<BX, 2, 1>(aw, has ? pair : -1, strips, 2 * pairs, sums, a.words, tag, [] {},
+                              [&](const double* t) { return rro / t[0]; }, pw, alpha);
         if (!ok) break;
         double ar[NV][2] = {};
         if (BS) {
@@ -318,8 +318,8 @@ static __global__ void __launch_bounds__(kChipT, 1) k_cg_chip(Geo g, ChipArgs a)
             }
             tl::word_store(a.words + row_w + BX, top, tag);
         }
-        ok = tl::strip_sum<BX, 2, NV>(ar, has ? pair : -1, strips, 2 * pairs, sums, a.words + 2 * pairs, tag, a.err,
-                               a.polls, [&] {
+        ok = tl::strip_sum<BX, 2, NV>(ar, has ? pair : -1, strips, 2 * pairs, sums, a.words + 2 * pairs, tag,
+                               [&] {
 #pragma unroll
                                    for (int q = 0; q < R; ++q) {
                                        if (kRegU) u[kRegU ? q : 0] += alpha * p[q];

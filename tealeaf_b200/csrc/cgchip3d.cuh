@@ -76,7 +76,7 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
         const int un = n / TW, h = n % TW, bz = un / (a.gx * a.gy) * T + h;
         sums.strip_of[n] = (short)(h < T && bz < a.tiles_z ? un % (a.gx * a.gy) + a.gx * a.gy * bz : -1);
     }
-    if (tid == 0) sums.bad = 0;
+    if (tid == 0) sums.waits = {a.err, a.polls, max(0, tl::kWordErrPoll - a.polls), 0};
     const int hd = g.hd, x = g.x, xy = g.x * g.y;   // a mesh that fits on chip has 32-bit indices
     const int k = hd + bx * BX + lane, j = hd + by * BY + ty;
     const int i0 = has ? hd + cz * R : hd, i1 = min(i0 + R, g.z - hd);
@@ -206,9 +206,9 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
             }
 #pragma unroll
             for (int q = 0; q < R; ++q) p[q] = beta * p[q] + r[q];
-            if (!gb) r_k = tl::word_wait(a.words + back_r, tag - 1, a.err, &sums.bad, a.polls);
-            if (!gf) r_f = tl::word_wait(a.words + front_r, tag - 1, a.err, &sums.bad, a.polls);
-            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, a.err, &sums.bad, a.polls);
+            if (!gb) r_k = tl::word_wait(a.words + back_r, tag - 1, &sums.waits);
+            if (!gf) r_f = tl::word_wait(a.words + front_r, tag - 1, &sums.waits);
+            if (!gs) r_s = tl::word_wait(a.words + side_r, tag - 1, &sums.waits);
             p_s = beta * p_s + r_s;
             p_k = beta * p_k + r_k;
             p_f = beta * p_f + r_f;
@@ -218,7 +218,7 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
                 if (!gy[m])
                     r_y[m] = tl::word_wait(a.words + rows_w +
                                                (side ? a.gx * 2 * R * 32 + q * 32 : (R + q - 2 * a.gx * R) * 32) + lane,
-                                           tag - 1, a.err, &sums.bad, a.polls);
+                                           tag - 1, &sums.waits);
                 if (n < 2 * R && q < nr && (side ? above : below)) YG[n * 32] = beta * YG[n * 32] + r_y[m];
             }
         }
@@ -232,8 +232,8 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
 #pragma unroll
             for (int h = 0; h < T; ++h) acc[0][h] = 0.0;
         // nothing to publish: every ghost was read before its reader's partial was formed
-        ok = tl::strip_sum<NT, T, 1>(acc, has ? unit : -1, strips, TW * units, sums, a.words, tag, a.err, a.polls,
-                                     [] {}, [&](const double* t) { return rro / t[0]; }, pw, alpha);
+        ok = tl::strip_sum<NT, T, 1>(acc, has ? unit : -1, strips, TW * units, sums, a.words, tag, [] {},
+                                     [&](const double* t) { return rro / t[0]; }, pw, alpha);
         if (!ok) break;
 #pragma unroll
         for (int h = 0; h < T; ++h) acc[0][h] = 0.0;
@@ -259,8 +259,8 @@ static __global__ void __launch_bounds__(2 * NT, 1) k3_cg_chip(Geo g, Chip3Args 
             }
             tl::word_store(a.words + ends_w + NT, top, tag);
         }
-        ok = tl::strip_sum<NT, T, 1>(acc, has ? unit : -1, strips, TW * units, sums, a.words + TW * units, tag, a.err,
-                                     a.polls, [&] {
+        ok = tl::strip_sum<NT, T, 1>(acc, has ? unit : -1, strips, TW * units, sums, a.words + TW * units, tag,
+                                     [&] {
 #pragma unroll
                                          for (int q = 0; q < R; ++q) {
                                              if (P::kRegU) u[P::kRegU ? q : 0] += alpha * p[q];

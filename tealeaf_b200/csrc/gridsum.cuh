@@ -13,7 +13,7 @@
 // each other up (6200 cycles). A word is reused with the
 // next tag; the callers see to it that it is rewritten only after all its
 // readers have taken the old value. Waits are bounded: a word that has not
-// come after `polls` polls raises the error word, which the other waits
+// come after a number of polls raises the error word, which the other waits
 // look at every kWordErrPoll polls. A block in which a wait gave up leaves the
 // loop as one, at the end of the sum it is in (StripSumSmem::ok): its threads
 // meet at barriers, so none may leave before the others.
@@ -24,7 +24,7 @@
 namespace tl {
 
 constexpr int kWordPolls = 1 << 22;    // default limit: each at least one L2 round trip, so seconds
-constexpr int kWordErrPoll = 1 << 10;
+constexpr int kWordErrPoll = 1 << 10;  // (a power of two)
 
 struct alignas(16) TagWord {
     double value;
@@ -58,21 +58,32 @@ __device__ __forceinline__ bool word_load(const TagWord* s, unsigned long long t
     return hi == tag;
 }
 
-// Waits for the word; sets *bad when the wait gave up (err raised).
-static __device__ __noinline__ double word_wait(const TagWord* s, unsigned long long tag, int* err, int* bad, int polls)
+// What the waits of a block share. They look at it, and at the error word, after
+// every kWordErrPoll polls only (a shorter limit starts the count late): a limit
+// looked at after every poll, here or as an argument of the call, took 3 to 5 %
+// of the preconditioned loop at 1013 x 777 (23.1 to 24.0 ms a timestep).
+struct WordWaits {
+    int* err;    // device word raised by the waits that give up
+    int polls;   // limit of a wait
+    int skip;    // polls the count starts at: kWordErrPoll - polls, 0 for a longer limit
+    int bad;     // a wait of this block gave up
+};
+
+// Waits for the word; sets waits->bad when the wait gave up (*waits->err raised).
+static __device__ __noinline__ double word_wait(const TagWord* s, unsigned long long tag, WordWaits* waits)
 {
     double v = 0.0;
-    for (int n = 0; n < polls; ++n) {
+    int n = waits->skip;
+    do {
         if (word_load(s, tag, v)) return v;
-        if ((n & (kWordErrPoll - 1)) == kWordErrPoll - 1 && *(volatile int*)err) break;
-    }
-    *(volatile int*)err = 1;
-    *bad = 1;
+        if ((n & (kWordErrPoll - 1)) == kWordErrPoll - 1 && (*(volatile int*)waits->err || n >= waits->polls)) break;
+    } while (++n < kWordPolls);
+    *(volatile int*)waits->err = 1;
+    waits->bad = 1;
     return v;
 }
 
-// Shared memory of strip_sum for up to NV sums of up to NH strips at once;
-// `bad` starts at 0.
+// Shared memory of strip_sum for up to NV sums of up to NH strips at once.
 constexpr int kStripMax = 1280;   // strips of a mesh
 // Words a group of NH strips has per sum: whole sectors.
 constexpr int strip_words(int nh) { return (nh + 1) / 2 * 2; }
@@ -83,7 +94,7 @@ struct StripSumSmem {
     double warp[NV][NH][16];   // warp sums of this block's strips
     double fin[NV][8];         // warp sums of the final pass
     double out[NV + 1];
-    int bad;                   // a wait of this block gave up
+    WordWaits waits;           // set before the first wait
     int ok;                    // as the last sum found it: the same for every thread
 };
 
@@ -110,8 +121,8 @@ __device__ __forceinline__ double warps_sum(const double* q)
 // wait of the block gave up in this sum or before it.
 template <int NT, int NH, int NV, int NS, typename Between, typename Scalar_>
 __device__ __forceinline__ bool strip_sum(double (&v)[NV][NH], int unit, int strips, int words,
-                                          StripSumSmem<NH, NS>& sm, TagWord* slots, unsigned long long tag, int* err,
-                                          int polls, Between between, Scalar_ scalar, double (&total)[NV], double& derived)
+                                          StripSumSmem<NH, NS>& sm, TagWord* slots, unsigned long long tag,
+                                          Between between, Scalar_ scalar, double (&total)[NV], double& derived)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
 #pragma unroll
@@ -147,7 +158,8 @@ __device__ __forceinline__ bool strip_sum(double (&v)[NV][NH], int unit, int str
 #pragma unroll
             for (int n = 0; n < NV; ++n)
                 if (strip_of[m] >= 0) {
-                    if (!got[m * NV + n]) x[m * NV + n] = word_wait(slots + n * words + tid + m * T, tag, err, &sm.bad, polls);
+                    if (!got[m * NV + n])
+                        x[m * NV + n] = word_wait(slots + n * words + tid + m * T, tag, &sm.waits);
                     sm.vals[n][strip_of[m]] = x[m * NV + n];
                 }
     }
@@ -180,14 +192,14 @@ __device__ __forceinline__ bool strip_sum(double (&v)[NV][NH], int unit, int str
 #pragma unroll
             for (int n = 0; n < NV; ++n) sm.out[n] = t[n];
             sm.out[NV] = d;
-            sm.ok = sm.bad == 0;
+            sm.ok = sm.waits.bad == 0;
         }
     }
     __syncthreads();
 #pragma unroll
     for (int n = 0; n < NV; ++n) total[n] = sm.out[n];
     derived = sm.out[NV];
-    return sm.ok != 0;   // (not sm.bad, which a thread already past this sum may set)
+    return sm.ok != 0;   // (not waits.bad, which a thread already past this sum may set)
 }
 
 }  // namespace tl
