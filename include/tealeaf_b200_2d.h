@@ -440,19 +440,19 @@ typedef struct TlBatchStats
     int total_iterations;   /* summed over the problems */
     int kernel_iterations;  /* iterations the persistent kernel ran */
     int tile_rows;          /* tile height in use */
-    int grid_blocks;        /* persistent grid in use */
+    int grid_blocks;        /* blocks the problems' groups are cut for (as many as fit at once are launched) */
     int graph;              /* 1 when the step ran as a CUDA graph replay */
     double device_ms;       /* device time of the whole batched timestep */
 } TlBatchStats;
 
-/* tile_rows, grid_blocks: 0 for the defaults (16; the co-residency limit);
+/* tile_rows, grid_blocks: 0 for the defaults (16; 8 blocks per SM, the most);
  * tile_rows -1: per-problem heights (see tl2d_batch_tune). */
 TlBatch* tl2d_batch_create(Chunk** chunks, Settings** settings, int count, int tile_rows, int grid_blocks);
 void tl2d_batch_destroy(TlBatch* batch);
 /* Autotuner: times trial_iters iterations of the batch (0: the whole solve)
  * for each tile height in {-1 = per problem, about one tile per block of the
- * grid, 8..64 rows; 4, 8, 16, 32, 64} and persistent grid of {2,4,6,8} blocks
- * per SM and keeps
+ * grid, 2..64 rows; 4, 8, 16, 32, 64} and number of {2,4,6,8} blocks per SM
+ * that the problems' groups are cut for, and keeps
  * the fastest (best_ms: its time). Leaves the energy fields unchanged. */
 int tl2d_batch_tune(TlBatch* batch, int trial_iters, double* best_ms);
 void tl2d_batch_config(TlBatch* batch, int* tile_rows, int* grid_blocks);

@@ -982,8 +982,9 @@ void tl2d_batch_destroy(TlBatch* B)
 // Autotuner: times `trial_iters` iterations of the batch's own CG (setup
 // included, energy untouched; 0: the whole solve) for each tile height in
 // {adaptive (-1), 4, 8, 16, 32, 64}
-// and each persistent grid of {2, 4, 6, 8} blocks per SM (within the
-// co-residency limit), and keeps the fastest. Returns 0 or an error code;
+// and each number of {2, 4, 6, 8} blocks per SM that the problems' groups are
+// cut for (of which as many as fit at once are launched, 4 or 6 per SM), and
+// keeps the fastest. Returns 0 or an error code;
 // the choice is readable with tl2d_batch_config.
 int tl2d_batch_tune(TlBatch* B, int trial_iters, double* best_ms)
 {

@@ -23,12 +23,20 @@
 // BS > 0: the preconditioned CG of pcg2d.cuh, BS rows to a block of M (1:
 // jac_diag, 4: jac_block), in strips of whole blocks. z takes w's registers
 // once r is updated, the edge cells handed over are z's (p = beta p + z),
-// mi stays in shared memory (strips of 7 and 8 rows read it through L2) and the second sum is the pair r.r, r.z. w of the
-// last trip is formed again at the end.
+// mi stays in shared memory (strips of 7 and 8 rows read it through L2) and the
+// second sum is the pair r.r, r.z. w of the last trip is formed again at the
+// end. The strips are rounded up to whole blocks, which the two-launch loop does
+// for its u/r/z sweep only: with jac_block on a mesh whose strips are not a
+// multiple of 4 rows, p.w is summed over another partition than there (3e-15
+// relative); everywhere else the two loops agree bit for bit.
 //
 // What bounds it: two sums per trip, each one hand-over through L2, three block
-// barriers and two shuffle trees (about 2 us of a trip); then, from about 8
-// rows a thread, shared-memory bandwidth. Measured, us per trip of a whole
+// barriers and two shuffle trees (about 2 us of a trip); then the latency of the
+// rows' own chains at 12 or 16 warps an SM. Captured: 512^2 and 1000^2 issue in 30
+// and 32 % of the slots, the largest stalls the block barriers and the polls;
+// at 14 rows a thread shared memory is 33 % busy, FP64 15 %. The kernel holds
+// its SMs from the first trip to the last: another stream's solve waits for it.
+// Measured, us per trip of a whole
 // timestep: 64^2 5.7 against 20 for the two launches per trip it replaces,
 // 512^2 6.5 against 27, 1000^2 10.2; 1080^2, just past the limit, still takes
 // 37 with two launches.
@@ -55,8 +63,10 @@ struct ChipArgs {
     int polls;                 // polls of a wait before it gives up
 };
 
-// Where a block keeps the arrays other than p, r and w: registers while 128 a
-// thread suffice, else shared memory, laid out for the largest block. The
+// Where a block keeps the arrays other than p, r and w: registers up to the rows
+// given here, else shared memory, laid out for the largest block. No form fits
+// its 128 registers a thread without spills: 56 bytes of stores at 3 rows and
+// jac_diag to 616 at 8 rows and jac_block. The
 // operator is held as the face coefficient left of each cell, the one below
 // and, while there is room, the diagonal 1 + (kxr + kxc) + (kyu + kyc); kx is
 // laid out 33 to a warp, the last being the one right of its columns.

@@ -13,6 +13,9 @@
 // cells of p itself and updates them from the edge cells of r that their
 // owners hand over.
 //
+// What bounds it: the sums' hand-overs and, of the unit's 128 registers a thread
+// (48 to 808 bytes of spill stores), one barrier per plane in the w sweep. 48^3
+// captured: 13 % of the issue slots, the largest stalls the polls and the barriers.
 // Measured, us per trip of a whole timestep, against the two launches per trip
 // it replaces: 32^3 6.7 / 23.0, 48^3 8.8 / 21.9, 64^3 9.2 / 23.8, 80^3 11.2 /
 // 30.2, 100 x 90 x 80 20.9 / 39.5.

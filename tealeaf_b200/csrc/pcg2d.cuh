@@ -25,7 +25,9 @@
 //
 // Algorithmic bytes per cell and iteration: the w sweep 48 (z, p_old, kx, ky
 // -> p, w), the u/r/z sweep 64 for jac_diag (u, p, r, w, mi -> u, r, z) and
-// 72 for jac_block (+ ky): 112 / 120 against plain CG's 96. The element-wise
+// 72 for jac_block (+ ky): 112 / 120 against plain CG's 84 (96 where u is
+// updated in every trip, as here). A mesh that fits on chip runs the loop in
+// cgchip2d.cuh, with no field traffic per trip. The element-wise
 // operations follow the oracle's restatement (oracle/tl_oracle.c,
 // o2_precond_factor, o2_precond) in order, so z is bit-identical to it.
 #pragma once
