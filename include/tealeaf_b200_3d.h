@@ -340,8 +340,10 @@ void tl3d_solve_step(Chunk* chunk, Settings* settings, int tt, TlStepStats3* sta
  * accumulates into grad (dJ/drho) the face-coefficient term
  * -sum_f dk_f/drho_c (lam_a - lam_b)(u_a - u_b). g_u, u (this step's forward
  * solution), lam and grad are device arrays in the chunk layout. The chunk's
- * p, r and w are overwritten. One chunk, six external faces, CG solver.
- * Returns 0, or an error code (message from tl3d_get_error). */
+ * p, r and w are overwritten. One chunk, six external faces, CG solver. At most
+ * settings->max_iters iterations, and no more than the chunk was initialised with
+ * (error 32 when the solve needs them). Returns 0, or an error code (message from
+ * tl3d_get_error). */
 int tl3d_solve_step_backward(Chunk* chunk, Settings* settings, const double* g_u, const double* u,
         double* lam, double* grad, double rel_tol, int* iterations);
 

@@ -169,7 +169,9 @@ void copy_field(TlSuite3D* s, double* dst, const double* src)
 }
 
 // CG solve A lam = rhs from lam = 0 to r.r <= rel_tol^2 rhs.rhs with the
-// forward loops; clobbers the chunk's p, r, w. Returns the iterations.
+// forward loops; clobbers the chunk's p, r, w. Returns the iterations. The loops
+// record every trip's alpha and beta in tables of the length the chunk was
+// initialised with, so no more trips run: a solve that needs them is an error.
 int adjoint_solve(TlSuite3D* s, Chunk* chunk, const double* rhs, double* lam, double rel_tol, int max_iters)
 {
     s->h_mirror[0] = 0;
@@ -184,20 +186,26 @@ int adjoint_solve(TlSuite3D* s, Chunk* chunk, const double* rhs, double* lam, do
     flush(s, chunk);
     DevParams prm{};
     prm.eps = rel_tol * rel_tol * gg;
-    prm.max_iters = max_iters;
+    prm.max_iters = std::min(max_iters, s->table_len);
+    auto trips = [&](const DevState& st) {
+        if (st.reason == 3 && max_iters > s->table_len)
+            tl::fail(32, "the adjoint solve needs more iterations than the %d the chunk was initialised with (max_iters %d)",
+                     s->table_len, max_iters);
+        return st.trip;
+    };
     if (cg_chip3(s, chunk, lam, prm)) {
         DevState st{};
         TL_CUDA(cudaMemcpyAsync(&st, s->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
         TL_CUDA(cudaStreamSynchronize(s->stream));
         check_chip(s);
-        return st.trip;
+        return trips(st);
     }
-    return cg_deferred3(s, chunk, lam, prm, [&](auto&& trip) {
-               batched(s, max_iters, trip);
-               DevState st{};
-               TL_CUDA(cudaMemcpy(&st, s->d_state, sizeof(DevState), cudaMemcpyDeviceToHost));
-               return st;
-           }).trip;
+    return trips(cg_deferred3(s, chunk, lam, prm, [&](auto&& trip) {
+        batched(s, prm.max_iters, trip);
+        DevState st{};
+        TL_CUDA(cudaMemcpy(&st, s->d_state, sizeof(DevState), cudaMemcpyDeviceToHost));
+        return st;
+    }));
 }
 
 void face_grad(TlSuite3D* s, Chunk* chunk, Settings* settings, const double* lam, const double* u, double* grad)
